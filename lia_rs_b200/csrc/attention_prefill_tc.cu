@@ -33,8 +33,8 @@
 // point and its sum in scratch memory, and attention_prefill_merge_kernel puts a row's ranges together.
 //
 // Rows are (token, head) pairs: row r is token r / g, head r % g of the CTA's tokens, so the keys of a kv
-// head are read once for all its query heads.  Head sizes 64 and 128, the keys' and the values' apart, g a divisor of
-// 128; the caller uses other kernels (attention_prefill.cu, attention_generic.cu) for everything else.
+// head are read once for all its query heads.  Head sizes 64 and 128, the keys' and the values' apart, or keys of 192 with
+// values of 128 and keys of 96 with values of 64 (what a latent's records expand to; two stages at 192), g a divisor of 128; the caller uses other kernels (attention_prefill.cu, attention_generic.cu) for everything else.
 #include "attention_tmem.cuh"
 
 using namespace tc5;
@@ -45,7 +45,10 @@ constexpr int KT = 128;                  // keys per tile: N of the first produc
 constexpr int SOFTMAX_WARPS = 8, LOAD_WARPS = 4;
 constexpr int THREADS = (SOFTMAX_WARPS + 1 + LOAD_WARPS) * 32;
 constexpr int LOADERS = LOAD_WARPS * 32;
-constexpr int STAGES = 3;                // K and V tiles in flight (the probabilities live in tensor memory, so three fit)
+// K and V tiles in flight: three (the probabilities live in tensor memory), or two of keys of more than 128 elements
+template <int D> __host__ __device__ constexpr int stages_of() { return D > 128 ? 2 : 3; }
+// Bytes of a tile of `rows` rows of D elements: blocks of 64 elements, the last one padded to a whole block
+template <int D> __host__ __device__ constexpr uint32_t tile_bytes(int rows) { return (uint32_t)rows * 128u * (uint32_t)((D + 63) / 64); }
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LAZY = 8.f;              // see the softmax
 
@@ -70,7 +73,13 @@ struct Params {
     long long n_rows_total;          // tokens * nq
     int sink;                        // 1: exp(the head's sink) is added to the softmax's denominator (a key of that score without a value)
     const float* sinks;              // [nq] the heads' sinks; null: zero for every head
+    long long k_row, v_row;          // elements from one cache row's keys (values) to the next: nkv D (nkv DV) where nothing lies between
+    const float* gate;               // [tokens, gate_row]: the output times sigmoid(gate), a number an element, or, with gate_head, a head; null: none
+    long long gate_row;
+    int gate_head, gate_vec;         // gate_vec: its rows and heads begin at 16-byte boundaries
 };
+
+__device__ __forceinline__ float sigmoid(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
 
 // The sink of head h as a base-2 logarithm.
 __device__ __forceinline__ float sink_log2(const Params& p, int h) { return p.sinks ? p.sinks[h] * LOG2E : 0.f; }
@@ -79,12 +88,13 @@ __device__ __forceinline__ float sink_log2(const Params& p, int h) { return p.si
 template <int D, int DV, bool CAP = false>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_prefill_tc_kernel(Params p) {
+    constexpr int STAGES = stages_of<D>();
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t q_full, k_full[STAGES], v_full[STAGES], k_empty[STAGES], v_empty[STAGES], s_full[2], p_ready, p_free[2];
     __shared__ uint32_t tmem_base_slot;
     __shared__ short pair_ref[2][2][ROWS];         // what the two threads of a row tell each other (16 bits: shared memory is full to the last KB)
     constexpr int PIECES = D / 8;                      // 16-byte pieces per row
-    constexpr uint32_t Q_BYTES = ROWS * D * 2, K_BYTES = KT * D * 2, KV_BYTES = KT * (D + DV) * 2;      // KV: a stage's keys and values
+    constexpr uint32_t Q_BYTES = tile_bytes<D>(ROWS), K_BYTES = tile_bytes<D>(KT), KV_BYTES = K_BYTES + tile_bytes<DV>(KT);      // KV: a stage's keys and values
     // tensor memory: two score buffers of 128 columns, the output's head_dim columns (128 kept), and two buffers of
     // probabilities of 64 columns (128 keys as bf16 pairs)
     constexpr int TMEM_COLS = 512;
@@ -93,10 +103,11 @@ attention_prefill_tc_kernel(Params p) {
     const uint32_t q_s = smem_base, kv_s = q_s + Q_BYTES;   // kv_s: [stage][K, V]
     uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
 
-    // ---- which portion, which tokens, which kv head (later tiles first: they have the most keys) ----
+    // ---- which portion, which tokens, which kv head (later tiles first, all heads of a tile together: the CTAs with the
+    //      most keys begin first, and the short ones fill what is left) ----
     const int group = p.nq / p.nkv;
-    const int kvh = blockIdx.y;
-    int tile = gridDim.x - 1 - blockIdx.x, seg = 0, q_offset = 0, seg_start = 0, seg_count = 0;
+    const int kvh = blockIdx.x % p.nkv;
+    int tile = (gridDim.x - 1 - blockIdx.x) / p.nkv, seg = 0, q_offset = 0, seg_start = 0, seg_count = 0;
     for (; seg < p.n_segments; ++seg) {
         q_offset = p.segments[seg * 3];
         seg_start = p.segments[seg * 3 + 1];
@@ -170,7 +181,35 @@ attention_prefill_tc_kernel(Params p) {
             const int key0 = key_begin + j * KT;
             // PIECES lanes share a key row (their 16-byte pieces make one coalesced request); lane j of them looks
             // up the row of pass j
-            {
+            if constexpr ((PIECES & (PIECES - 1)) != 0) {
+                // keys of 96 or 192 elements: eight lanes a row, a block of 64 elements after the other
+                constexpr int PASSES = KT / (LOADERS / 8);
+                static_assert(PASSES == 8, "one lane per pass");
+                const int sub = lt / 8, lane8 = lt % 8, key = key0 + sub + lane8 * (LOADERS / 8);
+                const int my_row = key < key_end ? cache_row_of(table, key, p.page_size, p.page_shift, p.num_pages, p.error_flag) : -1;
+                int rows[PASSES];
+#pragma unroll
+                for (int i = 0; i < PASSES; ++i) {
+                    const int row = __shfl_sync(0xffffffffu, my_row, (lane & ~7) + i);
+                    const bool valid = row >= 0;
+                    const size_t src = (size_t)(valid ? row : 0) * p.k_row + kvh * D + lane8 * 8;
+#pragma unroll
+                    for (int b = 0; b < PIECES; b += 8)
+                        if (b + lane8 < PIECES) cp_async_16(ks + tile_offset<KT>(sub + i * (LOADERS / 8), b + lane8), p.k_pages + src + b * 8, valid);
+                    rows[i] = row;
+                }
+                cp_async_commit();
+                if (j >= STAGES && !mbar_wait(smem_u32(&v_empty[st]), ((uint32_t)(j / STAGES) & 1u) ^ 1u)) { ok = false; break; }
+#pragma unroll
+                for (int i = 0; i < PASSES; ++i) {
+                    const bool valid = rows[i] >= 0;
+                    const size_t src = (size_t)(valid ? rows[i] : 0) * p.v_row + kvh * DV + lane8 * 8;
+#pragma unroll
+                    for (int b = 0; b < DV / 8; b += 8)
+                        cp_async_16(vs + tile_offset<KT>(sub + i * (LOADERS / 8), b + lane8), p.v_pages + src + b * 8, valid);
+                }
+                cp_async_commit();
+            } else {
                 constexpr int ROWS_PER_PASS = LOADERS / PIECES, PASSES = KT / ROWS_PER_PASS;
                 static_assert(PASSES <= PIECES, "one lane per pass");
                 const int sub = lt / PIECES, piece = lt % PIECES, lane_group = (lane / PIECES) * PIECES;
@@ -183,7 +222,7 @@ attention_prefill_tc_kernel(Params p) {
                 for (int i = 0; i < PASSES; ++i) {
                     const int row = __shfl_sync(0xffffffffu, my_row, lane_group + i);
                     const bool valid = row >= 0;
-                    const size_t src = ((size_t)(valid ? row : 0) * p.nkv + kvh) * D + piece * 8;
+                    const size_t src = (size_t)(valid ? row : 0) * p.k_row + kvh * D + piece * 8;
                     const uint32_t at = tile_offset<KT>(sub + i * ROWS_PER_PASS, piece);
                     cp_async_16(ks + at, p.k_pages + src, valid);
                     rows[i] = row;
@@ -194,7 +233,7 @@ attention_prefill_tc_kernel(Params p) {
 #pragma unroll
                     for (int i = 0; i < PASSES; ++i) {
                         const bool valid = rows[i] >= 0;
-                        const size_t src = ((size_t)(valid ? rows[i] : 0) * p.nkv + kvh) * D + piece * 8;
+                        const size_t src = (size_t)(valid ? rows[i] : 0) * p.v_row + kvh * D + piece * 8;
                         cp_async_16(vs + tile_offset<KT>(sub + i * ROWS_PER_PASS, piece), p.v_pages + src, valid);
                     }
                 } else {
@@ -211,7 +250,7 @@ attention_prefill_tc_kernel(Params p) {
                     for (int i = 0; i < V_PASSES; ++i) {
                         const int row = __shfl_sync(0xffffffffu, my_v_row, v_group + i);
                         const bool valid = row >= 0;
-                        const size_t src = ((size_t)(valid ? row : 0) * p.nkv + kvh) * DV + v_piece * 8;
+                        const size_t src = (size_t)(valid ? row : 0) * p.v_row + kvh * DV + v_piece * 8;
                         cp_async_16(vs + tile_offset<KT>(v_sub + i * V_ROWS, v_piece), p.v_pages + src, valid);
                     }
                 }
@@ -404,6 +443,31 @@ attention_prefill_tc_kernel(Params p) {
             mbar_arrive(smem_u32(&p_ready));
         }
         // ---- the row's output: the two threads' sums meet, each writes half the columns ----
+        // (a gate's numbers are asked for before the last product is awaited: a row a thread is 64 bytes a request, and
+        // fetched one group of columns after the other behind the products they doubled the kernel's time, 40 -> 83 us at 2,048
+        // tokens of 16 heads)
+        constexpr int SHARE = DV / 2;
+        float gates[SHARE];
+        if (p.gate && p.splits <= 1) {
+            const float* g = p.gate + (size_t)(q_offset + tok0 + (row_ok ? tok : 0)) * p.gate_row;
+            if (p.gate_head) {
+                const float z = g[kvh * group + head];
+#pragma unroll
+                for (int c = 0; c < SHARE; ++c) gates[c] = z;
+            } else {
+                g += (size_t)(kvh * group + head) * DV + half * SHARE;
+                if (p.gate_vec) {
+#pragma unroll
+                    for (int c = 0; c < SHARE; c += 4) {
+                        const float4 z = *reinterpret_cast<const float4*>(g + c);
+                        gates[c] = z.x, gates[c + 1] = z.y, gates[c + 2] = z.z, gates[c + 3] = z.w;
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < SHARE; ++c) gates[c] = g[c];
+                }
+            }
+        }
         if (ok && !mbar_wait(smem_u32(&p_free[(n_tiles - 1) & 1]), (uint32_t)((n_tiles - 1) >> 1) & 1u)) ok = false;
         tc_fence_after();
         float* pair_sum = reinterpret_cast<float*>(smem);                   // [2][ROWS], where Q was: every product is done
@@ -429,13 +493,19 @@ attention_prefill_tc_kernel(Params p) {
             }
         } else if (ok) {
             const float inv = 1.0f / (pair_sum[r] + pair_sum[ROWS + r] + (p.sink ? exp2f(sink_log2(p, kvh * group + head) - row_max) : 0.f));
-            __nv_bfloat16* dst = p.out + ((size_t)(q_offset + tok0 + (row_ok ? tok : 0)) * p.nq + kvh * group + head) * DV;
-#pragma unroll 1
-            for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 16) {
+            const size_t out_row = (size_t)(q_offset + tok0 + (row_ok ? tok : 0)) * p.nq + kvh * group + head;
+            __nv_bfloat16* dst = p.out + out_row * DV;
+#pragma unroll
+            for (int i = 0; i < SHARE / 16; ++i) {
+                const int c0 = half * SHARE + i * 16;
                 float o[16];
                 tmem_load16(tmem_o + lane_base + (uint32_t)c0, o);           // every lane takes part in the load
                 if (row_ok) {
                     uint32_t packed[8];
+                    if (p.gate) {
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) o[c] *= sigmoid(gates[i * 16 + c]);
+                    }
 #pragma unroll
                     for (int c = 0; c < 16; c += 2) {
                         __nv_bfloat162 pair = __floats2bfloat162_rn(o[c] * inv, o[c + 1] * inv);
@@ -523,20 +593,26 @@ __global__ void __launch_bounds__(128) attention_prefill_merge_kernel(Params p) 
     if (p.sink) total += exp2f(sink_log2(p, kvh * group + head) - top);                  // the sink joins once, where the ranges meet
     const float inv = 1.0f / total;
     __nv_bfloat16* dst = p.out + row * D + lane * E;
+    if (p.gate) {
+        const float* g = p.gate + (size_t)(q_offset + tok0 + tok) * p.gate_row;
+        const int out_head = kvh * group + head;
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e] *= sigmoid(g[p.gate_head ? out_head : out_head * D + lane * E + e]);
+    }
 #pragma unroll
     for (int e = 0; e < E; e += 2) *reinterpret_cast<__nv_bfloat162*>(dst + e) = __floats2bfloat162_rn(acc[e] * inv, acc[e + 1] * inv);
 }
 
 template <int D, int DV, bool CAP = false>
 int launch(const Params& p, int n_tiles, cudaStream_t stream) {
-    const size_t smem = (size_t)ROWS * D * 2 + (size_t)STAGES * KT * (D + DV) * 2 + 1024;
+    const size_t smem = (size_t)tile_bytes<D>(ROWS) + (size_t)stages_of<D>() * (tile_bytes<D>(KT) + tile_bytes<DV>(KT)) + 1024;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(attention_prefill_tc_kernel<D, DV, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return LIA_ERR_LAUNCH;
         configured = true;
     }
-    const int rc = lia_launch(attention_prefill_tc_kernel<D, DV, CAP>, dim3(n_tiles, p.nkv, p.splits), dim3(THREADS), smem, stream, p);
+    const int rc = lia_launch(attention_prefill_tc_kernel<D, DV, CAP>, dim3((unsigned)n_tiles * p.nkv, 1, p.splits), dim3(THREADS), smem, stream, p);
     if (rc != LIA_OK || p.splits <= 1) return rc;
     return lia_launch(attention_prefill_merge_kernel<DV>, dim3(n_tiles, p.nkv, ROWS / 4), dim3(128), 0, stream, p);
 }
@@ -545,7 +621,8 @@ int launch(const Params& p, int n_tiles, cudaStream_t stream) {
 // Tokens of a portion that one CTA takes for `group` query heads per kv head and these head sizes of keys and values (0:
 // the tcgen05 kernel does not take the combination; use another kernel).
 LIA_EXPORT int lia_attention_prefill_tc_tokens_per_tile(int group, int d, int dv) {
-    if ((d != 64 && d != 128) || (dv != 64 && dv != 128)) return 0;
+    // (keys of 192 or 96 elements: whole keys of an expanded latent, 128 + 64 and 64 + 32)
+    if (!((d == 192 && dv == 128) || (d == 96 && dv == 64)) && ((d != 64 && d != 128) || (dv != 64 && dv != 128))) return 0;
     return group >= 1 && group <= ROWS && ROWS % group == 0 ? ROWS / group : 0;
 }
 
@@ -554,17 +631,24 @@ LIA_EXPORT int lia_attention_prefill_tc_tokens_per_tile(int group, int d, int dv
 // 128-key tiles, each range a CTA of its own, and a second kernel merges them (few tokens over a long context
 // would otherwise leave most SMs idle); `partial` then holds splits * n_tokens * nq * (the values' head size + 2) 32-bit words,
 // `n_tokens` being the tokens of the whole batch that `q` and `out` cover.  `sink`: one is added to the softmax's denominator;
-// `sinks` [nq] (32-bit, or null): exp(sinks[h]) instead, of head h.
+// `sinks` [nq] (32-bit, or null): exp(sinks[h]) instead, of head h.  `k_row`, `v_row`: elements from one cache row to the next
+// (0: the rows lie side by side); `gate` (32-bit rows [n_tokens, gate_row], or null): the output times its sigmoid ahead of the
+// rounding, a number an element, or with `gate_head` a head.
 LIA_EXPORT int lia_attention_prefill_tc(const void* q, const void* k_pages, const void* v_pages, const int* segments,
                                         int n_segments, int n_tiles, const int* slots, const int* block_table,
                                         int table_stride, void* out, int nq, int nkv, int d, int dv, int page_size, int window,
                                         float scale, int num_pages, int splits, float* partial, int n_tokens, int sink,
-                                        const float* sinks, float softcap, int* error_flag, cudaStream_t stream) {
+                                        const float* sinks, float softcap, long long k_row, long long v_row, const float* gate,
+                                        long long gate_row, int gate_head, int* error_flag, cudaStream_t stream) {
     if (n_segments <= 0 || n_tiles <= 0) return LIA_OK;
     if (nq <= 0 || nkv <= 0 || nq % nkv || page_size <= 0 || nkv > 65535) return LIA_ERR_SIZE;
     if (splits < 1 || splits > 32 || (splits > 1 && (!partial || n_tokens <= 0))) return LIA_ERR_SIZE;
     const int per_tile = lia_attention_prefill_tc_tokens_per_tile(nq / nkv, d, dv);
     if (per_tile == 0) return LIA_ERR_SIZE;
+    if (k_row <= 0) k_row = (long long)nkv * d;
+    if (v_row <= 0) v_row = (long long)nkv * dv;
+    if (k_row < (long long)nkv * d || v_row < (long long)nkv * dv || k_row % 8 || v_row % 8 || (gate && gate_row <= 0))
+        return LIA_ERR_SIZE;
     if (((uintptr_t)q & 15u) || ((uintptr_t)out & 15u) || ((uintptr_t)k_pages & 15u) || ((uintptr_t)v_pages & 15u) ||
         ((uintptr_t)partial & 15u))
         return LIA_ERR_ALIGN;
@@ -585,9 +669,16 @@ LIA_EXPORT int lia_attention_prefill_tc(const void* q, const void* k_pages, cons
     p.splits = splits;
     p.sink = sink || sinks ? 1 : 0;
     p.sinks = sinks;
+    p.k_row = k_row; p.v_row = v_row;
+    p.gate = gate; p.gate_row = gate_row; p.gate_head = gate_head;
+    p.gate_vec = ((uintptr_t)gate & 15u) == 0 && gate_row % 4 == 0 ? 1 : 0;
     p.n_rows_total = (long long)n_tokens * nq;
     p.partial_o = partial;
     p.partial_ms = partial ? partial + (size_t)splits * p.n_rows_total * dv : nullptr;
+    if (d == 192 || d == 96) {
+        if (p.cap_in != 0.f) return LIA_ERR_SIZE;
+        return d == 192 ? launch<192, 128>(p, n_tiles, stream) : launch<96, 64>(p, n_tiles, stream);
+    }
     if (d != dv) {
         if (p.cap_in != 0.f) return d == 64 ? launch<64, 128, true>(p, n_tiles, stream) : launch<128, 64, true>(p, n_tiles, stream);
         return d == 64 ? launch<64, 128>(p, n_tiles, stream) : launch<128, 64>(p, n_tiles, stream);

@@ -120,7 +120,7 @@ template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bf
 template <typename TW, typename TO, int VPL>      // VPL: float4 per lane; the row has at most 128 * VPL elements
 __global__ void rmsnorm_warp_kernel(const float* __restrict__ x, const int* __restrict__ rows_index,
                                     const TW* __restrict__ weight, TO* __restrict__ out, int rows,
-                                    int hidden, float eps, float out_scale) {
+                                    int hidden, long long ld, float eps, float out_scale) {
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -143,7 +143,7 @@ __global__ void rmsnorm_warp_kernel(const float* __restrict__ x, const int* __re
         }
         return;
     }
-    const float* row = x + (size_t)src * hidden;
+    const float* row = x + (size_t)src * ld;
     float4 v[VPL];
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
@@ -172,7 +172,7 @@ __global__ void rmsnorm_warp_kernel(const float* __restrict__ x, const int* __re
 template <typename TW, typename TO>
 __global__ void rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ rows_index,
                                const TW* __restrict__ weight, TO* __restrict__ out, int rows,
-                               int hidden, float eps, float out_scale) {
+                               int hidden, long long ld, float eps, float out_scale) {
     __shared__ float scratch[32];
     pdl_launch_dependents();
     pdl_wait();
@@ -184,7 +184,7 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const int* __restric
         for (int i = threadIdx.x; i < hidden; i += blockDim.x) dst[i] = from_float<TO>(0.f);
         return;
     }
-    const float* row = x + (size_t)src * hidden;
+    const float* row = x + (size_t)src * ld;
     float sum = 0.f;
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
         const float v = row[i];
@@ -198,17 +198,17 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const int* __restric
 
 template <typename TW, typename TO>
 int launch_rmsnorm(const float* x, const int* rows_index, const void* weight, void* out, int rows, int hidden,
-                   float eps, float out_scale, cudaStream_t stream) {
-    const bool vector = hidden % 4 == 0 && hidden <= 4096 && ((uintptr_t)x & 15u) == 0 && ((uintptr_t)weight & 15u) == 0 &&
+                   long long ld, float eps, float out_scale, cudaStream_t stream) {
+    const bool vector = hidden % 4 == 0 && hidden <= 4096 && ld % 4 == 0 && ((uintptr_t)x & 15u) == 0 && ((uintptr_t)weight & 15u) == 0 &&
                         ((uintptr_t)out & 15u) == 0;
     if (!vector)
         return lia_launch(rmsnorm_kernel<TW, TO>, dim3(rows), dim3(hidden >= 1024 ? 256 : 128), 0, stream, x, rows_index,
-                          (const TW*)weight, (TO*)out, rows, hidden, eps, out_scale);
+                          (const TW*)weight, (TO*)out, rows, hidden, ld, eps, out_scale);
     const int warps = rows >= 256 ? 4 : 1;             // few rows: one warp per CTA, spread over the SMs
     const dim3 grid((rows + warps - 1) / warps), block(warps * 32);
 #define LIA_NORM_WARP(VPL)                                                                                          \
     return lia_launch(rmsnorm_warp_kernel<TW, TO, VPL>, grid, block, 0, stream, x, rows_index, (const TW*)weight, \
-                      (TO*)out, rows, hidden, eps, out_scale)
+                      (TO*)out, rows, hidden, ld, eps, out_scale)
     if (hidden <= 512) LIA_NORM_WARP(4);
     if (hidden <= 1024) LIA_NORM_WARP(8);
     if (hidden <= 2048) LIA_NORM_WARP(16);
@@ -216,19 +216,20 @@ int launch_rmsnorm(const float* x, const int* rows_index, const void* weight, vo
 #undef LIA_NORM_WARP
 }
 
-LIA_EXPORT int lia_rmsnorm(const float* x, const int* rows_index, const void* weight, int weight_dtype,
+// x: rows of `ld` elements, of which the first `hidden` are normed.
+LIA_EXPORT int lia_rmsnorm(const float* x, long long ld, const int* rows_index, const void* weight, int weight_dtype,
                            void* out, int out_dtype, int rows, int hidden, float eps, float out_scale,
                            cudaStream_t stream) {
     if (rows <= 0) return LIA_OK;
-    if (hidden <= 0) return LIA_ERR_SIZE;
+    if (hidden <= 0 || ld < hidden) return LIA_ERR_SIZE;
     if (weight_dtype == LIA_BF16 && out_dtype == LIA_BF16)
-        return launch_rmsnorm<__nv_bfloat16, __nv_bfloat16>(x, rows_index, weight, out, rows, hidden, eps, out_scale, stream);
+        return launch_rmsnorm<__nv_bfloat16, __nv_bfloat16>(x, rows_index, weight, out, rows, hidden, ld, eps, out_scale, stream);
     if (weight_dtype == LIA_BF16 && out_dtype == LIA_F32)
-        return launch_rmsnorm<__nv_bfloat16, float>(x, rows_index, weight, out, rows, hidden, eps, out_scale, stream);
+        return launch_rmsnorm<__nv_bfloat16, float>(x, rows_index, weight, out, rows, hidden, ld, eps, out_scale, stream);
     if (weight_dtype == LIA_F32 && out_dtype == LIA_BF16)
-        return launch_rmsnorm<float, __nv_bfloat16>(x, rows_index, weight, out, rows, hidden, eps, out_scale, stream);
+        return launch_rmsnorm<float, __nv_bfloat16>(x, rows_index, weight, out, rows, hidden, ld, eps, out_scale, stream);
     if (weight_dtype == LIA_F32 && out_dtype == LIA_F32)
-        return launch_rmsnorm<float, float>(x, rows_index, weight, out, rows, hidden, eps, out_scale, stream);
+        return launch_rmsnorm<float, float>(x, rows_index, weight, out, rows, hidden, ld, eps, out_scale, stream);
     return LIA_ERR_DTYPE;
 }
 
@@ -458,5 +459,35 @@ LIA_EXPORT int lia_gather_rows(const void* src, const int* index, void* dst, int
     if ((together & 1u) == 0)
         return lia_launch(gather_rows_kernel<uint16_t>, dim3(rows), dim3(threads), 0, stream, (const uint16_t*)src, index,
                           (uint16_t*)dst, rows, src_rows, src_stride_bytes / 2, dst_stride_bytes / 2, (int)(row_bytes / 2));
+    return LIA_ERR_ALIGN;
+}
+
+// Rows put where they belong: row r of src to row index[r] of dst, one warp-wide copy a row as in gather_rows (its mirror).
+template <typename V>
+__global__ void scatter_rows_kernel(const V* __restrict__ src, const int* __restrict__ index, V* __restrict__ dst, int dst_rows,
+                                    long long src_stride, long long dst_stride, int words) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int to = index[blockIdx.x];
+    if (to < 0 || to >= dst_rows) return;
+    const V* in = src + (size_t)blockIdx.x * src_stride;
+    V* out = dst + (size_t)to * dst_stride;
+    for (int i = threadIdx.x; i < words; i += blockDim.x) out[i] = in[i];
+}
+
+// src [rows, src_stride_bytes a row], dst [dst_rows, dst_stride_bytes a row], row_bytes copied per row; an index outside dst
+// names nobody.  Sizes, strides and bases multiples of 4 bytes.
+LIA_EXPORT int lia_scatter_rows(const void* src, const int* index, void* dst, int rows, int dst_rows, long long src_stride_bytes,
+                                long long dst_stride_bytes, long long row_bytes, cudaStream_t stream) {
+    if (rows <= 0 || row_bytes <= 0) return LIA_OK;
+    if (dst_rows <= 0 || src_stride_bytes < row_bytes || dst_stride_bytes < row_bytes || row_bytes > (1LL << 30)) return LIA_ERR_SIZE;
+    const uintptr_t together = (uintptr_t)src | (uintptr_t)dst | (uintptr_t)src_stride_bytes | (uintptr_t)dst_stride_bytes |
+                               (uintptr_t)row_bytes;
+    if ((together & 15u) == 0)
+        return lia_launch(scatter_rows_kernel<uint4>, dim3(rows), dim3(128), 0, stream, (const uint4*)src, index, (uint4*)dst,
+                          dst_rows, src_stride_bytes / 16, dst_stride_bytes / 16, (int)(row_bytes / 16));
+    if ((together & 3u) == 0)
+        return lia_launch(scatter_rows_kernel<uint32_t>, dim3(rows), dim3(128), 0, stream, (const uint32_t*)src, index,
+                          (uint32_t*)dst, dst_rows, src_stride_bytes / 4, dst_stride_bytes / 4, (int)(row_bytes / 4));
     return LIA_ERR_ALIGN;
 }

@@ -15,7 +15,7 @@
 // cut depends on the token's own span alone.
 //
 // q1 [heads, tokens, rank] and out [heads, tokens, rank] are planes per head (a head's rows are a matrix for the
-// products before and after), q2 [tokens, heads, dr].  rank a multiple of 32 up to 512, dr a multiple of 16 up to 128.
+// products before and after), q2 [tokens, heads, dr] by strides.  rank a multiple of 32 up to 512, dr a multiple of 16 up to 128.
 
 #include "common.cuh"
 
@@ -32,8 +32,10 @@ struct LatentParams {
     const __nv_bfloat16* part_pages;     // [pages, page_size, dr]
     const int* positions;
     const int* slots;
+    const int* rows;                     // [n_tokens] which of the step's tokens these are (null: token t is row t)
     const int* block_table;
     __nv_bfloat16* out;
+    long long q2_token, q2_head;         // strides of q2 in elements
     float* partial;                      // splits > 1: [splits][heads][tokens][rank] outputs, then [splits][heads][tokens][2] maximum and sum
     int n_tokens, heads, rank, dr, table_stride, page_size, window, num_pages, splits;
     float scale_log2;
@@ -69,9 +71,10 @@ latent_attention_kernel(LatentParams p) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x, h0 = blockIdx.y * 16;
-    const int slot = p.slots[t];
+    const int row_of_step = p.rows ? p.rows[t] : t;
+    const int slot = p.slots[row_of_step];
     if (slot < 0) return;
-    const int pos = p.positions[t];
+    const int pos = p.positions[row_of_step];
     const int first = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
     const int n_tiles = (pos - first + KEYS) / KEYS;
     const int per = (n_tiles + p.splits - 1) / p.splits;
@@ -88,7 +91,7 @@ latent_attention_kernel(LatentParams p) {
         if (r < heads_here) {
             const int h = h0 + r;
             v = c < p.rank ? *reinterpret_cast<const uint4*>(p.q1 + ((size_t)h * p.n_tokens + t) * p.rank + c)
-                           : *reinterpret_cast<const uint4*>(p.q2 + ((size_t)t * p.heads + h) * p.dr + (c - p.rank));
+                           : *reinterpret_cast<const uint4*>(p.q2 + (size_t)t * p.q2_token + (size_t)h * p.q2_head + (c - p.rank));
         }
         *reinterpret_cast<uint4*>(qs + r * ld + c) = v;
     }
@@ -248,7 +251,7 @@ __global__ void latent_merge_kernel(LatentParams p) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x, h = blockIdx.y;
-    if (p.slots[t] < 0) return;
+    if (p.slots[p.rows ? p.rows[t] : t] < 0) return;
     const size_t planes = (size_t)p.heads * p.n_tokens, plane = (size_t)h * p.n_tokens + t;
     const float* ms = p.partial + (size_t)p.splits * planes * p.rank;
     float top = -INFINITY;
@@ -298,22 +301,24 @@ LIA_EXPORT long long lia_latent_attention_partial_floats(int n_tokens, int heads
     return splits > 1 ? (long long)splits * heads * n_tokens * (rank + 2) : 0;
 }
 
-LIA_EXPORT int lia_latent_attention(const void* q1, const void* q2, const void* latent_pages, const void* part_pages,
-                                    const int* positions, const int* slots, const int* block_table, int table_stride,
+// q2: head h of token t at t * q2_token + h * q2_head elements.  `rows` (or null): token t is row rows[t] of positions and slots.
+LIA_EXPORT int lia_latent_attention(const void* q1, const void* q2, long long q2_token, long long q2_head,
+                                    const void* latent_pages, const void* part_pages, const int* positions, const int* slots,
+                                    const int* rows, const int* block_table, int table_stride,
                                     void* out, float* partial, int n_tokens, int heads, int rank, int dr, int page_size,
                                     int window, float scale, int num_pages, int splits, int* error_flag,
                                     cudaStream_t stream) {
     if (n_tokens <= 0) return LIA_OK;
-    if (!lia_latent_attention_accepts(rank, dr) || heads <= 0 || page_size <= 0 || splits < 1 || splits > 64 ||
+    if (!lia_latent_attention_accepts(rank, dr) || heads <= 0 || q2_token < dr || q2_head < dr || page_size <= 0 || splits < 1 || splits > 64 ||
         (splits > 1 && !partial))
         return LIA_ERR_SIZE;
-    if (((uintptr_t)q1 & 15u) || ((uintptr_t)q2 & 15u) || ((uintptr_t)latent_pages & 15u) || ((uintptr_t)part_pages & 15u) ||
+    if (((uintptr_t)q1 & 15u) || ((uintptr_t)q2 & 15u) || q2_token % 8 || q2_head % 8 || ((uintptr_t)latent_pages & 15u) || ((uintptr_t)part_pages & 15u) ||
         ((uintptr_t)out & 3u) || ((uintptr_t)partial & 7u))
         return LIA_ERR_ALIGN;
     LatentParams p;
     p.q1 = (const __nv_bfloat16*)q1; p.q2 = (const __nv_bfloat16*)q2;
     p.latent_pages = (const __nv_bfloat16*)latent_pages; p.part_pages = (const __nv_bfloat16*)part_pages;
-    p.positions = positions; p.slots = slots; p.block_table = block_table; p.out = (__nv_bfloat16*)out; p.partial = partial;
+    p.positions = positions; p.slots = slots; p.rows = rows; p.q2_token = q2_token; p.q2_head = q2_head; p.block_table = block_table; p.out = (__nv_bfloat16*)out; p.partial = partial;
     p.n_tokens = n_tokens; p.heads = heads; p.rank = rank; p.dr = dr; p.table_stride = table_stride; p.page_size = page_size;
     p.window = window; p.num_pages = num_pages; p.splits = splits; p.scale_log2 = scale * LOG2E; p.error_flag = error_flag;
     const dim3 grid(n_tokens, (heads + 15) / 16, splits);

@@ -39,7 +39,7 @@ def lib():
 
 class _Signatures:
     lia_embedding = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p]
-    lia_rmsnorm = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_float, c_void_p]
+    lia_rmsnorm = [c_void_p, ctypes.c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_float, c_void_p]
     lia_layernorm = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_void_p]
     lia_rope_kv_write = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
                          c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
@@ -71,7 +71,8 @@ class _Signatures:
                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p]
     lia_attention_prefill_tc = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int,
                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_int, c_int,
-                                c_void_p, c_float, c_void_p, c_void_p]
+                                c_void_p, c_float, ctypes.c_longlong, ctypes.c_longlong, c_void_p, ctypes.c_longlong, c_int,
+                                c_void_p, c_void_p]
     lia_attention_prefill_tc_tokens_per_tile = [c_int, c_int, c_int]
     lia_select_tokens = [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                          ctypes.c_longlong, c_void_p]
@@ -120,8 +121,13 @@ class _Signatures:
                        c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                        c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
     lia_latent_prepare = [c_void_p, ctypes.c_longlong, c_void_p, ctypes.c_longlong, c_void_p, c_float, c_void_p, c_int,
-                          c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                          c_void_p, c_void_p, c_void_p, c_int, c_void_p, ctypes.c_longlong, ctypes.c_longlong, c_void_p,
+                          ctypes.c_longlong, ctypes.c_longlong, c_void_p, c_void_p, c_int, c_int, c_int,
                           c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
+    lia_latent_gather = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                         c_int, c_int, c_int, c_void_p, c_void_p]
+    lia_scatter_rows = [c_void_p, c_void_p, c_void_p, c_int, c_int, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong,
+                        c_void_p]
     lia_causal_conv = [c_void_p, ctypes.c_longlong, c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_void_p, c_void_p,
                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
     lia_conv_state_update = [c_void_p, ctypes.c_longlong, c_void_p, ctypes.c_longlong, c_void_p, c_void_p, c_int, c_int,
@@ -134,7 +140,8 @@ class _Signatures:
                              c_void_p, c_int, c_int, ctypes.c_longlong, c_int, c_int, c_int, c_int, c_float, c_void_p]
 
     lia_latent_attention_accepts = [c_int, c_int]
-    lia_latent_attention = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
+    lia_latent_attention = [c_void_p, c_void_p, ctypes.c_longlong, ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                            c_void_p, c_int, c_void_p, c_void_p,
                             c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p]
     lia_gemm_mma_batched_accepts = [c_void_p, ctypes.c_longlong, ctypes.c_longlong, c_void_p, ctypes.c_longlong, ctypes.c_longlong, c_void_p, ctypes.c_longlong, ctypes.c_longlong, c_int, c_int, c_int]
     lia_embedding_streams = [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p]
@@ -340,12 +347,12 @@ def embedding_sinusoidal(tokens, positions, table, freq, out, scale: float, copy
 
 
 def rmsnorm(x, weight, out, eps: float, out_scale: float = 1.0, rows_index=None):
-    _cuda(x, weight, out, rows_index)
+    _cuda(weight, out, rows_index)
     rows, hidden = out.shape
-    if x.dtype != torch.float32 or x.shape[1] != hidden:
-        raise KernelError("rmsnorm takes 32-bit rows of the same width as its output")
+    if not x.is_cuda or x.dtype != torch.float32 or x.shape[1] != hidden or x.stride(1) != 1 or x.stride(0) < hidden:
+        raise KernelError("rmsnorm takes 32-bit rows (of any stride) of the same width as its output")
     with _timed("rmsnorm"):
-        _check(lib().lia_rmsnorm(_p(x), _p(rows_index), _p(weight), dtype_code(weight.dtype), _p(out),
+        _check(lib().lia_rmsnorm(_p(x), x.stride(0), _p(rows_index), _p(weight), dtype_code(weight.dtype), _p(out),
                                  dtype_code(out.dtype), rows, hidden, eps, out_scale, _stream()), "rmsnorm")
 
 
@@ -671,12 +678,21 @@ def attention_prefill_tc_tokens_per_tile(group: int, d: int, dv: int = None) -> 
 
 def attention_prefill_tc(q, k_pages, v_pages, segments, n_segments, n_tiles, slots, block_table, out, nq, nkv, d,
                          window, scale, error_flag=None, label=None, work_flops=0, splits=1, partial=None, sink=False,
-                         softcap=None, sinks=None):
-    """Prompt-portion attention on the tcgen05 tensor cores (bfloat16, head size 64 or 128, heads per kv head a
-    divisor of 128); see csrc/attention_prefill_tc.cu.  Arguments as `attention_prefill`.  `splits` > 1 cuts every
+                         softcap=None, sinks=None, gate=None, gate_head=False):
+    """Prompt-portion attention on the tcgen05 tensor cores (bfloat16, head sizes 64 or 128, or keys of 192 with values of
+    128, keys of 96 with values of 64; heads per kv head a divisor of 128); see csrc/attention_prefill_tc.cu.  Arguments as `attention_prefill`.  `splits` > 1 cuts every
     CTA's keys into that many ranges that run side by side and are merged by a second kernel; `partial` is their
-    32-bit scratch, `attention_prefill_tc_partial_floats` words long.  `sink`, `sinks`, `softcap`: as for `attention_decode`."""
-    _cuda(q, k_pages, v_pages, segments, slots, block_table, out, error_flag, partial, sinks)
+    32-bit scratch, `attention_prefill_tc_partial_floats` words long.  `sink`, `sinks`, `softcap`: as for `attention_decode`.
+    The pages' rows may lie apart (views [pages, page_size, nkv, d] of wider rows); `gate` (32-bit rows, an element each, or
+    with `gate_head` a head each): the output is multiplied by its sigmoid before it is rounded."""
+    _cuda(q, segments, slots, block_table, out, error_flag, partial, sinks)
+    for pages in (k_pages, v_pages):
+        if not pages.is_cuda or pages.stride(3) != 1 or pages.stride(2) != pages.shape[3] or \
+                pages.stride(0) != pages.stride(1) * pages.shape[1]:
+            raise KernelError("attention_prefill_tc: the pages' rows have one stride and whole heads side by side")
+    if gate is not None and (gate.dtype != torch.float32 or gate.stride(1) != 1 or gate.shape[0] != q.shape[0]
+                             or gate.shape[1] < (nq if gate_head else out.shape[1])):
+        raise KernelError("attention_prefill_tc: a gate is 32-bit rows of an element (or a head) each")
     _check_sinks(sinks, nq)
     if not (q.dtype == k_pages.dtype == v_pages.dtype == out.dtype == torch.bfloat16):
         raise KernelError("attention_prefill_tc is a bfloat16 kernel")
@@ -691,8 +707,9 @@ def attention_prefill_tc(q, k_pages, v_pages, segments, n_segments, n_tiles, slo
                                               _p(slots), _p(block_table), block_table.shape[1], _p(out), nq, nkv, d, dv,
                                               k_pages.shape[1], int(window or 0), scale, k_pages.shape[0], splits,
                                               _p(partial) if splits > 1 else None, q.shape[0], 1 if sink else 0, _p(sinks),
-                                              float(softcap or 0.0), _p(error_flag), _stream()),
-               "attention_prefill_tc")
+                                              float(softcap or 0.0), k_pages.stride(1), v_pages.stride(1), _p(gate),
+                                              0 if gate is None else gate.stride(0), 1 if gate_head else 0, _p(error_flag),
+                                              _stream()), "attention_prefill_tc")
 
 
 def attention_prefill_tc_partial_floats(n_tokens: int, nq: int, dv: int, splits: int) -> int:
@@ -1066,10 +1083,12 @@ def qkv_prepare(rows, bias, q_norm, k_norm, eps, freq, rot_dims, vmix_mode, vmix
 def latent_prepare(q_rows, shared_rows, latent_norm, eps, freq, rot_dims, positions, slots, block_table, q_plain,
                    q_rotated, latent_pages, key_pages, heads, d, dr, rank, write_kv=True, error_flag=None, pairs=False):
     """For attention through a latent: norm and append of the latent, encoding and append of the shared key part,
-    the queries' unrotated parts as planes [heads, tokens, d] and their rotated parts encoded [tokens, heads dr]; see
-    csrc/qk_prepare.cu.  `pairs`: the rotation pairs element 2i with 2i + 1 (else i with i + rot_dims / 2).
+    the queries' unrotated parts [heads, tokens, d] (planes, or any view with contiguous rows) and their rotated parts encoded
+    [tokens, heads dr] (or a view [tokens, heads, dr] with contiguous rows); see csrc/qk_prepare.cu.  `pairs`: the rotation pairs element 2i with 2i + 1 (else i with i + rot_dims / 2).
     `shared_rows` None: only the queries are prepared (the pages are filled by another layer)."""
-    _cuda(latent_norm, freq, positions, slots, block_table, q_plain, q_rotated, latent_pages, key_pages, error_flag)
+    _cuda(latent_norm, freq, positions, slots, block_table, latent_pages, key_pages, error_flag)
+    if not (q_plain.is_cuda and q_rotated.is_cuda) or q_plain.stride(-1) != 1 or q_rotated.stride(-1) != 1:
+        raise KernelError("latent_prepare: the queries go to CUDA tensors with contiguous rows")
     _f32(q_rows, shared_rows, latent_norm, freq)
     n = q_rows.shape[0]
     if q_rows.stride(1) != 1 or q_rows.shape[1] < heads * (d + dr):
@@ -1080,12 +1099,17 @@ def latent_prepare(q_rows, shared_rows, latent_norm, eps, freq, rot_dims, positi
     if not (q_plain.dtype == q_rotated.dtype == latent_pages.dtype == key_pages.dtype) or q_plain.numel() != heads * n * d \
             or q_rotated.numel() != n * heads * dr or latent_pages.shape[-1] != rank or key_pages.shape[-1] != dr:
         raise KernelError("latent_prepare: outputs and pages must have one element type and the parts' sizes")
+    if tuple(q_plain.shape) != (heads, n, d):
+        q_plain = q_plain.view(heads, n, d)
+    if q_rotated.dim() != 2 and tuple(q_rotated.shape) != (n, heads, dr):
+        q_rotated = q_rotated.view(n, heads * dr)
+    rotated_head = q_rotated.stride(1) if q_rotated.dim() == 3 else dr
     with _timed("latent_prepare"):
         _check(lib().lia_latent_prepare(_p(q_rows), q_rows.stride(0), _p(shared_rows),
                                         0 if shared_rows is None else shared_rows.stride(0),
                                         _p(latent_norm), float(eps), _p(freq), int(rot_dims), _p(positions), _p(slots),
-                                        _p(block_table), block_table.shape[1], _p(q_plain), _p(q_rotated),
-                                        _p(latent_pages), _p(key_pages), dtype_code(q_plain.dtype), n, heads, d, dr, rank,
+                                        _p(block_table), block_table.shape[1], _p(q_plain), q_plain.stride(0),
+                                        q_plain.stride(1), _p(q_rotated), rotated_head, q_rotated.stride(0), _p(latent_pages), _p(key_pages), dtype_code(q_plain.dtype), n, heads, d, dr, rank,
                                         latent_pages.shape[1], latent_pages.shape[0],
                                         1 if write_kv and shared_rows is not None else 0, 1 if pairs else 0,
                                         _p(error_flag), _stream()), "latent_prepare")
@@ -1176,25 +1200,60 @@ def latent_attention_accepts(rank: int, dr: int) -> bool:
     return bool(lib().lia_latent_attention_accepts(int(rank), int(dr)))
 
 
+def latent_gather(segments, n_segments, slots, block_table, latent_pages, part_pages, records, table, window, error_flag=None):
+    """The pages that a step's prompt portions see, side by side: records [pages, page_size, rank + dr] with
+    `table` [slots, blocks] saying where each block went; see csrc/latent_expand.cu.  `records` has room for every block
+    that the portions see."""
+    _cuda(segments, slots, block_table, latent_pages, part_pages, records, table, error_flag)
+    rank, dr = latent_pages.shape[-1], part_pages.shape[-1]
+    if not (latent_pages.dtype == part_pages.dtype == records.dtype == torch.bfloat16) or table.dtype != torch.int32:
+        raise KernelError("latent_gather takes bfloat16 pages and records and an int32 table")
+    if records.dim() != 3 or records.shape[1] != latent_pages.shape[1] or records.shape[2] != rank + dr or \
+            table.shape != block_table.shape or not records.is_contiguous() or not table.is_contiguous():
+        raise KernelError("latent_gather: records [pages, page_size, rank + dr], a table like the step's")
+    with _timed("latent_gather"):
+        _check(lib().lia_latent_gather(_p(segments), n_segments, _p(slots), _p(block_table), block_table.shape[1],
+                                       _p(latent_pages), _p(part_pages), _p(records), _p(table), records.shape[0], rank, dr,
+                                       latent_pages.shape[1], int(window or 0), latent_pages.shape[0], _p(error_flag), _stream()),
+               "latent_gather")
+
+
+def scatter_rows(src, index, dst):
+    """dst[index[r]] = src[r] for 2-D tensors of one element type and width; see csrc/elementwise.cu."""
+    _cuda(index)
+    if not (src.is_cuda and dst.is_cuda) or src.dim() != 2 or dst.dim() != 2 or src.dtype != dst.dtype \
+            or src.shape[1] != dst.shape[1] or src.stride(1) != 1 or dst.stride(1) != 1 or index.dtype != torch.int32 \
+            or index.numel() < src.shape[0]:
+        raise KernelError("scatter_rows: 2-D CUDA tensors of one type and width, int32 index of at least src's rows")
+    size = src.element_size()
+    with _timed("scatter_rows"):
+        _check(lib().lia_scatter_rows(_p(src), _p(index), _p(dst), src.shape[0], dst.shape[0], src.stride(0) * size,
+                                      dst.stride(0) * size, src.shape[1] * size, _stream()), "scatter_rows")
+
+
 def latent_attention(q1, q2, latent_pages, part_pages, positions, slots, block_table, out, heads, window, scale, splits=1,
-                     partial=None, error_flag=None, label=None, work_bytes=0, work_flops=0):
+                     partial=None, error_flag=None, label=None, work_bytes=0, work_flops=0, rows=None):
     """Attention in a latent's space on the tensor cores (bfloat16): q1 [heads, tokens, rank] with the latents, q2
-    [tokens, heads dr] with the rotated key parts, out [heads, tokens, rank]; see csrc/latent_attention_mma.cu.
+    [tokens, heads dr] (or a view [tokens, heads, dr]) with the rotated key parts, out [heads, tokens, rank]; see
+    csrc/latent_attention_mma.cu.  `rows` (int32 [tokens]): which of the step's `positions` and `slots` are the tokens'.
     `splits` > 1 cuts every token's keys into that many ranges; `partial` is their 32-bit scratch of
     splits * heads * tokens * (rank + 2) words."""
-    _cuda(q1, q2, latent_pages, part_pages, positions, slots, block_table, out, partial, error_flag)
+    _cuda(q1, latent_pages, part_pages, positions, slots, block_table, out, partial, error_flag, rows)
+    if not q2.is_cuda or q2.stride(-1) != 1 or (rows is not None and (rows.dtype != torch.int32 or rows.numel() < q2.shape[0])):
+        raise KernelError("latent_attention: q2 with contiguous rows, int32 rows for every token")
     if not (q1.dtype == q2.dtype == latent_pages.dtype == part_pages.dtype == out.dtype == torch.bfloat16):
         raise KernelError("latent_attention is a bfloat16 kernel")
     rank, dr = latent_pages.shape[-1], part_pages.shape[-1]
     n = q2.shape[0]
     splits = int(splits)
-    if tuple(q1.shape) != (heads, n, rank) or tuple(out.shape) != (heads, n, rank) or q2.shape[1] != heads * dr:
+    if tuple(q1.shape) != (heads, n, rank) or tuple(out.shape) != (heads, n, rank) or \
+            tuple(q2.shape) not in ((n, heads * dr), (n, heads, dr)):
         raise KernelError("latent_attention: q1 and out are [heads, tokens, rank], q2 [tokens, heads dr]")
     if splits > 1 and (partial is None or partial.dtype != torch.float32 or partial.numel() < splits * heads * n * (rank + 2)):
         raise KernelError("latent_attention: the ranges need 32-bit scratch of splits * heads * tokens * (rank + 2) words")
     with _timed("latent_attention", label, work_bytes, work_flops):
-        _check(lib().lia_latent_attention(_p(q1), _p(q2), _p(latent_pages), _p(part_pages), _p(positions), _p(slots),
-                                          _p(block_table), block_table.shape[1], _p(out), _p(partial) if splits > 1 else None,
+        _check(lib().lia_latent_attention(_p(q1), _p(q2), q2.stride(0), q2.stride(1) if q2.dim() == 3 else dr, _p(latent_pages),
+                                          _p(part_pages), _p(positions), _p(slots), _p(rows), _p(block_table), block_table.shape[1], _p(out), _p(partial) if splits > 1 else None,
                                           n, heads, rank, dr, latent_pages.shape[1], int(window or 0), scale,
                                           latent_pages.shape[0], splits, _p(error_flag), _stream()), "latent_attention")
 

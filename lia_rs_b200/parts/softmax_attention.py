@@ -217,7 +217,7 @@ class LatentAttention(Mixer):
              "k_up": "uk", "v_up": "uv", "gate": "g", "o": "o"}
 
     def graph_key(self, ctx) -> tuple:
-        return ()
+        return self._expansion(ctx) or ()
 
     @staticmethod
     def _names(params, prefix):
@@ -273,10 +273,11 @@ class LatentAttention(Mixer):
         self.gate_span = int(params["v_head_dim"]) if params.get("gate") == "sigmoid_head" else 1
         n = self._names(params, prefix)
         H, d, dv, rank = self.heads, self.d, self.dv, self.rank
-        # One product for everything that is read from the input beside a query latent: [W_q (queries straight from the
+        # One product for everything that is read from the input: [W_dq (a query latent) or W_q (queries straight from the
         # input) | W_dkv (a cache of the layer's own) | W_g (a gate)], padded with zero rows to a multiple of 8 columns.
         blocks, at, self.columns = [], 0, {}
-        for key, present, rows in (("q", self.q_rank is None, H * (d + self.dr)), ("kv_down", self.own_cache, rank + self.dr),
+        for key, present, rows in (("q_down", self.q_rank is not None, self.q_rank), ("q", self.q_rank is None, H * (d + self.dr)),
+                                   ("kv_down", self.own_cache, rank + self.dr),
                                    ("gate", self.gated, H * dv // self.gate_span)):
             if present:
                 blocks.append(tensors[n[key]])
@@ -285,9 +286,8 @@ class LatentAttention(Mixer):
         self.in_width = (at + 7) // 8 * 8
         if self.in_width > at:
             blocks.append(torch.zeros((self.in_width - at, self.hidden), dtype=blocks[0].dtype, device=blocks[0].device))
-        self.w_in = prepare_weight(torch.cat(blocks, dim=0), runtime) if at else None
+        self.w_in = prepare_weight(torch.cat(blocks, dim=0), runtime)
         if self.q_rank is not None:
-            self.w_q_down = prepare_weight(tensors[n["q_down"]], runtime)
             self.w_q_up = prepare_weight(tensors[n["q_up"]], runtime)
             norm_params = {"hidden": self.q_rank, "eps": self.eps, "tensor": ""}
             self.q_norm = lookup(NORMS, "rmsnorm", "norm")(norm_params, {n["q_norm"]: tensors[n["q_norm"]]}, n["q_norm"], runtime)
@@ -298,6 +298,91 @@ class LatentAttention(Mixer):
         self.kv_norm = tensors[n["kv_norm"]].to(torch.float32).contiguous() if self.own_cache else None
         self.rot_dims, self.freq = _frequencies(params.get("rot"), runtime.device)
         self.tensor_cores = runtime.compute_dtype == torch.bfloat16 and ops.latent_attention_accepts(self.rank, self.dr)
+        # prompt portions on the tensor cores: a record [latent | rotated part] times w_expand gives every head's whole key
+        # (the unit matrix behind a head's share of the key expansion hands the rotated part through unchanged) and value
+        self.per_tile = ops.attention_prefill_tc_tokens_per_tile(1, d + self.dr, dv) if self.tensor_cores and d % 8 == 0 else 0
+        if self.per_tile:
+            # (keys of all heads, then values of all heads)
+            self.w_expand = torch.zeros((H * (d + self.dr + dv), rank + self.dr), dtype=self.w_v_up.dtype, device=self.w_v_up.device)
+            w_keys = self.w_expand[:H * (d + self.dr)].view(H, d + self.dr, rank + self.dr)
+            w_keys[:, :d, :rank] = tensors[n["k_up"]].view(H, d, rank)
+            w_keys[:, d:, rank:] = torch.eye(self.dr, dtype=w_keys.dtype, device=w_keys.device)
+            self.w_expand[H * (d + self.dr):, :rank] = self.w_v_up.view(H * dv, rank)
+
+    EXPAND_FROM = 16                  # tokens a portion, on average, from which the records are expanded
+    EXPAND_BYTES = 1 << 30            # most memory that the expanded keys and values of one step may take
+
+    def _expansion(self, ctx):
+        """How a step's prompt portions attend: (pages whose records are expanded into whole keys and values, tiles of the
+        prompt kernel), or None where the portions stay in the latent's space.  The pages are those that the portions see,
+        rounded up to four significant bits, so that a captured step serves its neighbours.
+
+        In the latent's space a pair of query and key costs 2 rank + dr multiply-adds a head on `mma.sync`, expanded d + dr + dv
+        on tcgen05 (1,088 against 320 at 2B-widths) beside the expansion's d + dr + dv products of length rank a key and head,
+        whatever the number of queries: 2,048 tokens over themselves took 796 us beside 2 x 127 us for the queries' and the
+        outputs' way into that space and back."""
+        if not ctx.n_prefill_segments or not self.per_tile:
+            return None
+        size = ctx.runtime.cache.page_size
+        pages = tiles = tokens = 0
+        for _, start, count, _ in ctx.segments:
+            if count > 1:
+                first = max(0, start - self.window + 1) if self.window else 0
+                pages += (start + count - 1) // size - first // size + 1
+                tiles += (count + self.per_tile - 1) // self.per_tile
+                tokens += count
+        step = 1 << max(0, pages.bit_length() - 4)
+        pages = (pages + step - 1) // step * step
+        if tokens < self.EXPAND_FROM * ctx.n_prefill_segments or \
+                pages * size * self.heads * (self.d + self.dr + self.dv) * 2 > self.EXPAND_BYTES:
+            return None
+        return pages, tiles
+
+    def _attend_expanded(self, ctx, plan, q, kv, out, gate):
+        """out [tokens, heads dv] = attention of the step's prompt portions, queries q [tokens, heads, d + dr], times its gate."""
+        rt, (pages, tiles) = self.runtime, plan
+        H, d, dr, dv, rank = self.heads, self.d, self.dr, self.dv, self.rank
+        n, size, flag = q.shape[0], kv.page_size, ctx.error_flag
+        scratch = ctx.runtime.scratch
+        records = scratch("latent.records", pages * size * (rank + dr), torch.bfloat16).view(pages * size, rank + dr)
+        table = scratch("latent.table", kv.block_table.numel(), torch.int32).view(kv.block_table.shape)
+        ops.latent_gather(ctx.prefill_segments, ctx.n_prefill_segments, ctx.slots, kv.block_table, kv.k_pages, kv.v_pages,
+                          records.view(pages, size, rank + dr), table, self.window, error_flag=flag)
+        width = H * (d + dr + dv)
+        expanded = scratch("latent.expanded", pages * size * width, torch.bfloat16).view(pages * size, width)
+        linear(rt, STORE, records, self.w_expand, expanded, error_flag=flag, name="expand")
+        paged = expanded.view(pages, size, width)
+        keys, values = paged[:, :, :H * (d + dr)].unflatten(2, (H, d + dr)), paged[:, :, H * (d + dr):].unflatten(2, (H, dv))
+        longest = min(ctx.context_bucket, self.window + self.per_tile if self.window else ctx.context_bucket)
+        splits = max(1, min(ctx.runtime.sm_count // (tiles * H), 16, longest // 512))
+        more = {}
+        if splits > 1:
+            words = ops.attention_prefill_tc_partial_floats(n, H, dv, splits)
+            more = dict(splits=splits, partial=scratch("attn.prefill_partial", words, torch.float32))
+        ops.attention_prefill_tc(q.view(n, H * (d + dr)), keys, values, ctx.prefill_segments, ctx.n_prefill_segments, tiles,
+                                 ctx.slots, table, out, H, H, d + dr, self.window, self.scale, flag,
+                                 work_flops=self._work(ctx)[1], gate=gate, gate_head=self.gate_span > 1, **more)
+
+    def _attend_in_latent(self, ctx, q_plain, q_rotated, kv, out, rows=None):
+        """out [tokens, heads, dv] (any strides) = attention in the latent's space of the tokens whose queries these are, q_plain
+        [heads, tokens, d] and q_rotated [tokens, heads dr] or [tokens, heads, dr]; `rows`: which of the step's tokens they are."""
+        H, n, rank, dtype = self.heads, q_plain.shape[1], self.rank, self.runtime.compute_dtype
+        scratch = ctx.runtime.scratch
+        q_absorbed = scratch("latent.q_absorbed", H * n * rank, dtype).view(H, n, rank)
+        self._head_products(ctx, q_plain, self.w_k_up_t, q_absorbed, "k_up")
+        mixed = scratch("latent.mixed", H * n * rank, dtype).view(H, n, rank)
+        if self.tensor_cores:
+            splits = self._splits(ctx, n)
+            partial = scratch("latent.partial", splits * H * n * (rank + 2), torch.float32) if splits > 1 else None
+            work_bytes, work_flops = self._work(ctx)
+            ops.latent_attention(q_absorbed, q_rotated, kv.k_pages, kv.v_pages, ctx.positions, ctx.slots, kv.block_table,
+                                 mixed, H, self.window, self.scale, splits=splits, partial=partial, error_flag=ctx.error_flag,
+                                 work_bytes=work_bytes, work_flops=0 if rows is not None else work_flops, rows=rows)
+        else:
+            ops.attention_general(q_absorbed, (rank, n * rank), q_rotated, (H * self.dr, self.dr), kv.k_pages, kv.v_pages, kv.k_pages,
+                                  rank, rank, ctx.positions, ctx.slots, kv.block_table, mixed, (rank, n * rank), n, H, 1,
+                                  self.window, self.scale, sink=False, error_flag=ctx.error_flag)
+        self._head_products(ctx, mixed, self.w_v_up, out.transpose(0, 1), "v_up")
 
     def _splits(self, ctx, n: int) -> int:
         """Into how many ranges the tensor-core kernel cuts each token's keys: as many as give every SM two CTAs, none
@@ -331,42 +416,47 @@ class LatentAttention(Mixer):
         rt, n = self.runtime, x.shape[0]
         H, d, dr, dv, rank = self.heads, self.d, self.dr, self.dv, self.rank
         flag, dtype = ctx.error_flag, rt.compute_dtype
-        shared = gate = None
-        if self.w_in is not None:
-            rows = ctx.buffer("latent.in", (n, self.in_width), torch.float32)
-            linear(rt, STORE, x, self.w_in, rows, error_flag=flag, name="latent_in")
-            part = lambda key: rows[:, self.columns[key][0]:self.columns[key][1]] if key in self.columns else None
-            shared, gate = part("kv_down"), part("gate")
+        rows = ctx.buffer("latent.in", (n, self.in_width), torch.float32)
+        linear(rt, STORE, x, self.w_in, rows, error_flag=flag, name="latent_in")
+        part = lambda key: rows[:, self.columns[key][0]:self.columns[key][1]] if key in self.columns else None
+        shared, gate = part("kv_down"), part("gate")
         if self.q_rank is None:
             q_rows = part("q")
         else:
-            q_latent = ctx.buffer("latent.cq", (n, self.q_rank), torch.float32)
-            linear(rt, STORE, x, self.w_q_down, q_latent, error_flag=flag, name="q_down")
             q_rows = ctx.buffer("latent.q", (n, H * (d + dr)), torch.float32)
-            linear(rt, STORE, DeferredNorm(ctx, self.q_norm, q_latent, buffer_name="latent.cq_normed"), self.w_q_up, q_rows,
+            linear(rt, STORE, DeferredNorm(ctx, self.q_norm, part("q_down"), buffer_name="latent.cq_normed"), self.w_q_up, q_rows,
                    error_flag=flag, name="q_up")
         scratch = ctx.runtime.scratch
-        q_plain = scratch("latent.q_plain", H * n * d, dtype).view(H, n, d)
-        q_rotated = ctx.buffer("latent.q_rot", (n, H * dr), dtype)
+        plan = self._expansion(ctx)
+        if plan is None:
+            q_plain = scratch("latent.q_plain", H * n * d, dtype).view(H, n, d)
+            q_rotated = ctx.buffer("latent.q_rot", (n, H * dr), dtype)
+        else:
+            q = ctx.buffer("latent.q_whole", (n, H * (d + dr)), dtype)
+            heads = q.view(n, H, d + dr)
+            q_plain, q_rotated = heads[:, :, :d].transpose(0, 1), heads[:, :, d:]
         ops.latent_prepare(q_rows, shared, self.kv_norm, self.eps, self.freq, self.rot_dims, ctx.positions, ctx.slots,
                            kv.block_table, q_plain, q_rotated, kv.k_pages, kv.v_pages, H, d, dr, rank,
                            write_kv=kv.writes and self.own_cache, error_flag=flag, pairs=self.pairs)
-        q_absorbed = scratch("latent.q_absorbed", H * n * rank, dtype).view(H, n, rank)
-        self._head_products(ctx, q_plain, self.w_k_up_t, q_absorbed, "k_up")
-        mixed = scratch("latent.mixed", H * n * rank, dtype).view(H, n, rank)
-        if self.tensor_cores:
-            splits = self._splits(ctx, n)
-            partial = scratch("latent.partial", splits * H * n * (rank + 2), torch.float32) if splits > 1 else None
-            work_bytes, work_flops = self._work(ctx)
-            ops.latent_attention(q_absorbed, q_rotated, kv.k_pages, kv.v_pages, ctx.positions, ctx.slots, kv.block_table,
-                                 mixed, H, self.window, self.scale, splits=splits, partial=partial, error_flag=flag,
-                                 work_bytes=work_bytes, work_flops=work_flops)
-        else:
-            ops.attention_general(q_absorbed, (rank, n * rank), q_rotated, (H * dr, dr), kv.k_pages, kv.v_pages, kv.k_pages,
-                                  rank, rank, ctx.positions, ctx.slots, kv.block_table, mixed, (rank, n * rank), n, H, 1,
-                                  self.window, self.scale, sink=False, error_flag=flag)
         o = ctx.buffer("latent.o", (n, H * dv), dtype)
-        self._head_products(ctx, mixed, self.w_v_up, o.view(n, H, dv).transpose(0, 1), "v_up")
-        if gate is not None:
+        if plan is None:
+            self._attend_in_latent(ctx, q_plain, q_rotated, kv, o.view(n, H, dv))
+        else:
+            self._attend_expanded(ctx, plan, heads, kv, o, gate)
+            if ctx.n_single:
+                # the step's single tokens attend in the latent's space, side by side in buffers of their own
+                singles, rows = ctx.n_single, ctx.decode_rows
+                q_singles = scratch("latent.q_singles", singles * H * (d + dr), dtype).view(singles, H * (d + dr))
+                ops.gather_rows(q, rows, q_singles)
+                apart = q_singles.view(singles, H, d + dr)
+                o_singles = scratch("latent.o_singles", singles * H * dv, dtype).view(singles, H * dv)
+                self._attend_in_latent(ctx, apart[:, :, :d].transpose(0, 1), apart[:, :, d:], kv, o_singles.view(singles, H, dv),
+                                       rows=rows)
+                if gate is not None:
+                    gate_singles = scratch("latent.gate_singles", singles * gate.shape[1], torch.float32).view(singles, gate.shape[1])
+                    ops.gather_rows(gate, rows, gate_singles)
+                    ops.gate_rows(o_singles, gate_singles, ops.GATE_SIGMOID, span=self.gate_span)
+                ops.scatter_rows(o_singles, rows, o)
+        if plan is None and gate is not None:
             ops.gate_rows(o, gate, ops.GATE_SIGMOID, span=self.gate_span)
         linear(rt, STORE if store else ACCUM, o, self.w_o, residual, scale, error_flag=flag, name="o")

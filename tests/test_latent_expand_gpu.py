@@ -1,0 +1,91 @@
+"""Attention through a latent whose prompt portions are expanded into whole keys and values: portions around the tiles' and
+pages' edges, late in their prompts, windows, gates, and single tokens in the same step, against the plain functions in 64-bit."""
+import pytest
+import torch
+
+import plain_vatunex as pv
+import plain_zipelix as pz
+from test_botuvik_parts_gpu import PartRunner
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+# eight values are rounded to bfloat16 on the way (queries, latents, keys, values, probabilities, outputs and the two products'
+# operands), each by at most 2^-9 of itself, and the result is linear in each: 8 * 2^-9 of its size at most, in any norm
+REL = 8 * 2.0 ** -9
+
+
+def tensors(hidden, m, form, g):
+    H, d, dr, dv, rank = m["heads"], m["dim"], m["rot_dim"], m["vdim"], m["kv_rank"]
+    shapes = {"dkv": (rank + dr, hidden), "uk": (H * d, rank), "uv": (H * dv, rank), "o": (hidden, H * dv)}
+    if form == "windowed":
+        shapes.update({"dq": (64, hidden), "uq": (H * (d + dr), 64)})
+    else:
+        shapes.update({"q": (H * (d + dr), hidden), "g": (H * dv, hidden)})
+    w = {name: (torch.randn(*shape, generator=g) * shape[1] ** -0.5).to(torch.bfloat16) for name, shape in shapes.items()}
+    w["dkv.norm"] = (1 + 0.1 * torch.randn(rank, generator=g)).to(torch.bfloat16)
+    if form == "windowed":
+        w["dq.norm"] = (1 + 0.1 * torch.randn(64, generator=g)).to(torch.bfloat16)
+    return w
+
+
+@pytest.mark.parametrize("d,dr,dv,rank,page", [(128, 64, 128, 512, 16), (64, 32, 64, 256, 16), (64, 64, 64, 32, 5), (32, 32, 128, 96, 8)])
+@pytest.mark.parametrize("form", ["gated", "windowed"])
+def test_expanded_portions_against_plain_functions(d, dr, dv, rank, page, form):
+    g = torch.Generator().manual_seed(d + rank)
+    hidden, heads = 96, 3
+    m = dict(heads=heads, dim=d, rot_dim=dr, vdim=dv, kv_rank=rank, scale=(d + dr) ** -0.5, rot={"base": 100.0, "dims": dr})
+    if form == "windowed":
+        m["mask"] = {"size": 70}
+    w = tensors(hidden, m, form, g)
+    params = dict(hidden=hidden, heads=heads, head_dim=d, rot_dim=dr, v_head_dim=dv, kv_rank=rank, scale=m["scale"], norm_eps=1e-5,
+                  rot=m["rot"], **(dict(q_rank=None, gate="sigmoid", rot_pairs=True) if form == "gated" else
+                                   dict(q_rank=64, window=70)))
+    runner = PartRunner("latent_attention", params, w, "bfloat16", page_size=page, slots=4, tokens=1024)
+    part = runner.part
+    assert part.per_tile == 128
+    lengths = {"a": 420, "b": 257, "c": 140, "e": 40}
+    rows = {name: torch.randn(n, hidden, generator=g).to(torch.bfloat16).float() for name, n in lengths.items()}
+    # whole tiles and their neighbours, portions late in a prompt, single tokens beside portions and alone
+    steps = [[("a", 128), ("b", 129)], [("a", 127), ("c", 17), ("b", 1)], [("a", 1), ("b", 1)], [("a", 2), ("b", 33), ("c", 121), ("e", 20)],
+             [("a", 162), ("b", 1), ("e", 18), ("c", 1)], [("b", 92), ("c", 1), ("e", 2)]]
+    got = {name: [] for name in lengths}
+    for entries in steps:
+        for name, out in runner.step(entries, rows).items():
+            got[name].append(out)
+    for name, length in lengths.items():
+        h, positions = rows[name].to(F64), torch.arange(length)
+        if form == "gated":
+            cache = pz.latent_cache(h, positions, w["dkv"], w["dkv.norm"], m, 1e-5)
+            want = pz.latent_attention(h, positions, w, m, cache)
+        else:
+            want = pv.latent_attention(m, lambda key: w[key].to(F64), h, positions, 1e-5)
+        out = torch.cat(got[name])
+        assert out.shape == want.shape
+        assert float((out - want).norm() / want.norm()) < REL, (name, float((out - want).norm() / want.norm()))
+        assert float((out - want).norm(dim=-1).max() / want.norm(dim=-1).max()) < 2 * REL
+
+
+def test_which_portions_are_expanded():
+    """The rule looks at the portions alone: long enough on average and not beyond the memory it may take; the pages it names
+    cover what the portions see, rounded up by less than an eighth."""
+    from types import SimpleNamespace
+    params = dict(hidden=96, heads=2, head_dim=64, rot_dim=32, v_head_dim=64, kv_rank=32, scale=0.1, rot=None, q_rank=None)
+    g = torch.Generator().manual_seed(1)
+    m = dict(heads=2, dim=64, rot_dim=32, vdim=64, kv_rank=32)
+    w = tensors(96, m, "gated", g)
+    w.pop("g")
+    part = PartRunner("latent_attention", params, w, "bfloat16", page_size=16, slots=2, tokens=64).part
+
+    def plan(segments, page_size=16):
+        portions = sum(1 for _, _, count, _ in segments if count > 1)
+        return part._expansion(SimpleNamespace(n_prefill_segments=portions, segments=segments,
+                                               runtime=SimpleNamespace(cache=SimpleNamespace(page_size=page_size))))
+
+    assert plan([(0, 5, 1, 0)]) is None
+    assert plan([(0, 0, 15, 0)]) is None and plan([(0, 0, 16, 0)]) == (1, 1)
+    assert plan([(0, 0, 2048, 0), (1, 7, 1, 2048)]) == (128, 16)
+    for last in range(17, 3000, 41):
+        pages, tiles = plan([(0, last - 17, 17, 0), (1, 0, 130, 17)])
+        seen = (last + 15) // 16 + 9
+        assert seen <= pages < seen * 9 / 8 + 1 and tiles == 3
+    assert plan([(0, 1 << 24, 64, 0)]) is None
