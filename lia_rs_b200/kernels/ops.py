@@ -47,6 +47,9 @@ class _Signatures:
                      c_int, c_int, c_float, c_void_p]
     lia_attention_generic = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p]
+    lia_attention_prefill_f32 = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int,
+                                 c_int, c_int, c_float, c_int, c_void_p, c_void_p]
+    lia_attention_prefill_f32_tokens_per_tile = [c_int, c_int]
     lia_gather_rows = [c_void_p, c_void_p, c_void_p, c_int, c_int, ctypes.c_longlong, ctypes.c_longlong,
                        ctypes.c_longlong, c_void_p]
     lia_wait_probe = [c_int, c_void_p, c_void_p, c_void_p]
@@ -668,6 +671,24 @@ def attention_prefill(q, k_pages, v_pages, segments, n_segments, n_tiles, slots,
                                            _p(slots), _p(block_table), block_table.shape[1], _p(out), nq, nkv, d,
                                            k_pages.shape[1], int(window or 0), scale, k_pages.shape[0], 1 if sink else 0,
                                            _p(error_flag), _stream()), "attention_prefill")
+
+
+def attention_prefill_f32_tokens_per_tile(group: int, d: int) -> int:
+    """Tokens of a portion that one CTA of the 32-bit prompt kernel takes (0: it does not take this group or head size)."""
+    return int(lib().lia_attention_prefill_f32_tokens_per_tile(group, d))
+
+
+def attention_prefill_f32(q, k_pages, v_pages, segments, n_segments, n_tiles, slots, block_table, out, nq, nkv, d, scale,
+                          error_flag=None, label=None, work_flops=0):
+    """Prompt-portion attention of the 32-bit path over all visible keys, bit for bit what `attention_generic` gives; see
+    csrc/attention_prefill_f32.cu.  Arguments as `attention_prefill`."""
+    _cuda(q, k_pages, v_pages, segments, slots, block_table, out, error_flag)
+    if not (q.dtype == k_pages.dtype == v_pages.dtype == out.dtype == torch.float32):
+        raise KernelError("attention_prefill_f32 is a 32-bit kernel")
+    with _timed("attention_prefill_f32", label, 0, work_flops):
+        _check(lib().lia_attention_prefill_f32(_p(q), _p(k_pages), _p(v_pages), _p(segments), n_segments, n_tiles, _p(slots),
+                                               _p(block_table), block_table.shape[1], _p(out), nq, nkv, d, k_pages.shape[1], scale,
+                                               k_pages.shape[0], _p(error_flag), _stream()), "attention_prefill_f32")
 
 
 def attention_prefill_tc_tokens_per_tile(group: int, d: int, dv: int = None) -> int:

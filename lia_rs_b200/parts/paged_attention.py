@@ -11,7 +11,9 @@ once, and an unsupported size is refused there with its reason.  The kernels (cs
   (`ops.DECODE_HEAD_PAIRS`), and the kernel with a size for each (`ops.attention_general`) what they do not take;
 
   variant "generic"  everything else: the 32-bit path, and bfloat16 with another head size
-                     (attention_generic.cu: a warp per token and head, 32-bit probabilities).  On the bfloat16
+                     (attention_generic.cu: a warp per token and head, 32-bit probabilities; the 32-bit path's prompt
+                     portions without a window, at head sizes 32, 64, 96 and 128 and up to 64 query heads a kv head, go
+                     through attention_prefill_f32.cu, which forms the same numbers 64 rows at a time).  On the bfloat16
                      path this is a slow road, so it is said once when such a mixer is built.
 
 Head sizes are multiples of 16 up to 256 (what attention_generic.cu takes); `check` refuses others.
@@ -61,7 +63,7 @@ class PagedAttention:
         self.dv = self.d if v_head_dim is None else int(v_head_dim)
         if self.dv != self.d and (dtype != torch.bfloat16 or not self.takes(self.d, self.dv, self.nq // self.nkv)):
             raise ValueError("attention: keys and values of unequal head sizes that no tensor-core kernel behind this class takes")
-        self.window, self.scale = window, float(scale)
+        self.window, self.scale, self.dtype = window, float(scale), dtype
         self.group = self.nq // self.nkv
         self.variant = "tensor" if dtype == torch.bfloat16 and self.d in ops.DECODE_HEAD_DIMS else "generic"
         if (self.sink or self.softcap) and (self.variant != "tensor" or self.nq // self.nkv > 64):
@@ -132,6 +134,11 @@ class PagedAttention:
 
     def _prefill_kernel(self):
         """(kernel, tokens per tile) for prompt portions, asked of the library once."""
+        if self._prefill is None and self.variant == "generic":
+            # the 32-bit path's prompt kernel sees all keys (a window's walk begins at a place of the row's own)
+            per_tile = (ops.attention_prefill_f32_tokens_per_tile(self.group, self.d)
+                        if self.dtype == torch.float32 and not self.window and self.dv == self.d else 0)
+            self._prefill = (ops.attention_prefill_f32 if per_tile else None, per_tile)
         if self._prefill is None:
             per_tile = ops.attention_prefill_tc_tokens_per_tile(self.group, self.d, self.dv)
             if per_tile:
@@ -146,7 +153,7 @@ class PagedAttention:
         """What of a step's shape the launches below depend on beyond the numbers of tokens, single-token entries and
         portions and the context bucket: into how many tiles the prompt kernel cuts the portions.  (Where the
         portions begin and how long each is, the kernels read on the device.)"""
-        if self.variant != "tensor" or not ctx.n_prefill_segments:
+        if not ctx.n_prefill_segments:
             return ()
         per_tile = self._prefill_kernel()[1]
         if not per_tile:
@@ -172,8 +179,17 @@ class PagedAttention:
             return
         work_bytes, work_flops = self._work(ctx, q.element_size())
         if self.variant == "generic":
+            rows = None
+            if ctx.n_prefill_segments and self._prefill_kernel()[1]:
+                kernel, per_tile = self._prefill_kernel()
+                tiles = sum((count + per_tile - 1) // per_tile for _, _, count, _ in ctx.segments if count > 1)
+                kernel(q, kv.k_pages, kv.v_pages, ctx.prefill_segments, ctx.n_prefill_segments, tiles, ctx.slots, kv.block_table, out,
+                       nq, nkv, d, self.scale, error_flag=ctx.error_flag, work_flops=work_flops)
+                if not ctx.decode_rows.numel():
+                    return
+                rows = ctx.decode_rows
             ops.attention_generic(q, kv.k_pages, kv.v_pages, ctx.positions, ctx.slots, kv.block_table, out, nq, nkv, d,
-                                  self.window, self.scale, error_flag=ctx.error_flag, work_bytes=work_bytes)
+                                  self.window, self.scale, rows=rows, error_flag=ctx.error_flag, work_bytes=work_bytes)
             return
         if ctx.decode_rows.numel():
             self._decode(ctx, q, kv, out, ctx.decode_rows, ctx.decode_rows.numel(), work_bytes)
