@@ -27,6 +27,7 @@
 // Kernels launched by this library since it was loaded (every launcher calls lia_check_launch once per
 // kernel).  Read through lia_kernel_launches(); a benchmark's own count of its launches.
 #include <atomic>
+#include <utility>
 inline std::atomic<long long> lia_launch_counter{0};
 
 static inline int lia_check_launch() {
@@ -46,8 +47,8 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 inline std::atomic<int> lia_pdl_enabled{1};
 
 template <typename... KArgs, typename... Args>
-static inline int lia_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                             Args&&... args) {
+static inline int lia_launch_with(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                  Args&&... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
@@ -57,13 +58,25 @@ static inline int lia_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attribute[0].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attribute;
-    config.numAttrs = lia_pdl_enabled.load(std::memory_order_relaxed) ? 1 : 0;
+    config.numAttrs = early && lia_pdl_enabled.load(std::memory_order_relaxed) ? 1 : 0;
     lia_launch_counter.fetch_add(1, std::memory_order_relaxed);
     if (cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...) != cudaSuccess) {
         cudaGetLastError();
         return LIA_ERR_LAUNCH;
     }
     return cudaGetLastError() == cudaSuccess ? LIA_OK : LIA_ERR_LAUNCH;
+}
+
+template <typename... KArgs, typename... Args>
+static inline int lia_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    return lia_launch_with(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+}
+
+// The ordinary way, behind the end of the kernel ahead: for a kernel of many small CTAs that live long.  CTAs are placed when they
+// begin, and those that begin early only find the SMs that the kernel ahead leaves free.
+template <typename... KArgs, typename... Args>
+static inline int lia_launch_in_turn(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    return lia_launch_with(false, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 // Row of the paged cache [pages * page_size] that holds position `key` of a request whose block-table row is

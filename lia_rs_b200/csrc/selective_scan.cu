@@ -14,10 +14,13 @@
 //    keeping up to 8 states in registers (up to 256 states).
 //
 // A row whose slot is negative belongs to nobody and is skipped.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
 constexpr int MAX_TAPS = 8;
+constexpr int CONV_TILED_FROM = 64;    // rows of a step from which eight of them share a thread's window
 
 // how many of the rows just before row t continue the same run (at most `most`)
 __device__ __forceinline__ int run_before(const int* __restrict__ positions, const int* __restrict__ slots, int t,
@@ -69,6 +72,85 @@ __global__ void causal_conv_kernel(const float* __restrict__ x, long long ld, co
 #pragma unroll
             for (int i = 0; i < MAX_TAPS - 1; ++i)
                 if (i < taps - 1) mine[(size_t)i * channels + c] = kept[i];
+        }
+    }
+}
+
+// The same convolution for many tokens: a thread owns four channels of CONV_ROWS neighbouring rows, asks for all of them at once
+// and shifts the window of earlier inputs along; only the tile's first row, and a row that begins a run, look further back (into
+// the rows before the tile, or the slot's state).  The sums are those of the kernel above, term by term.  Bound by memory: 2,048
+// rows of 4,096 channels read 33 MB and write 50 (32-bit and bfloat16).
+constexpr int CONV_ROWS = 8, CONV_THREADS = 128;
+
+template <typename TO, int TAPS>
+__global__ void __launch_bounds__(CONV_THREADS)
+causal_conv_tile_kernel(const float* __restrict__ x, long long ld, const float* __restrict__ taps_weight,
+                        const float* __restrict__ bias, const float* __restrict__ state, long long state_stride,
+                        const int* __restrict__ positions, const int* __restrict__ slots, float* __restrict__ out,
+                        TO* __restrict__ out_copy, int n_tokens, int channels, int act) {
+    const int c = (blockIdx.x * CONV_THREADS + threadIdx.x) * 4;
+    float w[4][TAPS], b[4];
+    if (c < channels) {                                            // (weights wait for no one)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            b[i] = bias ? bias[c + i] : 0.f;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) w[i][j] = taps_weight[(size_t)(c + i) * TAPS + j];
+        }
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+    if (c >= channels) return;
+    const int t0 = blockIdx.y * CONV_ROWS, rows = min(CONV_ROWS, n_tokens - t0);
+    float4 v[CONV_ROWS];
+    int slot[CONV_ROWS], pos[CONV_ROWS];
+#pragma unroll
+    for (int r = 0; r < CONV_ROWS; ++r) {
+        const int t = min(t0 + r, n_tokens - 1);
+        v[r] = __ldg(reinterpret_cast<const float4*>(x + (size_t)t * ld + c));
+        slot[r] = slots[t];
+        pos[r] = positions[t];
+    }
+    float before[TAPS][4];                                         // [k]: the input k rows back (k >= 1)
+#pragma unroll
+    for (int r = 0; r < CONV_ROWS; ++r) {
+        if (r >= rows) break;
+        const int t = t0 + r;
+        const float now[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
+        if (slot[r] >= 0) {
+            const bool goes_on = r > 0 && slot[r > 0 ? r - 1 : 0] == slot[r] && pos[r > 0 ? r - 1 : 0] == pos[r] - 1;
+            if (!goes_on && TAPS > 1) {
+                const int m = run_before(positions, slots, t, slot[r], pos[r], TAPS - 1);
+                const float* own = state + (size_t)slot[r] * state_stride;
+#pragma unroll
+                for (int k = 1; k < TAPS; ++k)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) before[k][i] = input_before(x, ld, own, channels, TAPS, t, pos[r], m, k, c + i);
+            }
+            float y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                y[i] = b[i];
+#pragma unroll
+                for (int j = 0; j < TAPS - 1; ++j) y[i] = fmaf(w[i][j], before[TAPS - 1 - j][i], y[i]);
+                y[i] = fmaf(w[i][TAPS - 1], now[i], y[i]);
+                if (act == 1) y[i] = y[i] / (1.0f + expf(-y[i]));
+            }
+            *reinterpret_cast<float4*>(out + (size_t)t * channels + c) = make_float4(y[0], y[1], y[2], y[3]);
+            if (out_copy) {
+                struct alignas(4 * sizeof(TO)) Four { TO v[4]; } f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) f.v[i] = from_float<TO>(y[i]);
+                *reinterpret_cast<Four*>(out_copy + (size_t)t * channels + c) = f;
+            }
+        }
+#pragma unroll
+        for (int k = TAPS - 1; k > 1; --k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) before[k][i] = before[k - 1][i];
+        if (TAPS > 1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) before[1][i] = now[i];
         }
     }
 }
@@ -280,6 +362,189 @@ scan_carry_kernel(ScanArgs p) {
         if (n < p.states) own[n] = S[i];
     }
 }
+// Whole portions of up to 64 states a channel, walked once: sixteen lanes own a channel, SPL neighbouring states each, and a CTA
+// eight channels of one portion.  The rows of 32 tokens (x, step size, gate of the eight channels, B and C of all states) lie in
+// shared memory and the next 32 are on their way.  Every lane forms the step sizes of every sixteenth token, side by side, and
+// hands them round through shared memory; behind a group of sixteen tokens' recurrence (per state: an exponential, two
+// multiply-adds) the sixteen sums over the lanes' states meet so that every lane is left with one token's, whose skip, gate and
+// store are its own: what is not the recurrence is done once per token and channel.
+// A token costs its exponentials: 2,048 tokens x 4,096 channels x 16 states are 134 M, 40 us of issue over the device with the
+// multiply-adds around them.  Cutting the portions into chunks (below, for other sizes) does each of them twice, and one that
+// reads B and C from memory per thread spends more on the loads: 539 us for the same tokens.
+// With `conv_state` the CTA also leaves its channels' last taps - 1 inputs there (the convolution has long read them).
+constexpr int RUN_CHANNELS = 8, RUN_LANES = 16, RUN_TOKENS = 32, RUN_THREADS = RUN_CHANNELS * RUN_LANES;
+
+struct ConvTail {
+    float* state; long long state_stride;           // null: nothing to leave
+    const float* x; long long ld; int taps;
+};
+
+template <typename TO, int SPL>
+__global__ void __launch_bounds__(RUN_THREADS)
+scan_run_kernel(ScanArgs p, ConvTail tail) {
+    constexpr int GROUP = RUN_LANES, GROUPS = RUN_TOKENS / GROUP;         // a token of a group a lane
+    struct __align__(16) Stage {
+        float x[RUN_TOKENS][RUN_CHANNELS], dt[RUN_TOKENS][RUN_CHANNELS], z[RUN_TOKENS][RUN_CHANNELS];
+        float bc[RUN_TOKENS][RUN_LANES][2 * SPL];            // a lane's B and then its C
+    };
+    __shared__ Stage stages[2];
+    __shared__ __align__(16) float steps[RUN_CHANNELS][RUN_TOKENS][2];       // step size, step size times input
+    __shared__ __align__(16) TO results[RUN_TOKENS][RUN_CHANNELS];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int first = p.segments[3 * blockIdx.y], start = p.segments[3 * blockIdx.y + 1], count = p.segments[3 * blockIdx.y + 2];
+    if (first < 0 || count <= 0) return;
+    const int slot = p.slots[first];
+    if (slot < 0) return;
+    const int tid = threadIdx.x, lane = tid % RUN_LANES, ch = tid / RUN_LANES, c0 = blockIdx.x * RUN_CHANNELS, c = c0 + ch;
+    const int states = p.states;
+    // (channels and states are multiples of four: a piece of four lies inside or outside)
+    auto fetch = [&](int t0, int buffer) {
+        Stage& s = stages[buffer];
+        auto bring = [&](float* dst, const float* src, bool there) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                         "r"(there ? 16 : 0) : "memory");
+        };
+        if (tid < 2 * RUN_TOKENS) {
+            const int r = tid >> 1, piece = (tid & 1) * 4;
+            const bool there = t0 + r < count && c0 + piece < p.channels;
+            const size_t t = (size_t)first + (there ? t0 + r : 0);
+            const int column = there ? c0 + piece : 0;
+            bring(&s.x[r][piece], p.x + t * p.channels + column, there);
+            bring(&s.dt[r][piece], p.dt_raw + t * p.channels + column, there);
+            bring(&s.z[r][piece], p.z + t * p.ld_z + column, there);
+        }
+        // a lane's B (and its C) of a token: SPL elements, in pieces of at most 16 bytes
+        constexpr int PIECE = SPL < 4 ? SPL : 4, PER = SPL / PIECE;
+#pragma unroll
+        for (int e = tid; e < RUN_TOKENS * RUN_LANES * 2 * PER; e += RUN_THREADS) {
+            const int part = e % PER, l = (e / PER) % RUN_LANES, which = (e / (PER * RUN_LANES)) & 1, r = e / (PER * RUN_LANES * 2);
+            const int column = l * SPL + part * PIECE;
+            const bool there = t0 + r < count && column < states;
+            const float* src = p.bc + ((size_t)first + (there ? t0 + r : 0)) * p.ld_bc + (which ? p.c_offset : p.b_offset) + (there ? column : 0);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::
+                         "r"((uint32_t)__cvta_generic_to_shared(&s.bc[r][l][which * SPL + part * PIECE])), "l"(src), "n"(PIECE * 4),
+                         "r"(there ? PIECE * 4 : 0) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, 0);
+    const bool live = c < p.channels;
+    const int cc = live ? c : 0;
+    const float bias = p.dt_bias[cc], skip = p.D[cc];
+    float* own = p.state + (size_t)slot * p.state_stride + (size_t)cc * states + lane * SPL;
+    float S[SPL], a[SPL];
+#pragma unroll
+    for (int i = 0; i < SPL; ++i) {
+        const bool there = live && lane * SPL + i < states;
+        S[i] = there ? own[i] : 0.f;
+        a[i] = there ? p.A[(size_t)cc * states + lane * SPL + i] : 0.f;
+    }
+    if (tail.state && live && lane == 0) {
+        // row i of the new state lies taps - 2 - i inputs before the run's last; rows before the run come from the old state, zeros
+        // before the sequence's start
+        float kept[MAX_TAPS];
+        float* mine = tail.state + (size_t)slot * tail.state_stride + c;
+#pragma unroll
+        for (int i = 0; i < MAX_TAPS - 1; ++i) {
+            if (i < tail.taps - 1) {
+                const int r = count - 1 - (tail.taps - 2 - i);
+                kept[i] = start + r < 0 ? 0.f : r >= 0 ? tail.x[((size_t)first + r) * tail.ld + c] : mine[(size_t)(i + count) * p.channels];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < MAX_TAPS - 1; ++i)
+            if (i < tail.taps - 1) mine[(size_t)i * p.channels] = kept[i];
+    }
+    int buffer = 0;
+    for (int t0 = 0; t0 < count; t0 += RUN_TOKENS, buffer ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                     // these tokens are there, the ones before and their results are done with
+        if (t0 + RUN_TOKENS < count) fetch(t0 + RUN_TOKENS, buffer ^ 1);
+        const Stage& s = stages[buffer];
+        const bool full = t0 + RUN_TOKENS <= count;
+        // step sizes: a token of every group a lane, side by side (a chain of some hundred cycles each)
+        float xv[GROUPS];
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+            xv[g] = s.x[g * GROUP + lane][ch];
+            const float dt = softplus(s.dt[g * GROUP + lane][ch] + bias);
+            *reinterpret_cast<float2*>(steps[ch][g * GROUP + lane]) = make_float2(dt, dt * xv[g]);
+        }
+        __syncwarp();
+        float sum[GROUPS];
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+            float y[GROUP];
+            auto recur = [&](auto whole) {
+#pragma unroll
+                for (int u = 0; u < GROUP; u += 2) {
+                    const float4 step = *reinterpret_cast<const float4*>(steps[ch][g * GROUP + u]);
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        const float dtu = v ? step.z : step.x, dxu = v ? step.w : step.y;
+                        float bc[2 * SPL];
+                        if constexpr (SPL >= 2) {
+#pragma unroll
+                            for (int i = 0; i < 2 * SPL; i += 4) {
+                                const float4 four = *reinterpret_cast<const float4*>(&s.bc[g * GROUP + u + v][lane][i]);
+                                bc[i] = four.x, bc[i + 1] = four.y, bc[i + 2] = four.z, bc[i + 3] = four.w;
+                            }
+                        } else {
+                            const float2 pair = *reinterpret_cast<const float2*>(s.bc[g * GROUP + u + v][lane]);
+                            bc[0] = pair.x, bc[1] = pair.y;
+                        }
+                        y[u + v] = 0.f;
+                        if (!decltype(whole)::value && t0 + g * GROUP + u + v >= count) continue;
+#pragma unroll
+                        for (int i = 0; i < SPL; ++i) {
+                            S[i] = fmaf(expf(dtu * a[i]), S[i], dxu * bc[i]);
+                            y[u + v] = fmaf(S[i], bc[SPL + i], y[u + v]);
+                        }
+                    }
+                }
+            };
+            if (full) recur(std::true_type{});
+            else recur(std::false_type{});
+            // as many sums as lanes: at every turn a lane keeps half of its tokens and hands the other half on
+#pragma unroll
+            for (int half = GROUP / 2; half > 0; half >>= 1) {
+#pragma unroll
+                for (int u = 0; u < half; ++u) {
+                    const float mine = lane & half ? y[u + half] : y[u], other = lane & half ? y[u] : y[u + half];
+                    y[u] = mine + __shfl_xor_sync(0xffffffffu, other, half);
+                }
+            }
+            sum[g] = y[0];
+        }
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+            const float zv = s.z[g * GROUP + lane][ch];
+            results[g * GROUP + lane][ch] = from_float<TO>((sum[g] + skip * xv[g]) * (zv / (1.0f + expf(-zv))));
+        }
+        __syncthreads();
+        // a token's eight results lie side by side
+        constexpr int PER = 16 / (int)sizeof(TO), PIECES = RUN_CHANNELS / PER;
+        TO* out = reinterpret_cast<TO*>(p.out);
+        if (tid < RUN_TOKENS * PIECES) {
+            const int r = tid / PIECES, piece = (tid % PIECES) * PER;
+            if (t0 + r < count) {
+                TO* dst = out + ((size_t)first + t0 + r) * p.channels + c0 + piece;
+                if (c0 + RUN_CHANNELS <= p.channels && p.channels % PER == 0) {
+                    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(&results[r][piece]);
+                } else {
+                    for (int i = 0; i < PER; ++i)
+                        if (c0 + piece + i < p.channels) dst[i] = results[r][piece + i];
+                }
+            }
+        }
+    }
+    if (live) {
+#pragma unroll
+        for (int i = 0; i < SPL; ++i)
+            if (lane * SPL + i < states) own[i] = S[i];
+    }
+}
 }  // namespace
 
 // x [n, ld] 32-bit (the first `channels` columns), taps_weight [channels, taps], bias [channels] or null,
@@ -292,6 +557,27 @@ LIA_EXPORT int lia_causal_conv(const float* x, long long ld, const float* taps_w
     if (n_tokens <= 0) return LIA_OK;
     if (channels <= 0 || taps < 1 || taps > MAX_TAPS || ld < channels || (taps > 1 && !state) || act < 0 || act > 1)
         return LIA_ERR_SIZE;
+    const size_t copy_size = copy_dtype == LIA_BF16 ? 2 : 4;
+    if (!update_single && n_tokens >= CONV_TILED_FROM && taps >= 2 && taps <= 4 && channels % 4 == 0 && ld % 4 == 0 &&
+        (((uintptr_t)x | (uintptr_t)out) & 15u) == 0 && ((uintptr_t)out_copy & (4 * copy_size - 1)) == 0 &&
+        (n_tokens + CONV_ROWS - 1) / CONV_ROWS <= 65535) {
+        const dim3 tiles((channels / 4 + CONV_THREADS - 1) / CONV_THREADS, (n_tokens + CONV_ROWS - 1) / CONV_ROWS);
+#define LIA_CONV(TO, TAPS)                                                                                              \
+    return lia_launch(causal_conv_tile_kernel<TO, TAPS>, tiles, dim3(CONV_THREADS), 0, stream, x, ld, taps_weight, bias, state, \
+                      state_stride, positions, slots, out, (TO*)out_copy, n_tokens, channels, act)
+        if (!out_copy || copy_dtype == LIA_F32) {
+            if (taps == 2) LIA_CONV(float, 2);
+            if (taps == 3) LIA_CONV(float, 3);
+            LIA_CONV(float, 4);
+        }
+        if (copy_dtype == LIA_BF16) {
+            if (taps == 2) LIA_CONV(__nv_bfloat16, 2);
+            if (taps == 3) LIA_CONV(__nv_bfloat16, 3);
+            LIA_CONV(__nv_bfloat16, 4);
+        }
+#undef LIA_CONV
+        return LIA_ERR_DTYPE;
+    }
     const int threads = 128;
     // few tokens: a token's channels over several CTAs, so that the step's rows fill the device
     const dim3 grid(n_tokens, n_tokens >= 512 ? 1 : min(16, (channels + threads - 1) / threads));
@@ -357,19 +643,43 @@ int launch_scan(ScanArgs p, int n_tokens, bool chunked, cudaStream_t stream) {
 }
 }  // namespace
 
+namespace {
+template <typename TO>
+int launch_runs(const ScanArgs& p, const ConvTail& tail, cudaStream_t stream) {
+    const dim3 grid((p.channels + RUN_CHANNELS - 1) / RUN_CHANNELS, p.n_segments);
+    // (launched the ordinary way: CTAs that begin under the product ahead, whose own CTAs fill most SMs' shared memory, would all
+    // gather on the few SMs that it leaves free and stay there; 2,048 tokens of a whole layer took 603 us so, 343 in turn)
+    if (p.states <= 16) return lia_launch_in_turn(scan_run_kernel<TO, 1>, grid, dim3(RUN_THREADS), 0, stream, p, tail);
+    if (p.states <= 32) return lia_launch_in_turn(scan_run_kernel<TO, 2>, grid, dim3(RUN_THREADS), 0, stream, p, tail);
+    return lia_launch_in_turn(scan_run_kernel<TO, 4>, grid, dim3(RUN_THREADS), 0, stream, p, tail);
+}
+}  // namespace
+
+// 1 if the kernel that walks whole portions takes these: at most 64 states, every row's pieces of four elements aligned.
+LIA_EXPORT int lia_selective_scan_walks_runs(const void* x, const void* dt_raw, const void* bc, long long ld_bc, int b_offset,
+                                             int c_offset, const void* z, long long ld_z, const void* out, int channels, int states) {
+    return channels > 0 && states > 0 && states <= 64 && ((channels | states | b_offset | c_offset) & 3) == 0 && ((ld_bc | ld_z) & 3) == 0 &&
+                   (((uintptr_t)x | (uintptr_t)dt_raw | (uintptr_t)bc | (uintptr_t)z | (uintptr_t)out) & 15u) == 0
+               ? 1 : 0;
+}
+
+// `conv_state` (or null; slot s at conv_state + s conv_stride: [taps - 1, channels]): the portions leave their last taps - 1 inputs
+// there, read from conv_x [n, conv_ld]; only where lia_selective_scan_walks_runs says yes and the step has no single tokens.
 LIA_EXPORT int lia_selective_scan(const float* x, const float* dt_raw, const float* dt_bias, const float* A,
                                   const float* bc, long long ld_bc, int b_offset, int c_offset, const float* D,
                                   const float* z, long long ld_z, float* state, long long state_stride,
                                   const int* segments, int n_segments,
                                   const int* single_rows, int n_single, const int* slots, void* out, int out_dtype,
                                   int channels, int states, int n_tokens, float* chunk_scratch, long long chunk_floats,
+                                  float* conv_state, long long conv_stride, const float* conv_x, long long conv_ld, int taps,
                                   cudaStream_t stream) {
     const int runs = n_segments + n_single;
     if (runs <= 0) return LIA_OK;
+    if ((conv_state && (!conv_x || taps < 2 || taps > MAX_TAPS || n_single > 0)) || n_segments > 65535) return LIA_ERR_SIZE;
     if (channels <= 0 || states <= 0 || states > 32 * STATES_PER_LANE || n_segments < 0 || n_single < 0 ||
         ld_bc < b_offset + states || ld_bc < c_offset + states || ld_z < channels || n_tokens < n_single + 2 * n_segments)
         return LIA_ERR_SIZE;
-    const bool chunked = chunk_scratch && n_segments > 0;
+    bool chunked = chunk_scratch && n_segments > 0;
     if (chunked && chunk_floats < lia_selective_scan_chunk_floats(n_tokens, n_segments, channels, states)) return LIA_ERR_SIZE;
     ScanArgs p;
     p.x = x; p.dt_raw = dt_raw; p.dt_bias = dt_bias; p.A = A; p.bc = bc; p.ld_bc = ld_bc; p.b_offset = b_offset;
@@ -378,6 +688,16 @@ LIA_EXPORT int lia_selective_scan(const float* x, const float* dt_raw, const flo
     p.out = out; p.channels = channels; p.states = states;
     p.chunk_state = chunk_scratch;
     p.chunk_dt = chunk_scratch ? chunk_scratch + ((long long)n_tokens / CHUNK + n_segments) * channels * states : nullptr;
+    if (n_segments > 0 && lia_selective_scan_walks_runs(x, dt_raw, bc, ld_bc, b_offset, c_offset, z, ld_z, out, channels, states)) {
+        const int rc = out_dtype == LIA_F32 ? launch_runs<float>(p, {conv_state, conv_stride, conv_x, conv_ld, taps}, stream)
+                     : out_dtype == LIA_BF16 ? launch_runs<__nv_bfloat16>(p, {conv_state, conv_stride, conv_x, conv_ld, taps}, stream)
+                                             : LIA_ERR_DTYPE;
+        if (rc != LIA_OK || n_single <= 0) return rc;
+        p.n_segments = 0;
+        chunked = false;
+    } else if (conv_state) {
+        return LIA_ERR_SIZE;
+    }
     int lpc = 1;
     while (lpc * STATES_PER_LANE < states) lpc *= 2;
 #define LIA_SCAN_LANES(TO)                                                     \

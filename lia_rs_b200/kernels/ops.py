@@ -137,7 +137,10 @@ class _Signatures:
                              c_int, c_void_p]
     lia_selective_scan = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_void_p,
                           c_void_p, ctypes.c_longlong, c_void_p, ctypes.c_longlong, c_void_p, c_int, c_void_p, c_int, c_void_p,
-                          c_void_p, c_int, c_int, c_int, c_int, c_void_p, ctypes.c_longlong, c_void_p]
+                          c_void_p, c_int, c_int, c_int, c_int, c_void_p, ctypes.c_longlong, c_void_p, ctypes.c_longlong, c_void_p,
+                          ctypes.c_longlong, c_int, c_void_p]
+    lia_selective_scan_walks_runs = [c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_void_p, ctypes.c_longlong, c_void_p,
+                                     c_int, c_int]
     lia_selective_scan_chunk_floats = [c_int, c_int, c_int, c_int]
     lia_gemm_simt_batched = [c_int, c_void_p, c_int, c_int, ctypes.c_longlong, c_void_p, c_int, c_int, ctypes.c_longlong,
                              c_void_p, c_int, c_int, ctypes.c_longlong, c_int, c_int, c_int, c_int, c_float, c_void_p]
@@ -1178,12 +1181,22 @@ def selective_scan_chunk_floats(n_tokens: int, n_segments: int, channels: int, s
     return int(fn(int(n_tokens), int(n_segments), int(channels), int(states)))
 
 
+def selective_scan_walks_runs(x, dt_raw, bc, b_offset, c_offset, z, out, states: int) -> bool:
+    """Whether a step's portions are walked whole by the kernel that keeps a channel in eight lanes (it needs no scratch and can
+    leave the convolution's state): at most 64 states, rows whose pieces of four elements are aligned."""
+    return bool(lib().lia_selective_scan_walks_runs(_p(x), _p(dt_raw), _p(bc), bc.stride(0), int(b_offset), int(c_offset), _p(z),
+                                                    z.stride(0), _p(out), x.shape[1], int(states)))
+
+
 def selective_scan(x, dt_raw, dt_bias, A, bc, b_offset, c_offset, D, z, state, segments, n_segments, single_rows, slots, out,
-                   chunk_scratch=None):
+                   chunk_scratch=None, conv_state=None, conv_x=None):
     """The recurrence S <- exp(dt A) S + dt x B, y = (S C + D x) silu(z) with dt = softplus(dt_raw + dt_bias), along the
     step's runs (`segments` [n, 3] and `single_rows`), state [slots, channels, states] 32-bit; see csrc/selective_scan.cu.
-    With `chunk_scratch` (32-bit, `selective_scan_chunk_floats` words) the portions are cut into chunks of 64 tokens that
-    run side by side: a pass from zero states, a carry along each portion, a pass from the true start states."""
+    Portions that `selective_scan_walks_runs` takes are walked whole.  Others, with `chunk_scratch` (32-bit,
+    `selective_scan_chunk_floats` words), are cut into chunks of 64 tokens that run side by side: a pass from zero states, a
+    carry along each portion, a pass from the true start states.  `conv_state` [slots, taps - 1, channels] (only where
+    `selective_scan_walks_runs`, and in steps without single tokens): the portions also leave their last inputs there, from the
+    rows `conv_x`, as `conv_state_update` does."""
     _cuda(x, dt_raw, dt_bias, A, D, segments, single_rows, slots, out, chunk_scratch)
     _f32(x, dt_raw, dt_bias, A, bc, D, z, state, chunk_scratch)
     n, channels = x.shape
@@ -1192,12 +1205,19 @@ def selective_scan(x, dt_raw, dt_bias, A, bc, b_offset, c_offset, D, z, state, s
     if tuple(dt_raw.shape) != (n, channels) or tuple(A.shape) != (channels, states) or bc.stride(1) != 1 or z.stride(1) != 1 \
             or tuple(state.shape[1:]) != (channels, states) or not state[0].is_contiguous() or tuple(out.shape) != (n, channels):
         raise KernelError("selective_scan: shapes do not agree")
+    tail = (None, 0, None, 0, 0)
+    if conv_state is not None:
+        _f32(conv_state, conv_x)
+        if conv_state.shape[2] != channels or not conv_state[0].is_contiguous() or conv_x.stride(1) != 1 or \
+                conv_x.shape[0] != n or conv_x.shape[1] < channels:
+            raise KernelError("selective_scan: conv_state [slots, taps - 1, channels] and the step's input rows")
+        tail = (_p(conv_state), conv_state.stride(0), _p(conv_x), conv_x.stride(0), conv_state.shape[1] + 1)
     with _timed("selective_scan", nbytes=n * channels * (12 + out.element_size())):
         _check(lib().lia_selective_scan(_p(x), _p(dt_raw), _p(dt_bias), _p(A), _p(bc), bc.stride(0), int(b_offset),
                                         int(c_offset), _p(D), _p(z), z.stride(0), _p(state), state.stride(0), _p(segments), int(n_segments),
                                         _p(single_rows), n_single, _p(slots), _p(out), dtype_code(out.dtype), channels,
                                         states, n, _p(chunk_scratch), 0 if chunk_scratch is None else chunk_scratch.numel(),
-                                        _stream()), "selective_scan")
+                                        *tail, _stream()), "selective_scan")
 
 
 def gemm_simt_batched(mode, a, w, out, alpha: float = 1.0, label=None):

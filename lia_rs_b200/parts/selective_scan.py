@@ -10,9 +10,10 @@
 What a request carries from token to token is one 32-bit state per slot: the convolution's last taps - 1 inputs and
 S.  The products may run in the compute element type; the convolution and its activation, step sizes, decays,
 exponentials, the state and the sums over it are 32-bit (csrc/selective_scan.cu).  A step's runs (prompt portions and
-single tokens) are walked token by token on the device, so a portion cut anywhere continues from the slot's state.  In a
-step of many tokens the portions are cut into chunks of 64 tokens that run side by side: the recurrence is linear in the
-state, so a chunk's end state is its end state from zero plus the decayed state it started from.
+single tokens) are walked token by token on the device, so a portion cut anywhere continues from the slot's state.  Portions
+of sizes that the kernel for whole portions does not take (more than 64 states, sizes that are no multiples of four) are, in a
+step of many tokens, cut into chunks of 64 tokens that run side by side: the recurrence is linear in the state, so a chunk's
+end state is its end state from zero plus the decayed state it started from.
 
 Parameters: hidden, inner, state, dt_rank, taps, and optionally `names` (checkpoint names behind the part's prefix)."""
 from __future__ import annotations
@@ -95,8 +96,6 @@ class SelectiveScan(Mixer):
         single = ctx.decode_only                  # single tokens only: the convolution leaves its new state itself
         ops.causal_conv(uz, self.conv, self.conv_bias, conv_state, ctx.positions, ctx.slots, u, u_rounded, act=1,
                         update_single=single)
-        if taps > 1 and not single:
-            ops.conv_state_update(uz, conv_state, ctx.positions, ctx.slots, inner)
         projected = ctx.buffer("scan.x", (n, rank + 2 * states), torch.float32)
         linear(rt, STORE, u if u_rounded is None else u_rounded, self.w_x, projected, error_flag=flag, name="x")
         low = ctx.buffer("scan.dt_in", (n, rank), dtype)
@@ -104,11 +103,17 @@ class SelectiveScan(Mixer):
         dt_raw = ctx.buffer("scan.dt", (n, inner), torch.float32)
         linear(rt, STORE, low, self.w_dt, dt_raw, error_flag=flag, name="dt")
         y = ctx.buffer("scan.y", (n, inner), dtype)
-        chunk_scratch = None
-        if ctx.n_prefill_segments and n >= self.CHUNKED_FROM:
+        chunk_scratch, more = None, {}
+        bc = (projected, rank, rank + states)
+        whole = ctx.n_prefill_segments and ops.selective_scan_walks_runs(u, dt_raw, *bc, uz[:, inner:], y, states)
+        if taps > 1 and not single:
+            if whole and not ctx.n_single:           # the scan's kernel leaves the convolution's state too
+                more = dict(conv_state=conv_state, conv_x=uz)
+            else:
+                ops.conv_state_update(uz, conv_state, ctx.positions, ctx.slots, inner)
+        if ctx.n_prefill_segments and n >= self.CHUNKED_FROM and not whole:
             words = ops.selective_scan_chunk_floats(n, ctx.n_prefill_segments, inner, states)
             chunk_scratch = ctx.runtime.scratch("scan.chunks", words, torch.float32)
-        ops.selective_scan(u, dt_raw, self.dt_bias, self.decay, projected, rank, rank + states, self.skip, uz[:, inner:],
-                           scan_state, ctx.prefill_segments, ctx.n_prefill_segments, ctx.decode_rows, ctx.slots, y,
-                           chunk_scratch=chunk_scratch)
+        ops.selective_scan(u, dt_raw, self.dt_bias, self.decay, *bc, self.skip, uz[:, inner:], scan_state, ctx.prefill_segments,
+                           ctx.n_prefill_segments, ctx.decode_rows, ctx.slots, y, chunk_scratch=chunk_scratch, **more)
         linear(rt, STORE if store else ACCUM, y, self.w_o, residual, scale, error_flag=flag, name="o")
