@@ -108,28 +108,62 @@ class StepRuntime:
         self._host = host_library()
         self._summary = (ctypes.c_int * 8)()
         self._buffers = {}
+        self._views = {}
         self._attentions = {}
         self._logits_buffer = None
         self.generation = 0            # grows whenever a buffer is (re)allocated: captured graphs are stale then
 
     # ---- memory ----
+    # (`_views`: the part of a buffer that a step was given, by name and size: a step asks for the same few again and again, and
+    # making each view anew cost more than the look; emptied when a buffer moves, and bounded)
+    MOST_VIEWS = 4096
+
+    def _keep_view(self, key, view):
+        if len(self._views) >= self.MOST_VIEWS:
+            self._views.clear()
+        self._views[key] = view
+        return view
+
+    def _moved(self):
+        self.generation += 1
+        self._views.clear()
+
     def workspace(self, name, shape, dtype):
+        view = self._views.get((name, shape, dtype))
+        return view if view is not None else self._keep_view((name, shape, dtype), self._workspace(name, shape, dtype))
+
+    def _workspace(self, name, shape, dtype):
         rows, width = shape
         key = (name, width, dtype)
         buf = self._buffers.get(key)
         if buf is None or buf.shape[0] < rows:
             buf = torch.empty((max(rows, self.max_batch_tokens), width), dtype=dtype, device=self.device)
             self._buffers[key] = buf
-            self.generation += 1
+            self._moved()
         return buf[:rows]
 
     def scratch(self, name, numel, dtype):
         """A flat scratch buffer of at least `numel` elements (grows, never shrinks)."""
+        view = self._views.get((name, numel, dtype))
+        return view if view is not None else self._keep_view((name, numel, dtype), self._scratch(name, numel, dtype))
+
+    def shaped(self, name, shape, dtype):
+        """`scratch` of as many elements as `shape` has, in that shape."""
+        view = self._views.get((name, dtype, shape))
+        if view is None:
+            numel = 1
+            for size in shape:
+                numel *= size
+            view = self._scratch(name, numel, dtype).view(shape)
+            self._keep_view((name, dtype, shape), view)
+        return view
+
+    def _scratch(self, name, numel, dtype):
         buf = self._buffers.get((name, dtype))
         if buf is None or buf.numel() < numel:
             buf = torch.empty(max(numel, 1), dtype=dtype, device=self.device)
             self._buffers[(name, dtype)] = buf
-            self.generation += 1
+            self._moved()
         return buf[:numel]
 
     def counters(self, count):
@@ -138,7 +172,7 @@ class StepRuntime:
         if buf is None or buf.numel() < count:
             buf = torch.zeros(max(count, 4096), dtype=torch.int32, device=self.device)
             self._buffers["counters"] = buf
-            self.generation += 1
+            self._moved()
         return buf[:count]
 
     def logits(self, rows, vocab):
@@ -146,7 +180,7 @@ class StepRuntime:
         if buf is None or buf.shape[0] < rows or buf.shape[1] != vocab:
             buf = torch.empty((max(rows, self.cache.max_slots), vocab), dtype=torch.float32, device=self.device)
             self._logits_buffer = buf
-            self.generation += 1
+            self._moved()
         return buf[:rows]
 
     # ---- a step's metadata ----

@@ -227,13 +227,15 @@ def _p(t):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream():
     """The current stream's handle.  Asked for at every launch (a graph capture runs on a stream of its own), so through
-    torch's direct call where this torch has it: building a Stream object each time cost several microseconds a launch."""
+    torch's direct calls where this torch has them: building a Stream object each time cost several microseconds a launch.
+    (A launch's tensors are on the device, so CUDA is initialised.)"""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_current_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -502,6 +504,54 @@ def gemm_cluster(mode, a, w, out, alpha: float = 1.0, error_flag=None, label=Non
     with _timed("gemm_cluster", label, work=lambda: _gemm_work(a, w, out)):
         _check(lib().lia_gemm_cluster(mode, _p(a), a.stride(0), _p(w), w.stride(0), _p(out), dtype_code(out.dtype),
                                       out.stride(0), M, N, K, alpha, sms, _p(error_flag), _stream()), "gemm_cluster")
+
+
+def bind_product(kernel: str, mode, a, w, out):
+    """A product of these sizes, strides and element types as a function of its addresses, call(a, w, out, alpha,
+    error_flag): what a call has to look up and convert anew although it follows from the sizes is looked up once.  `kernel` is
+    "tc", "cluster" or "simt"; the arguments' agreement is checked here, once.  The caller keeps the function by the very sizes,
+    strides and types and gives it tensors of the same."""
+    (M, K), N = a.shape, out.shape[1]
+    if w.shape[1] != K or out.shape[0] != M or w.shape[0] != (2 * N if mode == GEMM_SWIGLU else N):
+        raise KernelError(f"gemm: shapes do not agree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    lda, ldw, ldo, code = a.stride(0), w.stride(0), out.stride(0), dtype_code(out.dtype)
+    if kernel == "tc":
+        fn, (scratch, sms) = lib().lia_gemm_tc, _device_scratch(a.device)
+        scratch_at, scratch_floats = scratch.data_ptr(), scratch.numel()
+
+        def call(a, w, out, alpha, error_flag):
+            _check(fn(mode, a.data_ptr(), lda, w.data_ptr(), ldw, out.data_ptr(), code, ldo, M, N, K, alpha, scratch_at, scratch_floats,
+                      sms, 0.0, 0.0, None if error_flag is None else error_flag.data_ptr(), _stream()), "gemm_tc")
+    elif kernel == "cluster":
+        fn, sms = lib().lia_gemm_cluster, _device_scratch(a.device)[1]
+
+        def call(a, w, out, alpha, error_flag):
+            _check(fn(mode, a.data_ptr(), lda, w.data_ptr(), ldw, out.data_ptr(), code, ldo, M, N, K, alpha, sms,
+                      None if error_flag is None else error_flag.data_ptr(), _stream()), "gemm_cluster")
+    else:
+        fn, a_code, w_code = lib().lia_gemm_simt, dtype_code(a.dtype), dtype_code(w.dtype)
+
+        def call(a, w, out, alpha, error_flag):
+            _check(fn(mode, a.data_ptr(), a_code, lda, w.data_ptr(), w_code, ldw, out.data_ptr(), code, ldo, M, N, K, alpha,
+                      _stream()), "gemm_simt")
+    return call
+
+
+def bind_batched(a, w, out):
+    """As `bind_product` for `gemm_mma_batched`: call(a, w, out), or None where that kernel does not take these sizes."""
+    if not gemm_mma_batched_accepts(a, w, out):
+        return None
+    (_, lda, a_plane, _, ldw, w_plane, _, ldo, o_plane), (B, M, N, K) = _batched_arguments(a, w, out)
+    fn = lib().lia_gemm_mma_batched
+
+    def call(a, w, out):
+        _check(fn(a.data_ptr(), lda, a_plane, w.data_ptr(), ldw, w_plane, out.data_ptr(), ldo, o_plane, B, M, N, K, _stream()),
+               "gemm_mma_batched")
+    return call
+
+
+def profiling() -> bool:
+    return _profiler is not None
 
 
 SKINNY_MAX_TOKENS = 32

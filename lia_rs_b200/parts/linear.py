@@ -39,6 +39,9 @@ CLUSTER_MAX_TOKENS = 256        # beyond, narrow tiles of the persistent kernel 
 
 _TC, _SKINNY, _CLUSTER, _SIMT, _STREAM = range(5)
 _choices = {}          # what decides the choice -> the kernel chosen (the checks cost more than the lookup)
+_bound = {}            # the same -> the product as a function of its addresses (plain products of the kernels that more than a few tokens take)
+_BOUND_KERNELS = {_TC: "tc", _CLUSTER: "cluster", _SIMT: "simt"}
+_MOST_BOUND = 1024     # sizes kept; beyond, all are looked up anew (a step's sizes are few: a batch's and a prompt's)
 
 
 def _choose(mode, a, w, out) -> int:
@@ -55,6 +58,12 @@ def _choose(mode, a, w, out) -> int:
     if tensor_cores:
         return _TC
     return _SKINNY if few else _SIMT
+
+
+def _bind(choice, key, mode, a, w, out):
+    if len(_bound) >= _MOST_BOUND:
+        _bound.clear()
+    _bound[key] = ops.bind_product(_BOUND_KERNELS[choice], mode, a, w, out)
 
 
 def linear(runtime, mode: int, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float = 1.0,
@@ -91,12 +100,20 @@ def linear(runtime, mode: int, a: torch.Tensor, w: torch.Tensor, out: torch.Tens
                                 activation=activation or gate_activation, act_constants=activation_constants)
                 return bool(activation)
         a = a.tensor()
+    # everything the kernels' acceptance looks at: sizes, row strides, element types, 16-byte alignment of the bases
+    key = (mode, a.shape, a.stride(), a.dtype, a.data_ptr() & 15, w.shape, w.stride(), w.dtype, w.data_ptr() & 15,
+           out.shape, out.stride(), out.dtype, out.data_ptr() & 15, a.device.index)
+    plain = not (activation or gate_activation or ops.profiling())
+    if plain:
+        call = _bound.get(key)
+        if call is not None:
+            call(a, w, out, alpha, error_flag)
+            return False
     if a.dtype != torch.bfloat16:
+        if plain and a.dtype == torch.float32 == w.dtype and a.stride(1) == 1 == w.stride(1):
+            _bind(_SIMT, key, mode, a, w, out)
         ops.gemm_simt(mode, a, w, unactivated if activation else out, alpha, label=name, act=gate_activation)
         return False
-    # everything the kernels' acceptance looks at: sizes, row strides, element types, 16-byte alignment of the bases
-    key = (mode, a.shape, a.stride(), a.data_ptr() & 15, w.shape, w.stride(), w.dtype, w.data_ptr() & 15,
-           out.shape[1], out.stride(), out.dtype, out.data_ptr() & 15, a.device.index)
     choice = _choices.get(key)
     if choice is None:
         choice = _choices[key] = _choose(mode, a, w, out)
@@ -114,6 +131,8 @@ def linear(runtime, mode: int, a: torch.Tensor, w: torch.Tensor, out: torch.Tens
         # the two kernels for products in between have the SiLU gate alone: the cluster kernel's shapes go to the persistent
         # tcgen05 kernel, the one-CTA-per-16-rows kernel's to the product on the 32-bit pipes
         choice = _TC if choice == _CLUSTER else _SIMT
+    if plain and choice in _BOUND_KERNELS:
+        _bind(choice, key, mode, a, w, out)
     if choice == _TC:
         ops.gemm_tc(mode, a, w, out, alpha, error_flag, label=name, act=gate_activation)
     elif choice == _STREAM:

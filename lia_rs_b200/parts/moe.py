@@ -135,9 +135,9 @@ class ExpertMixture(FeedForward):
         rt, n = self.runtime, x.shape[0]
         top, experts, dtype = self.top, self.experts, rt.compute_dtype
         pairs = n * top
-        scratch = ctx.runtime.scratch
-        ids = scratch("moe.ids", pairs, torch.int32).view(n, top)
-        weights = scratch("moe.weights", pairs, torch.float32).view(n, top)
+        scratch, shaped = ctx.runtime.scratch, ctx.runtime.shaped
+        ids = shaped("moe.ids", (n, top), torch.int32)
+        weights = shaped("moe.weights", (n, top), torch.float32)
         shared_gate = scratch("moe.shared_gate", n, torch.float32) if self.shared and self.shared_gated else None
         ops.moe_route(x, self.router, top, self.router_scale, ids, weights, shared_gate, correction=self.correction,
                       groups=self.groups, keep=self.keep, renormalise=self.renormalise, sigmoid=self.sigmoid, two_best=self.two_best)
@@ -156,10 +156,10 @@ class ExpertMixture(FeedForward):
         tiles = lists[experts + 2 + rows + pairs:]
         # (pairs whose output names no expert, the identity outputs, get no row: `inverse` is negative there)
         ops.moe_plan(ids.view(-1), experts, offsets, order, inverse, tiles, n_tiles, tile_rows, pad=self.grouped)
-        act = scratch("moe.act", rows * self.ff, dtype).view(rows, self.ff)
-        y = scratch("moe.y", rows * self.hidden, torch.float32).view(rows, self.hidden)
+        act = shaped("moe.act", (rows, self.ff), dtype)
+        y = shaped("moe.y", (rows, self.hidden), torch.float32)
         if self.grouped:
-            sorted_x = scratch("moe.x", rows * self.hidden, dtype).view(rows, self.hidden)
+            sorted_x = shaped("moe.x", (rows, self.hidden), dtype)
             ops.moe_gather(x, order, top, sorted_x)
             if self.gated:
                 ops.gemm_tc_grouped(SWIGLU, sorted_x, self.w_gate_up, act, tile_rows, tiles, n_tiles, max_tiles, pairs,

@@ -208,6 +208,9 @@ class SinkAttention(Mixer):
         linear(rt, STORE if store else ACCUM, o, self.w_o, residual, scale, error_flag=flag, name="o")
 
 
+_batched = {}            # sizes, strides and alignment of a product of all heads -> the kernel's call (0: another kernel serves them)
+
+
 @register_mixer("latent_attention")
 class LatentAttention(Mixer):
     graph_safe = True
@@ -344,12 +347,12 @@ class LatentAttention(Mixer):
         H, d, dr, dv, rank = self.heads, self.d, self.dr, self.dv, self.rank
         n, size, flag = q.shape[0], kv.page_size, ctx.error_flag
         scratch = ctx.runtime.scratch
-        records = scratch("latent.records", pages * size * (rank + dr), torch.bfloat16).view(pages * size, rank + dr)
-        table = scratch("latent.table", kv.block_table.numel(), torch.int32).view(kv.block_table.shape)
+        records = ctx.runtime.shaped("latent.records", (pages * size, rank + dr), torch.bfloat16)
+        table = ctx.runtime.shaped("latent.table", kv.block_table.shape, torch.int32)
         ops.latent_gather(ctx.prefill_segments, ctx.n_prefill_segments, ctx.slots, kv.block_table, kv.k_pages, kv.v_pages,
                           records.view(pages, size, rank + dr), table, self.window, error_flag=flag)
         width = H * (d + dr + dv)
-        expanded = scratch("latent.expanded", pages * size * width, torch.bfloat16).view(pages * size, width)
+        expanded = ctx.runtime.shaped("latent.expanded", (pages * size, width), torch.bfloat16)
         linear(rt, STORE, records, self.w_expand, expanded, error_flag=flag, name="expand")
         paged = expanded.view(pages, size, width)
         keys, values = paged[:, :, :H * (d + dr)].unflatten(2, (H, d + dr)), paged[:, :, H * (d + dr):].unflatten(2, (H, dv))
@@ -367,10 +370,10 @@ class LatentAttention(Mixer):
         """out [tokens, heads, dv] (any strides) = attention in the latent's space of the tokens whose queries these are, q_plain
         [heads, tokens, d] and q_rotated [tokens, heads dr] or [tokens, heads, dr]; `rows`: which of the step's tokens they are."""
         H, n, rank, dtype = self.heads, q_plain.shape[1], self.rank, self.runtime.compute_dtype
-        scratch = ctx.runtime.scratch
-        q_absorbed = scratch("latent.q_absorbed", H * n * rank, dtype).view(H, n, rank)
+        scratch, shaped = ctx.runtime.scratch, ctx.runtime.shaped
+        q_absorbed = shaped("latent.q_absorbed", (H, n, rank), dtype)
         self._head_products(ctx, q_plain, self.w_k_up_t, q_absorbed, "k_up")
-        mixed = scratch("latent.mixed", H * n * rank, dtype).view(H, n, rank)
+        mixed = shaped("latent.mixed", (H, n, rank), dtype)
         if self.tensor_cores:
             splits = self._splits(ctx, n)
             partial = scratch("latent.partial", splits * H * n * (rank + 2), torch.float32) if splits > 1 else None
@@ -407,7 +410,18 @@ class LatentAttention(Mixer):
         """out[h] = a[h] @ w[h]^T for every head (3-D tensors, a head a plane), all heads in one launch: in
         bfloat16 on the tensor cores (csrc/gemm_mma_batched.cu) where that kernel takes the sizes (8 tokens of 16 heads:
         5 us against 29 on the 32-bit pipes), else, and on the 32-bit path, on the 32-bit pipes."""
-        if a.dtype == torch.bfloat16 and a.shape[1] >= self.TENSOR_CORES_FROM and ops.gemm_mma_batched_accepts(a, w, out):
+        key = (a.shape, a.stride(), a.data_ptr() & 15, w.shape, out.stride(), out.data_ptr() & 3, a.device.index)
+        if a.dtype == torch.bfloat16 and a.shape[1] >= self.TENSOR_CORES_FROM and not ops.profiling():
+            call = _batched.get(key)
+            if call is None:
+                if len(_batched) >= 256:
+                    _batched.clear()
+                call = _batched[key] = ops.bind_batched(a, w, out) or 0
+            if call:
+                call(a, w, out)
+            else:
+                ops.gemm_simt_batched(STORE, a, w, out, label=name)
+        elif a.dtype == torch.bfloat16 and a.shape[1] >= self.TENSOR_CORES_FROM and ops.gemm_mma_batched_accepts(a, w, out):
             ops.gemm_mma_batched(a, w, out, label=name)
         else:
             ops.gemm_simt_batched(STORE, a, w, out, label=name)
@@ -426,10 +440,10 @@ class LatentAttention(Mixer):
             q_rows = ctx.buffer("latent.q", (n, H * (d + dr)), torch.float32)
             linear(rt, STORE, DeferredNorm(ctx, self.q_norm, part("q_down"), buffer_name="latent.cq_normed"), self.w_q_up, q_rows,
                    error_flag=flag, name="q_up")
-        scratch = ctx.runtime.scratch
+        shaped = ctx.runtime.shaped
         plan = self._expansion(ctx)
         if plan is None:
-            q_plain = scratch("latent.q_plain", H * n * d, dtype).view(H, n, d)
+            q_plain = shaped("latent.q_plain", (H, n, d), dtype)
             q_rotated = ctx.buffer("latent.q_rot", (n, H * dr), dtype)
         else:
             q = ctx.buffer("latent.q_whole", (n, H * (d + dr)), dtype)
@@ -446,14 +460,14 @@ class LatentAttention(Mixer):
             if ctx.n_single:
                 # the step's single tokens attend in the latent's space, side by side in buffers of their own
                 singles, rows = ctx.n_single, ctx.decode_rows
-                q_singles = scratch("latent.q_singles", singles * H * (d + dr), dtype).view(singles, H * (d + dr))
+                q_singles = shaped("latent.q_singles", (singles, H * (d + dr)), dtype)
                 ops.gather_rows(q, rows, q_singles)
                 apart = q_singles.view(singles, H, d + dr)
-                o_singles = scratch("latent.o_singles", singles * H * dv, dtype).view(singles, H * dv)
+                o_singles = shaped("latent.o_singles", (singles, H * dv), dtype)
                 self._attend_in_latent(ctx, apart[:, :, :d].transpose(0, 1), apart[:, :, d:], kv, o_singles.view(singles, H, dv),
                                        rows=rows)
                 if gate is not None:
-                    gate_singles = scratch("latent.gate_singles", singles * gate.shape[1], torch.float32).view(singles, gate.shape[1])
+                    gate_singles = shaped("latent.gate_singles", (singles, gate.shape[1]), torch.float32)
                     ops.gather_rows(gate, rows, gate_singles)
                     ops.gate_rows(o_singles, gate_singles, ops.GATE_SIGMOID, span=self.gate_span)
                 ops.scatter_rows(o_singles, rows, o)
