@@ -27,7 +27,12 @@ using namespace tc5;
 #define GEMM_SWIGLU 2
 
 namespace {
-constexpr int THREADS = 224;            // warp 0: TMA, warps 1 and 6: MMA, warps 2-5: accumulator to shared memory
+// Sixteen warps: behind the last product everything waits for memory of some kind (the accumulators, the neighbours' shared memory,
+// the residual row), so the items of the sum are cut over as many threads as the registers allow.  224 threads, of which four warps
+// emptied the accumulators load by load, took at 64 tokens (2B-class layer) q|k|v 8.8, o 7.4, gate/up 19.5, down 12.2 us; now 8.4, 7.0,
+// 18.1, 11.8; at 128 tokens 11.9, 9.3, 23.2, 15.5 and now 10.5, 8.6, 20.6, 14.8; at 17 tokens the same.
+constexpr int THREADS = 512;            // warp 0: TMA, warps 1 and 2: MMA, warps 4-15: accumulator to shared memory
+constexpr int DRAIN_WARP = 4, DRAIN_SETS = 3;      // first of the warps that empty the accumulators; sets of four such warps
 constexpr int MAX_STAGES = 12;
 constexpr int MAX_CLUSTER = 8;
 constexpr int SMEM_LIMIT = 200 * 1024;
@@ -159,13 +164,13 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             for (int i = max(0, issued - s.stages); i < issued; ++i)      // copies in flight must land before the CTA may end
                 mbar_wait(smem_u32(&full_bar[i % s.stages]), (uint32_t)(i / s.stages) & 1u);
         }
-    } else if ((warp == 1 || warp == 6) && lane == 0) {
+    } else if ((warp == 1 || warp == 2) && lane == 0) {
         // ---- MMA issuers.  Issuing one tcgen05.mma costs a thread some 130 cycles, four times what a tile this
         //      narrow computes for, so two threads issue: they take the K blocks in turn, each into accumulators of
         //      its own (an MMA that adds to the accumulator of the one before it would wait for it, too).  The
         //      epilogue adds the accumulators up in a fixed order. ----
         const int issuers = s.chains >= 2 ? 2 : 1;
-        const int me = warp == 1 ? 0 : 1;
+        const int me = warp - 1;
         const int own = s.chains / issuers;                   // accumulators of this issuer
         const uint32_t idesc = instr_desc(TILE_F, s.n_tile);
         bool ok = true;
@@ -197,42 +202,45 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             if (ok) tc_commit(smem_u32(&acc_full));
             else if (s.error_flag) atomicExch(s.error_flag, 3);
         }
-    } else if (warp >= 2 && warp <= 5) {
-        // ---- accumulator to the exchange buffer: warp w holds TMEM lanes 32*(w%4) .. +31 = features ----
+    } else if (warp >= DRAIN_WARP) {
+        // ---- accumulator to the exchange buffer: warp w holds TMEM lanes 32*(w%4) .. +31 = features.  A unit is sixteen
+        //      tokens of one tile of W; the sets take the units in turn, and all chains' columns are asked for before one
+        //      of them is waited for ----
         const int group = warp & 3;
         const bool ok = nkb <= 0 || mbar_wait(smem_u32(&acc_full), 0u);     // all MMAs done: the ring is free to reuse
         tc_fence_after();
         if (!ok && lane == 0 && s.error_flag) atomicExch(s.error_flag, 3);
         const uint32_t lane_addr = tmem_base + ((uint32_t)(group * 32) << 16);
         const int valid = min(s.n_tile, s.M - t0);
-        for (int c0 = 0; c0 < valid; c0 += 16) {
-            float acc[16], up[16];
+        const int live = (s.chains >= 2 && nkb < 2) ? s.chains / 2 : s.chains;   // the second issuer's stay untouched with one K block
+        for (int unit = (warp - DRAIN_WARP) >> 2; unit < (valid + 15) / 16 * A_TILES; unit += DRAIN_SETS) {
+            const int c0 = unit / A_TILES * 16, half = unit % A_TILES;
+            float acc[4][16];
             if (ok && nkb > 0) {
-                tmem_load16(lane_addr + (uint32_t)c0, acc);
-                if (MODE == GEMM_SWIGLU) tmem_load16(lane_addr + (uint32_t)(s.n_tile + c0), up);
-                const int live = (s.chains >= 2 && nkb < 2) ? s.chains / 2 : s.chains;   // the second issuer's stay untouched with one K block
-                for (int chain = 1; chain < live; ++chain) {              // in chain order: the same sum in every run
-                    float more[16];
-                    tmem_load16(lane_addr + (uint32_t)(chain * A_TILES * s.n_tile + c0), more);
+                const uint32_t column = lane_addr + (uint32_t)(half * s.n_tile + c0), step = (uint32_t)(A_TILES * s.n_tile);
+                tmem_load16_nowait(column, acc[0]);
+                if (live >= 2) tmem_load16_nowait(column + step, acc[1]);
+                if (live == 4) {
+                    tmem_load16_nowait(column + 2 * step, acc[2]);
+                    tmem_load16_nowait(column + 3 * step, acc[3]);
+                }
+                tmem_load_wait();
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) acc[c] += more[c];
-                    if (MODE == GEMM_SWIGLU) {
-                        tmem_load16(lane_addr + (uint32_t)(chain * A_TILES * s.n_tile + s.n_tile + c0), more);
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) up[c] += more[c];
+                for (int c = 0; c < 16; ++c) {                            // in chain order: the same sum in every run
+                    if (live >= 2) acc[0][c] += acc[1][c];
+                    if (live == 4) {
+                        acc[0][c] += acc[2][c];
+                        acc[0][c] += acc[3][c];
                     }
                 }
             } else {
 #pragma unroll
-                for (int c = 0; c < 16; ++c) acc[c] = up[c] = 0.f;
+                for (int c = 0; c < 16; ++c) acc[0][c] = 0.f;
             }
+            float* row = exchange + (size_t)c0 * ACC_W + half * TILE_F + group * 32 + lane;
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                if (c0 + c < valid) {
-                    exchange[(size_t)(c0 + c) * ACC_W + group * 32 + lane] = acc[c];
-                    if (MODE == GEMM_SWIGLU) exchange[(size_t)(c0 + c) * ACC_W + TILE_F + group * 32 + lane] = up[c];
-                }
-            }
+            for (int c = 0; c < 16; ++c)
+                if (c0 + c < valid) row[(size_t)c * ACC_W] = acc[0][c];
         }
     }
     tc_fence_before();
