@@ -339,6 +339,61 @@ __global__ void moe_combine_kernel(float* __restrict__ residual, const float* __
         *dst = store ? alpha * acc : fmaf(alpha, acc, *dst);
     }
 }
+
+// The same for rows of whole fours, a thread four elements: every row's loads are 16 bytes and a thread's choices are asked for
+// before the first is added (512 tokens of 2,048 elements, two choices and a shared expert: 21 MB mostly in L2, 6.6 us element by element,
+// 3.3 so; 64 tokens 5.3 and 1.6).
+template <typename T>
+__global__ void moe_combine4_kernel(float* __restrict__ residual, const float* __restrict__ y, const int* __restrict__ inverse,
+                                    const float* __restrict__ weights, const float* __restrict__ shared_y,
+                                    const float* __restrict__ shared_gate, const T* __restrict__ x, long long ld_x, int hidden, int top,
+                                    float alpha, int store) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (i >= hidden) return;
+    const int* rows = inverse + (size_t)t * top;
+    const float* w = weights + (size_t)t * top;
+    const float gate = shared_y ? (shared_gate ? shared_gate[t] : 1.f) : 0.f;
+    float4 shared = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (shared_y) shared = *reinterpret_cast<const float4*>(shared_y + (size_t)t * hidden + i);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c0 = 0; c0 < top; c0 += 4) {
+        float v[4][4], wc[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const bool there = c0 + c < top;
+            const int row = there ? rows[c0 + c] : -1;
+            wc[c] = there ? w[c0 + c] : 0.f;
+            float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (there && row >= 0) u = *reinterpret_cast<const float4*>(y + (size_t)row * hidden + i);
+            else if (there && x) {
+                // a choice without a row is an identity output: the token's own input
+                const T* own = x + (size_t)t * ld_x + i;
+                u = make_float4(to_float(own[0]), to_float(own[1]), to_float(own[2]), to_float(own[3]));
+            }
+            v[c][0] = u.x, v[c][1] = u.y, v[c][2] = u.z, v[c][3] = u.w;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (c0 + c < top) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[e] = fmaf(wc[c], v[c][e], acc[e]);
+            }
+    }
+    if (shared_y) {
+        const float s[4] = {shared.x, shared.y, shared.z, shared.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] = fmaf(gate, s[e], acc[e]);
+    }
+    float4* dst = reinterpret_cast<float4*>(residual + (size_t)t * hidden + i);
+    if (store) {
+        *dst = make_float4(alpha * acc[0], alpha * acc[1], alpha * acc[2], alpha * acc[3]);
+    } else {
+        const float4 old = *dst;
+        *dst = make_float4(fmaf(alpha, acc[0], old.x), fmaf(alpha, acc[1], old.y), fmaf(alpha, acc[2], old.z), fmaf(alpha, acc[3], old.w));
+    }
+}
 }  // namespace
 
 LIA_EXPORT int lia_moe_tile_rows() { return TILE_M; }
@@ -442,6 +497,15 @@ LIA_EXPORT int lia_moe_combine(float* residual, const float* y, const int* inver
     if (n <= 0) return LIA_OK;
     if (hidden <= 0 || top <= 0 || top > MOE_MAX_TOP || (x && ld_x < hidden)) return LIA_ERR_SIZE;
     const int threads = hidden >= 1024 ? 256 : 128;
+    if (hidden % 4 == 0 && n <= 65535 && (((uintptr_t)residual | (uintptr_t)y | (uintptr_t)shared_y) & 15u) == 0 &&
+        (!x || x_dtype == LIA_BF16 || x_dtype == LIA_F32)) {
+        const dim3 grid((hidden / 4 + threads - 1) / threads, n);
+        if (x && x_dtype == LIA_BF16)
+            return lia_launch(moe_combine4_kernel<__nv_bfloat16>, grid, dim3(threads), 0, stream, residual, y, inverse, weights, shared_y,
+                              shared_gate, (const __nv_bfloat16*)x, ld_x, hidden, top, alpha, store);
+        return lia_launch(moe_combine4_kernel<float>, grid, dim3(threads), 0, stream, residual, y, inverse, weights, shared_y,
+                          shared_gate, (const float*)x, ld_x, hidden, top, alpha, store);
+    }
     if (x && x_dtype == LIA_BF16)
         return lia_launch(moe_combine_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0, stream, residual, y, inverse, weights,
                           shared_y, shared_gate, (const __nv_bfloat16*)x, ld_x, hidden, top, alpha, store);
