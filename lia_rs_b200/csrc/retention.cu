@@ -7,7 +7,8 @@
 //  * `retention_encode` rotates q and k in place (element i of a head with i + rot_dims/2 over the first rot_dims
 //    elements, angle float(position) * freq[i]) and multiplies k by d^(-1/2) after the rotation.
 //  * Single tokens (`retention_single`): one CTA per (token, head) updates the state in place and forms o from it.
-//  * Prompt portions are cut into chunks of CHUNK tokens that run side by side, in three launches:
+//  * Prompt portions are cut into chunks of CHUNK tokens (LONG for heads of 64 or 128 elements) that run side by side, in three
+//    launches:
 //      sums    U_c = sum_j decay^(len-1-j) k_j v_j^T of each chunk, from zero;
 //      carry   along each portion: the state that each chunk starts from takes U_c's place in scratch,
 //              S <- decay^len S + U_c, and the last S goes back to the request's state;
@@ -177,6 +178,7 @@ retention_sums_kernel(const float* __restrict__ rows, long long ld, const float*
 }
 
 // along each portion: scratch[c] <- the state chunk c starts from; S <- decay^len S + U_c; state <- the last S
+template <int LENGTH>
 __global__ void __launch_bounds__(RET_THREADS)
 retention_carry_kernel(const float* __restrict__ decay, const int* __restrict__ segments, int n_segments,
                        const int* __restrict__ slots, float* __restrict__ sums, float* __restrict__ state,
@@ -189,11 +191,11 @@ retention_carry_kernel(const float* __restrict__ decay, const int* __restrict__ 
     const int slot = slots[first];
     if (slot < 0) return;
     int before = 0;
-    for (int p = 0; p < s; ++p) before += (segments[3 * p + 2] + CHUNK - 1) / CHUNK;
-    const int chunks = (count + CHUNK - 1) / CHUNK;
+    for (int p = 0; p < s; ++p) before += (segments[3 * p + 2] + LENGTH - 1) / LENGTH;
+    const int chunks = (count + LENGTH - 1) / LENGTH;
     const float log_a = log2f(decay[h]);
-    const float full = exp2f((float)CHUNK * log_a);
-    const float last = exp2f((float)(count - (chunks - 1) * CHUNK) * log_a);
+    const float full = exp2f((float)LENGTH * log_a);
+    const float last = exp2f((float)(count - (chunks - 1) * LENGTH) * log_a);
     const int size = d * dv;
     float* S = state + (size_t)slot * state_stride + (size_t)h * size;
     // (a thread walks its element's chunks eight at a time: the eight loads are in flight together)
@@ -369,6 +371,229 @@ retention_output_kernel(const float* __restrict__ rows, long long ld, const floa
     }
 }
 
+// ---- heads of 64 or 128 elements: chunks of LONG tokens, a thread a tile of eight by eight ----
+// The chunks' sums and their states pass through memory, so twice the tokens a chunk halve that traffic (2,048 tokens of 16 heads
+// of 128 x 128: 134 MB in place of 268); what a chunk costs more is the lower triangle of its score matrix.  The multiply-adds are
+// bound by the loads from shared memory beside them (128 bytes a cycle and SM), so a thread owns eight rows and up to eight columns:
+// sixteen numbers loaded for 64 multiply-adds, where four by four load eight for sixteen.  2,048 tokens of 16 heads of 128 x 128:
+// sums 42 -> 33 us (32 TFLOP/s), carry 33 -> 14 us (4.8 TB/s), outputs 141 -> 95 us (23 TFLOP/s;
+// bound by the shared-memory loads of three products one behind the other, two CTAs an SM).  The three launches in a row: 2 tokens
+// 31 -> 22 us, 33 tokens 53 -> 44, 300 tokens 70 -> 60, 2,048 tokens 215 -> 140.  Other head sizes, and rows that 16-byte loads
+// cannot read, keep the kernels above.
+constexpr int LONG = 64;
+
+// U [chunk, head, D, DV]: a CTA a chunk and head, the keys weighted as they come in.
+template <int D, int DV>
+__global__ void __launch_bounds__(256)
+retention_tile_sums_kernel(const float* __restrict__ rows, long long ld, const float* __restrict__ decay,
+                           const int* __restrict__ segments, int n_segments, float* __restrict__ sums, int heads) {
+    extern __shared__ __align__(16) float tile_sums_shared[];         // k [LONG][D] weighted, v [LONG][DV]
+    float* ks = tile_sums_shared;
+    float* vs = ks + LONG * D;
+    pdl_launch_dependents();
+    pdl_wait();
+    int first, len, segment, chunk;
+    if (!find_chunk<LONG>(segments, n_segments, blockIdx.x, &first, &len, &segment, &chunk)) return;
+    const int h = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int filled = (len + 3) & ~3;                                // rows that are brought (zeros behind the chunk's end)
+    const float* k = rows + (size_t)first * ld + (size_t)(heads + h) * D;
+    const float* v = rows + (size_t)first * ld + (size_t)2 * heads * D + (size_t)h * DV;
+#pragma unroll
+    for (int e = tid; e < LONG * (DV / 4); e += 256) {
+        const int t = e / (DV / 4), c = (e % (DV / 4)) * 4;
+        if (t < filled) bring16(vs + t * DV + c, v + (size_t)(t < len ? t : 0) * ld + c, t < len);
+    }
+    bring_commit();
+    const float log_a = log2f(decay[h]);
+#pragma unroll
+    for (int e = tid; e < LONG * (D / 4); e += 256) {
+        const int t = e / (D / 4), c = (e % (D / 4)) * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < len) x = scaled(*reinterpret_cast<const float4*>(k + (size_t)t * ld + c), exp2f((float)(len - 1 - t) * log_a));
+        if (t < filled) *reinterpret_cast<float4*>(ks + t * D + c) = x;
+    }
+    bring_wait<0>();
+    __syncthreads();
+    constexpr int RI = D / 64, CJ = DV / 64;
+    float acc[RI * 4][CJ * 4] = {};
+#pragma unroll 4
+    for (int t = 0; t < filled; ++t) {
+        float a[RI * 4], b[CJ * 4];
+#pragma unroll
+        for (int r = 0; r < RI; ++r) {
+            const float4 x = *reinterpret_cast<const float4*>(ks + t * D + r * 64 + ty * 4);
+            a[4 * r] = x.x, a[4 * r + 1] = x.y, a[4 * r + 2] = x.z, a[4 * r + 3] = x.w;
+        }
+#pragma unroll
+        for (int c = 0; c < CJ; ++c) {
+            const float4 x = *reinterpret_cast<const float4*>(vs + t * DV + c * 64 + tx * 4);
+            b[4 * c] = x.x, b[4 * c + 1] = x.y, b[4 * c + 2] = x.z, b[4 * c + 3] = x.w;
+        }
+#pragma unroll
+        for (int i = 0; i < RI * 4; ++i)
+#pragma unroll
+            for (int j = 0; j < CJ * 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    }
+    float* U = sums + ((size_t)blockIdx.x * heads + h) * D * DV;
+#pragma unroll
+    for (int i = 0; i < RI * 4; ++i)
+#pragma unroll
+        for (int c = 0; c < CJ; ++c)
+            *reinterpret_cast<float4*>(U + (size_t)((i / 4) * 64 + ty * 4 + (i & 3)) * DV + c * 64 + tx * 4) =
+                make_float4(acc[i][4 * c], acc[i][4 * c + 1], acc[i][4 * c + 2], acc[i][4 * c + 3]);
+}
+
+// The outputs of a chunk and head by 128 threads: warp w owns tokens 16 w .. 16 w + 15, a thread eight of them (every other one) and
+// four or eight columns, so the score matrix's rows stay inside the warp that made them and its keys behind the warp's last token
+// are never looked at.  The incoming state comes sixteen rows at a time, two stages ahead; the values take the keys' place.
+template <typename TO, int D, int DV>
+__global__ void __launch_bounds__(128)
+retention_tile_output_kernel(const float* __restrict__ rows, long long ld, const float* __restrict__ decay,
+                             const int* __restrict__ segments, int n_segments, const float* __restrict__ sums,
+                             TO* __restrict__ out, int heads, float eps) {
+    constexpr int LQ = D + 4, LV = DV + 4, LKV = LQ > LV ? LQ : LV, LA = LONG + 4, STEP = 16, CJ = DV / 64;
+    extern __shared__ __align__(16) float tile_out_shared[];
+    float* qs = tile_out_shared;                      // [LONG][LQ]
+    float* kv = qs + LONG * LQ;                       // [LONG][LKV]: the keys, later the values
+    float* As = kv + LONG * LKV;                      // [LONG][LA]
+    float* ss = As + LONG * LA;                       // [3][STEP][DV]
+    float* powers = ss + 3 * STEP * DV;               // [LONG + 1]
+    pdl_launch_dependents();
+    pdl_wait();
+    int first, len, segment, chunk;
+    if (!find_chunk<LONG>(segments, n_segments, blockIdx.x, &first, &len, &segment, &chunk)) return;
+    const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = lane & 15, odd = lane >> 4;
+    const float* chunk_rows = rows + (size_t)first * ld;
+    const float* S = sums + ((size_t)blockIdx.x * heads + h) * D * DV;
+#pragma unroll 4
+    for (int e = tid; e < LONG * (D / 4); e += 128) {
+        const int t = e / (D / 4), c = (e % (D / 4)) * 4;
+        const float* src = chunk_rows + (size_t)(t < len ? t : 0) * ld + c;
+        bring16(qs + t * LQ + c, src + (size_t)h * D, t < len);
+        bring16(kv + t * LQ + c, src + (size_t)(heads + h) * D, t < len);
+    }
+    bring_commit();
+    auto fetch_state = [&](int step) {
+        if (step < D / STEP)
+            for (int e = tid; e < STEP * (DV / 4); e += 128) bring16(ss + (step % 3) * STEP * DV + e * 4, S + (size_t)step * STEP * DV + e * 4, true);
+        bring_commit();
+    };
+    fetch_state(0);
+    fetch_state(1);
+    const float log_a = log2f(decay[h]);
+    if (tid <= LONG) powers[tid] = exp2f((float)tid * log_a);
+    bring_wait<2>();
+    __syncthreads();
+    const int t0 = warp * 16;                         // this thread's tokens: t0 + 2 i + odd
+    const bool here = t0 < len;                       // (a warp without tokens only brings rows and waits with the others)
+    const float* q0 = qs + (t0 + odd) * LQ;
+    // A[t][j] = decay^(t-j) q_t . k_j for j <= t: sixteen keys at a time up to the warp's own
+#pragma unroll 1
+    for (int jb = 0; here && jb <= warp; ++jb) {
+        float acc[8] = {};
+        const float* k0 = kv + (jb * 16 + tx) * LQ;
+#pragma unroll 4
+        for (int k = 0; k < D; k += 4) {
+            const float4 b = *reinterpret_cast<const float4*>(k0 + k);
+            float4 a[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(q0 + 2 * i * LQ + k);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = fmaf(a[i].x, b.x, acc[i]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = fmaf(a[i].y, b.y, acc[i]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = fmaf(a[i].z, b.z, acc[i]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = fmaf(a[i].w, b.w, acc[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = t0 + 2 * i + odd, j = jb * 16 + tx;
+            As[t * LA + j] = j <= t ? acc[i] * powers[t - j] : 0.f;
+        }
+    }
+    __syncthreads();                                  // every warp is done with the keys
+#pragma unroll 4
+    for (int e = tid; e < LONG * (DV / 4); e += 128) {
+        const int t = e / (DV / 4), c = (e % (DV / 4)) * 4;
+        bring16(kv + t * LV + c, chunk_rows + (size_t)(t < len ? t : 0) * ld + (size_t)2 * heads * D + (size_t)h * DV + c, t < len);
+    }
+    bring_commit();
+    float acc[8][CJ * 4] = {};
+    // o = decay^(t+1) q S_in  (groups in flight at step s: its own, the values and up to two later stages)
+#pragma unroll 1
+    for (int s = 0; s < D / STEP; ++s) {
+        if (s < 2) bring_wait<2>();
+        else bring_wait<1>();
+        __syncthreads();
+        fetch_state(s + 2);
+        if (here) multiply_tiles<8, CJ>(acc, q0 + s * STEP, LQ, ss + (s % 3) * STEP * DV + tx * 4, DV, STEP);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < CJ * 4; ++j) acc[i][j] *= powers[t0 + 2 * i + odd + 1];
+    bring_wait<0>();
+    __syncthreads();                                  // the values are there
+    if (!here) return;
+    // ... + A v, up to the warp's own tokens (rows behind the chunk's end are zeros)
+    multiply_tiles<8, CJ>(acc, As + (t0 + odd) * LA, LA, kv + tx * 4, LV, min(t0 + 16, (len + 3) & ~3));
+    // the head's norm over its DV elements (sixteen lanes share a token) and the gate
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = t0 + 2 * i + odd;
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < CJ * 4; ++j) sum = fmaf(acc[i][j], acc[i][j], sum);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        const float inv = 1.0f / sqrtf(sum / (float)DV + eps);
+        if (t < len) {
+            const float* g = chunk_rows + (size_t)t * ld + (size_t)2 * heads * D + (size_t)(heads + h) * DV + tx * 4;
+            TO* dst = out + (size_t)(first + t) * heads * DV + (size_t)h * DV + tx * 4;
+#pragma unroll
+            for (int c = 0; c < CJ; ++c) {
+                const float4 z = *reinterpret_cast<const float4*>(g + c * 64);
+                const float zs[4] = {z.x, z.y, z.z, z.w};
+                struct alignas(4 * sizeof(TO)) Four { TO v[4]; } f;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) f.v[e] = from_float<TO>(acc[i][4 * c + e] * inv * (zs[e] / (1.0f + expf(-zs[e]))));
+                *reinterpret_cast<Four*>(dst + c * 64) = f;
+            }
+        }
+    }
+}
+
+template <int D, int DV>
+constexpr size_t tile_output_bytes() {
+    return ((size_t)LONG * (D + 4) + LONG * ((D > DV ? D : DV) + 4) + LONG * (LONG + 4) + 3 * 16 * DV + LONG + 1) * sizeof(float);
+}
+
+// The three launches of the portions for heads of D and DV elements.
+template <typename TO, int D, int DV>
+int launch_tiles(const float* rows, long long ld, const float* decay, float* state, long long state_stride, const int* segments,
+                 int n_segments, int max_chunks, const int* slots, TO* out, int heads, float eps, float* scratch, cudaStream_t stream) {
+    constexpr size_t sums_bytes = (size_t)LONG * (D + DV) * sizeof(float), out_bytes = tile_output_bytes<D, DV>();
+    static std::atomic<bool> raised{false};
+    if (!raised.load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(retention_tile_sums_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sums_bytes) != cudaSuccess ||
+            cudaFuncSetAttribute(retention_tile_output_kernel<TO, D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return LIA_ERR_LAUNCH;
+        }
+        raised.store(true, std::memory_order_release);
+    }
+    int code = lia_launch(retention_tile_sums_kernel<D, DV>, dim3(max_chunks, heads), dim3(256), sums_bytes, stream, rows, ld, decay,
+                          segments, n_segments, scratch, heads);
+    if (code != LIA_OK) return code;
+    code = lia_launch(retention_carry_kernel<LONG>, dim3(n_segments, heads, D * DV / RET_THREADS), dim3(RET_THREADS), 0, stream, decay,
+                      segments, n_segments, slots, scratch, state, state_stride, heads, D, DV);
+    if (code != LIA_OK) return code;
+    return lia_launch(retention_tile_output_kernel<TO, D, DV>, dim3(max_chunks, heads), dim3(128), out_bytes, stream, rows, ld, decay,
+                      segments, n_segments, (const float*)scratch, out, heads, eps);
+}
+
 size_t output_shared_bytes(int d, int dv) {
     const int dp = (d + 3) & ~3, dvp = (dv + 3) & ~3;
     return ((size_t)2 * CHUNK * dp + (size_t)2 * CHUNK * dvp + CHUNK * CHUNK + CHUNK + 1) * sizeof(float);
@@ -414,6 +639,19 @@ LIA_EXPORT int lia_retention(const float* rows, long long ld, const float* decay
             return LIA_ERR_SIZE;
         const int dp = (d + 3) & ~3, dvp = (dv + 3) & ~3;
         const int vec = ((d | dv) & 3) == 0 && (ld & 3) == 0 && (((uintptr_t)rows | (uintptr_t)scratch) & 15u) == 0 ? 1 : 0;
+        // heads of 64 or 128 elements: longer chunks, of which there are no more than the caller made room for
+        const bool tiled = vec && (d == 64 || d == 128) && (dv == 64 || dv == 128) &&
+                           ((uintptr_t)out & (out_dtype == LIA_F32 ? 15u : 7u)) == 0;
+        if (tiled) {
+#define LIA_TILES(TO, D, DV)                                                                                                  \
+    launch_tiles<TO, D, DV>(rows, ld, decay, state, state_stride, segments, n_segments, max_chunks, slots, (TO*)out, heads, eps, scratch, stream)
+#define LIA_TILES_OF(TO)                                                                                                      \
+    (d == 64 ? (dv == 64 ? LIA_TILES(TO, 64, 64) : LIA_TILES(TO, 64, 128)) : (dv == 64 ? LIA_TILES(TO, 128, 64) : LIA_TILES(TO, 128, 128)))
+            code = out_dtype == LIA_F32 ? LIA_TILES_OF(float) : LIA_TILES_OF(__nv_bfloat16);
+#undef LIA_TILES_OF
+#undef LIA_TILES
+            if (code != LIA_OK) return code;
+        } else {
         const size_t sums_bytes = (size_t)CHUNK * (dp + dvp) * sizeof(float);
         const size_t out_bytes = output_shared_bytes(d, dv);
         static bool raised = false;
@@ -427,7 +665,7 @@ LIA_EXPORT int lia_retention(const float* rows, long long ld, const float* decay
                           decay, segments, n_segments, scratch, heads, d, dv, vec);
         if (code != LIA_OK) return code;
         const int parts = (d * dv + RET_THREADS - 1) / RET_THREADS;          // one element a thread
-        code = lia_launch(retention_carry_kernel, dim3(n_segments, heads, parts), dim3(RET_THREADS), 0, stream, decay,
+        code = lia_launch(retention_carry_kernel<CHUNK>, dim3(n_segments, heads, parts), dim3(RET_THREADS), 0, stream, decay,
                           segments, n_segments, slots, scratch, state, state_stride, heads, d, dv);
         if (code != LIA_OK) return code;
         if (out_dtype == LIA_F32)
@@ -438,6 +676,7 @@ LIA_EXPORT int lia_retention(const float* rows, long long ld, const float* decay
                               stream, rows, ld, decay, segments, n_segments, (const float*)scratch, (__nv_bfloat16*)out,
                               heads, d, dv, eps, vec);
         if (code != LIA_OK) return code;
+        }
     }
     if (n_single > 0) {
         const size_t bytes = ((size_t)2 * d + (dv > RET_THREADS ? dv : RET_THREADS)) * sizeof(float);
