@@ -246,29 +246,58 @@ latent_attention_kernel(LatentParams p) {
     }
 }
 
-// out[h, t] = sum_s 2^(m_s - M) O_s / sum_s 2^(m_s - M) l_s over the ranges that saw a key, in ascending order.
-__global__ void latent_merge_kernel(LatentParams p) {
+// out[h, t] = sum_s 2^(m_s - M) O_s / sum_s 2^(m_s - M) l_s over the ranges that saw a key, in ascending order.  A thread owns four
+// columns; the ranges' maxima and sums are read once, and eight ranges' columns are asked for before the first is added (nine
+// ranges of 32 tokens and 16 heads, rank 512: 12.7 us when every thread walked the ranges one load behind the other, 4.3 so).
+__global__ void __launch_bounds__(128) latent_merge_kernel(LatentParams p) {
     pdl_launch_dependents();
     pdl_wait();
-    const int t = blockIdx.x, h = blockIdx.y;
+    const int t = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
+    const int c = threadIdx.x * 4;                            // (rank is a multiple of 32 of at most 512)
     if (p.slots[p.rows ? p.rows[t] : t] < 0) return;
     const size_t planes = (size_t)p.heads * p.n_tokens, plane = (size_t)h * p.n_tokens + t;
-    const float* ms = p.partial + (size_t)p.splits * planes * p.rank;
-    float top = -INFINITY;
-    for (int s = 0; s < p.splits; ++s) top = fmaxf(top, ms[((size_t)s * planes + plane) * 2]);
+    const float* ms = p.partial + (size_t)p.splits * planes * p.rank + plane * 2;
+    // (lane s holds ranges s and s + 32)
+    float2 low = make_float2(-INFINITY, 0.f), high = make_float2(-INFINITY, 0.f);
+    if (lane < p.splits) low = *reinterpret_cast<const float2*>(ms + (size_t)lane * planes * 2);
+    if (lane + 32 < p.splits) high = *reinterpret_cast<const float2*>(ms + (size_t)(lane + 32) * planes * 2);
+    const float top = warp_max(fmaxf(low.x, high.x));
+    const uint32_t seen_low = __ballot_sync(0xffffffffu, low.x > -INFINITY), seen_high = __ballot_sync(0xffffffffu, high.x > -INFINITY);
+    const float w_low = low.x > -INFINITY ? exp2f(low.x - top) : 0.f, w_high = high.x > -INFINITY ? exp2f(high.x - top) : 0.f;
     float total = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-        const float m = ms[((size_t)s * planes + plane) * 2];
-        if (m > -INFINITY) total += exp2f(m - top) * ms[((size_t)s * planes + plane) * 2 + 1];
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* o = p.partial + plane * p.rank + c;
+    for (int s0 = 0; s0 < p.splits; s0 += 8) {
+        float2 v[8][2];
+        float w[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int s = s0 + k;
+            const float a = __shfl_sync(0xffffffffu, w_low, s & 31), b = __shfl_sync(0xffffffffu, w_high, s & 31);
+            const float la = __shfl_sync(0xffffffffu, low.y, s & 31), lb = __shfl_sync(0xffffffffu, high.y, s & 31);
+            const bool seen = ((s < 32 ? seen_low : seen_high) >> (s & 31)) & 1;     // (a range that saw no key has left no columns)
+            w[k] = s < 32 ? a : b;
+            if (seen) total = fmaf(w[k], s < 32 ? la : lb, total);
+            v[k][0] = v[k][1] = make_float2(0.f, 0.f);
+            if (seen && c < p.rank) {
+                const float* columns = o + (size_t)s * planes * p.rank;               // (8-byte aligned)
+                v[k][0] = *reinterpret_cast<const float2*>(columns);
+                v[k][1] = *reinterpret_cast<const float2*>(columns + 2);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            acc[0] = fmaf(w[k], v[k][0].x, acc[0]);
+            acc[1] = fmaf(w[k], v[k][0].y, acc[1]);
+            acc[2] = fmaf(w[k], v[k][1].x, acc[2]);
+            acc[3] = fmaf(w[k], v[k][1].y, acc[3]);
+        }
     }
     const float inv = total > 0.f ? 1.0f / total : 0.f;
-    for (int c = threadIdx.x; c < p.rank; c += blockDim.x) {
-        float acc = 0.f;
-        for (int s = 0; s < p.splits; ++s) {
-            const float m = ms[((size_t)s * planes + plane) * 2];
-            if (m > -INFINITY) acc += exp2f(m - top) * p.partial[((size_t)s * planes + plane) * p.rank + c];
-        }
-        p.out[plane * p.rank + c] = __float2bfloat16_rn(acc * inv);
+    if (c < p.rank) {
+        uint32_t* dst = reinterpret_cast<uint32_t*>(p.out + plane * p.rank + c);
+        dst[0] = pack2(acc[0] * inv, acc[1] * inv);
+        dst[1] = pack2(acc[2] * inv, acc[3] * inv);
     }
 }
 

@@ -10,7 +10,8 @@ from test_botuvik_parts_gpu import PartRunner
 pytestmark = pytest.mark.gpu
 F64 = torch.float64
 # eight values are rounded to bfloat16 on the way (queries, latents, keys, values, probabilities, outputs and the two products'
-# operands), each by at most 2^-9 of itself, and the result is linear in each: 8 * 2^-9 of its size at most, in any norm
+# operands), each by at most 2^-8 of itself and by less than 2^-9 in the root mean square (a uniform error over the numbers between
+# two powers of two: 0.41 * 2^-8), and the result is linear in each: 8 * 2^-9 of its size in the Euclidean norm, if all add up
 REL = 8 * 2.0 ** -9
 
 
