@@ -30,7 +30,8 @@ constexpr int MOE_MAX_EXPERTS = 1024, MOE_MAX_TOP = 32;
 
 // TOKENS tokens a CTA: a router row is read once for all of them.  A score's additions have the same order whatever TOKENS is.
 template <typename T, int TOKENS>
-__global__ void moe_route_kernel(const T* __restrict__ x, long long ld, const float* __restrict__ router, int n, int hidden,
+__global__ void __launch_bounds__(1024)
+moe_route_kernel(const T* __restrict__ x, long long ld, const float* __restrict__ router, int n, int hidden,
                                  int experts, int top, float scale, int extra, const float* __restrict__ correction,
                                  int groups, int keep, int renormalise, int sigmoid, int two_best, int* __restrict__ ids,
                                  float* __restrict__ weights, float* __restrict__ shared_gate) {
@@ -418,20 +419,30 @@ LIA_EXPORT int lia_moe_route(const void* x, int dtype, long long ld, const float
         cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(moe_route_kernel<float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(moe_route_kernel<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         raised = true;
     }
-    const bool many = n >= 4 * 148 && 4 * one <= 200 * 1024;
-    const int threads = many || experts + extra <= 8 ? 256 : experts + extra <= 16 ? 512 : 1024;      // (few tokens: a warp an output)
+    // As many tokens a CTA (up to four) as keep the CTAs resident at once, two an SM with up to 16 outputs, one with more: the router's
+    // rows come from L2 once a CTA.  Hidden size 2,048, us with one token a CTA (256 to 1,024 threads; four a CTA of 256 threads from 592
+    // tokens) and so: 9 outputs 300 tokens 9.8 -> 6.1, 512 tokens 10.2 -> 6.2, 1,024 tokens 13.6 -> 8.4; 65 outputs 200 tokens
+    // 19.4 -> 12.8, 512 tokens 38 -> 19.5, 1,024 tokens 47 -> 38.
+    const int resident = experts + extra <= 16 ? 2 * 148 : 148;
+    int tokens = n <= resident ? 1 : n <= 2 * resident ? 2 : 4;
+    while (tokens > 1 && tokens * one > 200 * 1024) tokens /= 2;
+    const int threads = experts + extra <= 8 ? 256 : experts + extra <= 16 ? 512 : 1024;
 #define LIA_ROUTE(T, TOKENS)                                                                                             \
     return lia_launch(moe_route_kernel<T, TOKENS>, dim3((n + TOKENS - 1) / TOKENS), dim3(threads), TOKENS * one, stream,     \
                       (const T*)x, ld, router, n, hidden, experts, top, scale, extra, correction, groups, keep,          \
                       renormalise, sigmoid, two_best, ids, weights, shared_gate)
     if (dtype == LIA_F32) {
-        if (many) LIA_ROUTE(float, 4);
+        if (tokens == 4) LIA_ROUTE(float, 4);
+        if (tokens == 2) LIA_ROUTE(float, 2);
         LIA_ROUTE(float, 1);
     }
     if (dtype == LIA_BF16) {
-        if (many) LIA_ROUTE(__nv_bfloat16, 4);
+        if (tokens == 4) LIA_ROUTE(__nv_bfloat16, 4);
+        if (tokens == 2) LIA_ROUTE(__nv_bfloat16, 2);
         LIA_ROUTE(__nv_bfloat16, 1);
     }
 #undef LIA_ROUTE
