@@ -29,20 +29,20 @@ using namespace tc5;
 namespace {
 // Sixteen warps: behind the last product everything waits for memory of some kind (the accumulators, the neighbours' shared memory,
 // the residual row), so the items of the sum are cut over as many threads as the registers allow.  224 threads, of which four warps
-// emptied the accumulators load by load, took at 64 tokens (2B-class layer) q|k|v 8.8, o 7.4, gate/up 19.5, down 12.2 us; now 8.4, 7.0,
-// 18.1, 11.8; at 128 tokens 11.9, 9.3, 23.2, 15.5 and now 10.5, 8.6, 20.6, 14.8; at 17 tokens the same.
+// emptied the accumulators load by load, took at 64 tokens (2B-class layer) q|k|v 8.8, o 7.4, gate/up 19.5, down 12.2 us; so 8.4, 7.0,
+// 18.1, 11.8; at 128 tokens 11.9, 9.3, 23.2, 15.5 and so 10.5, 8.6, 20.6, 14.8; at 17 tokens the same.
 constexpr int THREADS = 512;            // warp 0: TMA, warps 1 and 2: MMA, warps 4-15: accumulator to shared memory
 constexpr int DRAIN_WARP = 4, DRAIN_SETS = 3;      // first of the warps that empty the accumulators; sets of four such warps
 constexpr int MAX_STAGES = 12;
 constexpr int MAX_CLUSTER = 8;
-constexpr int SMEM_LIMIT = 200 * 1024;
+constexpr int SMEM_LIMIT = 224 * 1024;
 
 struct Shape {
     int M, N, K;
     int n_tile;               // tokens per tile: a multiple of 16, at most 128
-    int box_rows;             // rows of W per TMA box (divides 128, a multiple of 8)
     int stages, batch, kblocks, splits, f_tiles, t_tiles;   // batch: K blocks whose W boxes are issued together
     int tmem_cols;
+    int fours;                // groups of four features in a tile: 32
     int chains;               // accumulators that take the K steps in turn (1, 2 or 4)
     int ldo, vector_ok;       // vector_ok: rows of out may be stored 4 elements at a time
     float alpha;
@@ -123,19 +123,16 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     if (warp == 0 && lane == 0) {
         // ---- TMA producer: W at once, X when the kernel ahead has finished ----
-        // W comes in boxes of 8 rows x 64 k (one 1024-byte swizzle atom each), issued k-major inside a
-        // batch of K blocks: consecutive requests then read consecutive 128-byte pieces of the same 8
-        // rows of W, which is what DRAM pages want; a 128-row box per K block would touch 128 rows
-        // before it came back to the first.
+        // (a batch's boxes are issued tile by tile of W, so that consecutive requests read consecutive 128-byte pieces of the
+        // same rows)
         auto issue_w = [&](int it0, int count) {
             for (int j = 0; j < count; ++j) mbar_expect_tx(smem_u32(&full_bar[(it0 + j) % s.stages]), stage_bytes);
             for (int a = 0; a < A_TILES; ++a)
-                for (int g = 0; g < TILE_F / s.box_rows; ++g)
-                    for (int j = 0; j < count; ++j) {
-                        const int st = (it0 + j) % s.stages;
-                        tma_load_2d(smem_base + (uint32_t)st * stage_bytes + (uint32_t)a * a_bytes + (uint32_t)(g * s.box_rows) * 128u, &map_w,
-                                    (kb_begin + it0 + j) * BLOCK_K, a * s.N + f0 + g * s.box_rows, smem_u32(&full_bar[st]));
-                    }
+                for (int j = 0; j < count; ++j) {
+                    const int st = (it0 + j) % s.stages;
+                    tma_load_2d(smem_base + (uint32_t)st * stage_bytes + (uint32_t)a * a_bytes, &map_w, (kb_begin + it0 + j) * BLOCK_K,
+                                a * s.N + f0, smem_u32(&full_bar[st]));
+                }
         };
         auto issue_x = [&](int it0, int count) {
             for (int j = 0; j < count; ++j) {
@@ -253,9 +250,12 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const int valid = min(s.n_tile, s.M - t0);
         const int mine = valid > (int)rank ? (valid - (int)rank + s.splits - 1) / s.splits : 0;
         const uint32_t exchange_addr = smem_base;
-        for (int item = threadIdx.x; item < mine * (TILE_F / 4); item += THREADS) {
-            const int tl = (int)rank + (item / (TILE_F / 4)) * s.splits;
-            const int q = item % (TILE_F / 4);
+        // (a plain product's loop is better compiled with the count of fours unknown, q|k|v at 64 tokens 7.8 against 8.3 us; a gated
+        // one's, which has twice the loads, with it known, 16.3 against 16.6)
+        const int fours = MODE == GEMM_SWIGLU ? TILE_F / 4 : s.fours;
+        for (int item = threadIdx.x; item < mine * fours; item += THREADS) {
+            const int tl = (int)rank + (item / fours) * s.splits;
+            const int q = item % fours;
             const int f = f0 + q * 4;
             if (f >= s.N) continue;
             const uint32_t at = exchange_addr + (uint32_t)((tl * ACC_W + q * 4) * 4);
@@ -437,17 +437,18 @@ LIA_EXPORT int lia_gemm_cluster(int mode, const void* X, int ldx, const void* W,
     const int longest = (s.kblocks + plan.splits - 1) / plan.splits;
     s.stages = max(1, min(min(MAX_STAGES, longest), SMEM_LIMIT / stage_bytes));
     s.batch = s.stages;
-    if (longest > s.stages && s.stages >= 2) {       // the ring is used again: two batches, one lands while the other is multiplied
-        s.batch = s.stages / 2;
-        s.stages = 2 * s.batch;
-    }
+    s.fours = TILE_F / 4;
+    // The ring is used again: half of it lands while the other half is multiplied.  As many stages as there is room for, an odd number
+    // too (200 KB and an even number: gate/up of a 2B-class layer at 17 / 64 / 128 tokens 16.5 / 18.1 / 20.6 us, down 10.5 / 11.7 /
+    // 14.8; so 13.7 / 16.3 / 19.5 and 9.8 / 11.2 / 13.7).  Single stages as they fall free give up what consecutive boxes of the same
+    // rows of W save: 17.1 / 19.2 / 22.1 and 11.7 / 13.7 / 16.4.
+    if (longest > s.stages && s.stages >= 2) s.batch = s.stages / 2;
     const int smem = max(s.stages * stage_bytes, exchange_bytes) + 1024;
     if (smem > SMEM_LIMIT + 1024) return LIA_ERR_SIZE;
 
     CUtensorMap mw, mx;
     int rc;
-    s.box_rows = TILE_F;
-    if ((rc = make_map(&mw, W, swiglu ? 2 * N : N, K, ldw, s.box_rows)) != LIA_OK) return rc;
+    if ((rc = make_map(&mw, W, swiglu ? 2 * N : N, K, ldw, TILE_F)) != LIA_OK) return rc;
     if ((rc = make_map(&mx, X, M, K, ldx, plan.n_tile)) != LIA_OK) return rc;
     if (mode == GEMM_STORE && out_dtype == LIA_F32) return launch<GEMM_STORE, float>(mw, mx, (float*)out, s, smem, stream);
     if (mode == GEMM_STORE) return launch<GEMM_STORE, __nv_bfloat16>(mw, mx, (__nv_bfloat16*)out, s, smem, stream);
