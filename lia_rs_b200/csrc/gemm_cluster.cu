@@ -41,6 +41,7 @@ struct Shape {
     int M, N, K;
     int n_tile;               // tokens per tile: a multiple of 16, at most 128
     int stages, batch, kblocks, splits, f_tiles, t_tiles;   // batch: K blocks whose W boxes are issued together
+    int bars;                 // full barriers that the K blocks take in turn: a multiple of the stages (see ring_of)
     int tmem_cols;
     int fours;                // groups of four features in a tile: 32
     int chains;               // accumulators that take the K steps in turn (1, 2 or 4)
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     TO* __restrict__ out, Shape s) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], acc_full;
+    __shared__ __align__(8) uint64_t full_bar[2 * MAX_STAGES], empty_bar[MAX_STAGES], acc_full;
     __shared__ uint32_t tmem_base_slot;
 
     constexpr int A_TILES = (MODE == GEMM_SWIGLU) ? 2 : 1;
@@ -99,10 +100,8 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const int nkb = kb_end - kb_begin;
 
     if (warp == 0 && lane == 0) {
-        for (int i = 0; i < s.stages; ++i) {
-            mbar_init(smem_u32(&full_bar[i]), 1);
-            mbar_init(smem_u32(&empty_bar[i]), 1);
-        }
+        for (int i = 0; i < s.bars; ++i) mbar_init(smem_u32(&full_bar[i]), 1);
+        for (int i = 0; i < s.stages; ++i) mbar_init(smem_u32(&empty_bar[i]), 1);
         mbar_init(smem_u32(&acc_full), s.chains >= 2 ? 2 : 1);       // one arrival per MMA issuer
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
@@ -126,19 +125,19 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // (a batch's boxes are issued tile by tile of W, so that consecutive requests read consecutive 128-byte pieces of the
         // same rows)
         auto issue_w = [&](int it0, int count) {
-            for (int j = 0; j < count; ++j) mbar_expect_tx(smem_u32(&full_bar[(it0 + j) % s.stages]), stage_bytes);
+            for (int j = 0; j < count; ++j) mbar_expect_tx(smem_u32(&full_bar[(it0 + j) % s.bars]), stage_bytes);
             for (int a = 0; a < A_TILES; ++a)
                 for (int j = 0; j < count; ++j) {
                     const int st = (it0 + j) % s.stages;
                     tma_load_2d(smem_base + (uint32_t)st * stage_bytes + (uint32_t)a * a_bytes, &map_w, (kb_begin + it0 + j) * BLOCK_K,
-                                a * s.N + f0, smem_u32(&full_bar[st]));
+                                a * s.N + f0, smem_u32(&full_bar[(it0 + j) % s.bars]));
                 }
         };
         auto issue_x = [&](int it0, int count) {
             for (int j = 0; j < count; ++j) {
                 const int st = (it0 + j) % s.stages;
                 tma_load_2d(smem_base + (uint32_t)st * stage_bytes + A_TILES * a_bytes, &map_x, (kb_begin + it0 + j) * BLOCK_K, t0,
-                            smem_u32(&full_bar[st]));
+                            smem_u32(&full_bar[(it0 + j) % s.bars]));
             }
         };
         const int ahead = min(nkb, s.stages);
@@ -159,13 +158,14 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (!ok) {
             if (s.error_flag) atomicExch(s.error_flag, 3);
             for (int i = max(0, issued - s.stages); i < issued; ++i)      // copies in flight must land before the CTA may end
-                mbar_wait(smem_u32(&full_bar[i % s.stages]), (uint32_t)(i / s.stages) & 1u);
+                mbar_wait(smem_u32(&full_bar[i % s.bars]), (uint32_t)(i / s.bars) & 1u);
         }
     } else if ((warp == 1 || warp == 2) && lane == 0) {
         // ---- MMA issuers.  Issuing one tcgen05.mma costs a thread some 130 cycles, four times what a tile this
         //      narrow computes for, so two threads issue: they take the K blocks in turn, each into accumulators of
         //      its own (an MMA that adds to the accumulator of the one before it would wait for it, too).  The
-        //      epilogue adds the accumulators up in a fixed order. ----
+        //      epilogue adds the accumulators up in a fixed order.  An issuer does not wait for the blocks it skips, so
+        //      every full barrier has one issuer that waits for all its fills in turn (their number is even) ----
         const int issuers = s.chains >= 2 ? 2 : 1;
         const int me = warp - 1;
         const int own = s.chains / issuers;                   // accumulators of this issuer
@@ -173,15 +173,15 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         bool ok = true;
         int mine = 0;                                         // K blocks this issuer has taken
         if (me < issuers) {
-            // (the stage and its phase are counted along, and the descriptors are the first stage's plus an offset in
+            // (the stage, the barrier and its phase are counted along, and the descriptors are the first stage's plus an offset in
             // their lowest field, the start address in 16-byte units: what this thread does between two MMAs is
             // what a K block of a narrow tile takes)
             const uint64_t desc_a0 = smem_desc(smem_base), desc_b0 = smem_desc(smem_base + A_TILES * a_bytes);
             const uint32_t stage_step = stage_bytes >> 4, a_step = a_bytes >> 4;
-            int st = me % s.stages;
-            uint32_t phase = (uint32_t)(me / s.stages) & 1u;
+            int st = me % s.stages, bar = me % s.bars;
+            uint32_t phase = (uint32_t)(me / s.bars) & 1u;
             for (int it = me; it < nkb; it += issuers, ++mine) {
-                if (!mbar_wait(smem_u32(&full_bar[st]), phase)) { ok = false; break; }
+                if (!mbar_wait(smem_u32(&full_bar[bar]), phase)) { ok = false; break; }
                 tc_fence_after();
                 const uint64_t da0 = desc_a0 + (uint64_t)((uint32_t)st * stage_step), db0 = desc_b0 + (uint64_t)((uint32_t)st * stage_step);
 #pragma unroll
@@ -194,7 +194,9 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 }
                 tc_commit(smem_u32(&empty_bar[st]));
                 st += issuers;
-                while (st >= s.stages) { st -= s.stages; phase ^= 1u; }
+                while (st >= s.stages) st -= s.stages;
+                bar += issuers;
+                while (bar >= s.bars) { bar -= s.bars; phase ^= 1u; }
             }
             if (ok) tc_commit(smem_u32(&acc_full));
             else if (s.error_flag) atomicExch(s.error_flag, 3);
@@ -368,6 +370,29 @@ Plan make_plan(int M, int N, int K, int sm_count) {
     return p;
 }
 
+// The ring of one CTA for `longest` K blocks: how many stages, over how many accumulators the K steps go, K blocks a batch, and how
+// many full barriers the blocks take in turn.
+// The ring is used again: half of it lands while the other half is multiplied.  As many stages as there is room for, an odd number
+// too (200 KB and an even number: gate/up of a 2B-class layer at 17 / 64 / 128 tokens 16.5 / 18.1 / 20.6 us, down 10.5 / 11.7 /
+// 14.8; so 13.7 / 16.3 / 19.5 and 9.8 / 11.2 / 13.7).  Single stages as they fall free give up what consecutive boxes of the same
+// rows of W save: 17.1 / 19.2 / 22.1 and 11.7 / 13.7 / 16.4.
+// An odd ring hands a stage from one of two issuers to the other, and a wait by parity cannot tell the fill that is wanted from the
+// one two fills before: an issuer that skips a fill could pass early and multiply what has not landed.  Then twice as many barriers
+// as stages, of which each belongs to one issuer.
+struct Ring {
+    int stages, chains, batch, bars;
+};
+Ring ring_of(bool swiglu, int n_tile, int longest) {
+    Ring r;
+    const int a_tiles = swiglu ? 2 : 1, stage_bytes = a_tiles * TILE_F * BLOCK_K * 2 + n_tile * BLOCK_K * 2;
+    r.chains = 4;
+    while (r.chains > 1 && r.chains * a_tiles * n_tile > 512) r.chains /= 2;
+    r.stages = max(1, min(min(MAX_STAGES, longest), SMEM_LIMIT / stage_bytes));
+    r.batch = longest > r.stages && r.stages >= 2 ? r.stages / 2 : r.stages;
+    r.bars = r.chains >= 2 && r.stages % 2 ? 2 * r.stages : r.stages;
+    return r;
+}
+
 template <int MODE, typename TO>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, TO* out, const Shape& s, int smem, cudaStream_t stream) {
     static int configured = 0;
@@ -407,6 +432,14 @@ LIA_EXPORT int lia_gemm_cluster_splits(int mode, int M, int N, int K, int sm_cou
     return make_plan(M, N, K, sm_count).splits;
 }
 
+// The ring of a CTA with tiles of `n_tile` tokens and `longest` K blocks: stages, full barriers, MMA issuers, K blocks a batch.
+LIA_EXPORT int lia_gemm_cluster_ring(int gated, int n_tile, int longest, int* out) {
+    if (n_tile < 16 || n_tile > 128 || n_tile % 16 || longest <= 0 || !out) return LIA_ERR_SIZE;
+    const Ring r = ring_of(gated != 0, n_tile, longest);
+    out[0] = r.stages; out[1] = r.bars; out[2] = r.chains >= 2 ? 2 : 1; out[3] = r.batch;
+    return LIA_OK;
+}
+
 // Arguments as lia_gemm_tc without the scratch.  Refuses (LIA_ERR_SIZE) a product that
 // lia_gemm_cluster_splits gives fewer than 2 CTAs per cluster, K or row strides that are not multiples of
 // 8 elements, and (LIA_ERR_ALIGN) pointers that are not 16-byte aligned.
@@ -426,23 +459,16 @@ LIA_EXPORT int lia_gemm_cluster(int mode, const void* X, int ldx, const void* W,
     s.M = M; s.N = N; s.K = K;
     s.n_tile = plan.n_tile; s.splits = plan.splits; s.f_tiles = plan.f_tiles; s.t_tiles = plan.t_tiles;
     s.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
-    s.chains = 4;
-    while (s.chains > 1 && s.chains * (swiglu ? 2 : 1) * plan.n_tile > 512) s.chains /= 2;
+    const int longest = (s.kblocks + plan.splits - 1) / plan.splits;
+    const Ring ring = ring_of(swiglu, plan.n_tile, longest);
+    s.stages = ring.stages; s.chains = ring.chains; s.batch = ring.batch; s.bars = ring.bars;
     s.tmem_cols = pow2_columns(s.chains * (swiglu ? 2 : 1) * plan.n_tile);
     s.ldo = ldo; s.alpha = alpha; s.error_flag = error_flag;
     const int esize = out_dtype == LIA_F32 ? 4 : 2;
     s.vector_ok = (((uintptr_t)out % (4 * esize)) == 0 && ldo % 4 == 0) ? 1 : 0;
     const int stage_bytes = (swiglu ? 2 : 1) * TILE_F * BLOCK_K * 2 + plan.n_tile * BLOCK_K * 2;
     const int exchange_bytes = plan.n_tile * TILE_F * (swiglu ? 2 : 1) * 4;
-    const int longest = (s.kblocks + plan.splits - 1) / plan.splits;
-    s.stages = max(1, min(min(MAX_STAGES, longest), SMEM_LIMIT / stage_bytes));
-    s.batch = s.stages;
     s.fours = TILE_F / 4;
-    // The ring is used again: half of it lands while the other half is multiplied.  As many stages as there is room for, an odd number
-    // too (200 KB and an even number: gate/up of a 2B-class layer at 17 / 64 / 128 tokens 16.5 / 18.1 / 20.6 us, down 10.5 / 11.7 /
-    // 14.8; so 13.7 / 16.3 / 19.5 and 9.8 / 11.2 / 13.7).  Single stages as they fall free give up what consecutive boxes of the same
-    // rows of W save: 17.1 / 19.2 / 22.1 and 11.7 / 13.7 / 16.4.
-    if (longest > s.stages && s.stages >= 2) s.batch = s.stages / 2;
     const int smem = max(s.stages * stage_bytes, exchange_bytes) + 1024;
     if (smem > SMEM_LIMIT + 1024) return LIA_ERR_SIZE;
 

@@ -63,6 +63,7 @@ class _Signatures:
                    c_void_p, ctypes.c_longlong, c_int, c_float, c_float, c_void_p, c_void_p]
     lia_gemm_cluster = [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                         c_int, c_void_p, c_void_p]
+    lia_gemm_cluster_ring = [c_int, c_int, c_int, c_void_p]
     lia_gemm_cluster_splits = [c_int, c_int, c_int, c_int, c_int]
     lia_gemm_skinny = [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                        c_void_p, c_void_p]
@@ -504,6 +505,14 @@ def gemm_cluster(mode, a, w, out, alpha: float = 1.0, error_flag=None, label=Non
     with _timed("gemm_cluster", label, work=lambda: _gemm_work(a, w, out)):
         _check(lib().lia_gemm_cluster(mode, _p(a), a.stride(0), _p(w), w.stride(0), _p(out), dtype_code(out.dtype),
                                       out.stride(0), M, N, K, alpha, sms, _p(error_flag), _stream()), "gemm_cluster")
+
+
+def gemm_cluster_ring(gated: bool, n_tile: int, blocks: int) -> tuple:
+    """(stages, full barriers, MMA issuers, K blocks a batch) of a CTA of the cluster kernel with tiles of `n_tile` tokens and
+    `blocks` K blocks."""
+    found = (c_int * 4)()
+    _check(lib().lia_gemm_cluster_ring(1 if gated else 0, n_tile, blocks, found), "gemm_cluster_ring")
+    return tuple(found)
 
 
 def bind_product(kernel: str, mode, a, w, out):
