@@ -220,7 +220,11 @@ class LatentAttention(Mixer):
              "k_up": "uk", "v_up": "uv", "gate": "g", "o": "o"}
 
     def graph_key(self, ctx) -> tuple:
-        return self._expansion(ctx) or ()
+        # (the plan with what it follows from beside the step: layers of other windows or sizes plan the same step differently, and
+        # a model keeps each distinct answer once)
+        if not ctx.n_prefill_segments or not self.per_tile:
+            return ()
+        return ((self.window, self.per_tile, self.heads * (self.d + self.dr + self.dv), self._expansion(ctx)),)
 
     @staticmethod
     def _names(params, prefix):

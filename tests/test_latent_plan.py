@@ -1,0 +1,27 @@
+"""How a step's prompt portions attend through a latent, decided on the host: what a captured step is replayed for."""
+from types import SimpleNamespace
+
+from lia_rs_b200.models.decoder import DecoderModel
+from lia_rs_b200.parts.softmax_attention import LatentAttention
+
+
+def layer(window):
+    part = LatentAttention.__new__(LatentAttention)
+    part.window, part.per_tile, part.heads, part.d, part.dr, part.dv = window, 128, 16, 128, 64, 128
+    return part
+
+
+def step(start, count=2048, page_size=16):
+    cache = SimpleNamespace(page_size=page_size)
+    return SimpleNamespace(n_tokens=count, n_out=1, context_bucket=4096, n_single=0, n_prefill_segments=1,
+                           segments=[(0, start, count, 0)], runtime=SimpleNamespace(cache=cache))
+
+
+def test_steps_of_one_graph_key_have_the_same_plans():
+    layers = [layer(None), layer(128), layer(256)]
+    model = SimpleNamespace(_key_layers=layers)
+    plans = {}
+    for start in list(range(200, 400)) + list(range(0, 40000, 97)):
+        ctx = step(start)
+        plan = [part._expansion(ctx) for part in layers]
+        assert plans.setdefault(DecoderModel.graph_key(model, ctx), plan) == plan, start
