@@ -45,6 +45,8 @@ _MOST_BOUND = 1024     # sizes kept; beyond, all are looked up anew (a step's si
 
 
 def _choose(mode, a, w, out) -> int:
+    if not (a.is_cuda and a.get_device() == w.get_device() == out.get_device()):
+        raise ops.KernelError("a product's tensors lie on one CUDA device")
     tensor_cores = ops.gemm_tc_accepts(mode, a, w, out)
     few = ops.gemm_skinny_accepts(mode, a, w, out)
     if a.shape[0] <= ops.STREAM_MAX_TOKENS and ops.gemm_stream_accepts(mode, a, w, out):
@@ -61,6 +63,9 @@ def _choose(mode, a, w, out) -> int:
 
 
 def _bind(choice, key, mode, a, w, out):
+    """Keep a product that has just been checked and launched, for calls of the same key."""
+    if not a.get_device() == w.get_device() == out.get_device():
+        return
     if len(_bound) >= _MOST_BOUND:
         _bound.clear()
     _bound[key] = ops.bind_product(_BOUND_KERNELS[choice], mode, a, w, out)
@@ -100,9 +105,10 @@ def linear(runtime, mode: int, a: torch.Tensor, w: torch.Tensor, out: torch.Tens
                                 activation=activation or gate_activation, act_constants=activation_constants)
                 return bool(activation)
         a = a.tensor()
-    # everything the kernels' acceptance looks at: sizes, row strides, element types, 16-byte alignment of the bases
+    # everything the kernels' acceptance looks at: sizes, row strides, element types, 16-byte alignment of the bases, devices
     key = (mode, a.shape, a.stride(), a.dtype, a.data_ptr() & 15, w.shape, w.stride(), w.dtype, w.data_ptr() & 15,
-           out.shape, out.stride(), out.dtype, out.data_ptr() & 15, a.device.index)
+           out.shape, out.stride(), out.dtype, out.data_ptr() & 15, a.get_device(), w.get_device(),
+           out.get_device())
     plain = not (activation or gate_activation or ops.profiling())
     if plain:
         call = _bound.get(key)
@@ -110,9 +116,9 @@ def linear(runtime, mode: int, a: torch.Tensor, w: torch.Tensor, out: torch.Tens
             call(a, w, out, alpha, error_flag)
             return False
     if a.dtype != torch.bfloat16:
-        if plain and a.dtype == torch.float32 == w.dtype and a.stride(1) == 1 == w.stride(1):
-            _bind(_SIMT, key, mode, a, w, out)
         ops.gemm_simt(mode, a, w, unactivated if activation else out, alpha, label=name, act=gate_activation)
+        if plain and a.dtype == torch.float32 == w.dtype:
+            _bind(_SIMT, key, mode, a, w, out)
         return False
     choice = _choices.get(key)
     if choice is None:
@@ -131,8 +137,6 @@ def linear(runtime, mode: int, a: torch.Tensor, w: torch.Tensor, out: torch.Tens
         # the two kernels for products in between have the SiLU gate alone: the cluster kernel's shapes go to the persistent
         # tcgen05 kernel, the one-CTA-per-16-rows kernel's to the product on the 32-bit pipes
         choice = _TC if choice == _CLUSTER else _SIMT
-    if plain and choice in _BOUND_KERNELS:
-        _bind(choice, key, mode, a, w, out)
     if choice == _TC:
         ops.gemm_tc(mode, a, w, out, alpha, error_flag, label=name, act=gate_activation)
     elif choice == _STREAM:
@@ -143,3 +147,5 @@ def linear(runtime, mode: int, a: torch.Tensor, w: torch.Tensor, out: torch.Tens
         ops.gemm_cluster(mode, a, w, out, alpha, error_flag, label=name)
     else:
         ops.gemm_simt(mode, a, w, out, alpha, label=name, act=gate_activation)
+    if plain and choice in _BOUND_KERNELS:
+        _bind(choice, key, mode, a, w, out)
