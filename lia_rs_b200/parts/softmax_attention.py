@@ -208,7 +208,7 @@ class SinkAttention(Mixer):
         linear(rt, STORE if store else ACCUM, o, self.w_o, residual, scale, error_flag=flag, name="o")
 
 
-_batched = {}            # sizes, strides and alignment of a product of all heads -> the kernel's call (0: another kernel serves them)
+_batched = {}            # sizes, strides, types, alignment and devices of a product of all heads -> the kernel's call (0: another kernel serves them)
 
 
 @register_mixer("latent_attention")
@@ -414,8 +414,10 @@ class LatentAttention(Mixer):
         """out[h] = a[h] @ w[h]^T for every head (3-D tensors, a head a plane), all heads in one launch: in
         bfloat16 on the tensor cores (csrc/gemm_mma_batched.cu) where that kernel takes the sizes (8 tokens of 16 heads:
         5 us against 29 on the 32-bit pipes), else, and on the 32-bit path, on the 32-bit pipes."""
-        key = (a.shape, a.stride(), a.data_ptr() & 15, w.shape, out.stride(), out.data_ptr() & 3, a.device.index)
         if a.dtype == torch.bfloat16 and a.shape[1] >= self.TENSOR_CORES_FROM and not ops.profiling():
+            # everything that the kernel's acceptance looks at and that the kept call takes for granted
+            key = (a.shape, a.stride(), a.data_ptr() & 15, w.shape, w.stride(), w.dtype, w.data_ptr() & 15, out.shape, out.stride(),
+                   out.dtype, out.data_ptr() & 3, a.get_device(), w.get_device(), out.get_device())
             call = _batched.get(key)
             if call is None:
                 if len(_batched) >= 256:

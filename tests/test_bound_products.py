@@ -71,3 +71,30 @@ def test_dropped_products_are_looked_up_anew(dtype, monkeypatch):
                 linear(None, ACCUM, a, w, out)
                 close(out / 2, a, w)
             assert len(module._bound) <= 3
+
+
+@pytest.mark.gpu
+def test_products_of_all_heads_are_only_for_tensors_like_their_own():
+    from lia_rs_b200.parts.softmax_attention import LatentAttention
+    part = LatentAttention.__new__(LatentAttention)
+    B, M, N, K = 3, 40, 64, 32
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a = torch.randn(B, M, K, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(B, N, K, device="cuda", generator=g).to(torch.bfloat16)
+    out = torch.zeros(B, M, N, device="cuda", dtype=torch.bfloat16)
+    exact = torch.einsum("bmk,bnk->bmn", a.double(), w.double())
+    shifted = torch.empty(B * N * K + 1, device="cuda", dtype=torch.bfloat16)[1:].view(B, N, K)      # no 16-byte loads
+    wide = torch.zeros(B, N, K + 8, device="cuda", dtype=torch.bfloat16)[:, :, :K]                   # rows that lie apart
+    rounded32 = torch.zeros(B, M, N, device="cuda")
+    for weight, result in ((w, out), (shifted, out), (wide, out), (w, rounded32), (w, out)):
+        weight.copy_(w)
+        for _ in range(2):
+            result.zero_()
+            part._head_products(None, a, weight, result, "k_up")
+            # the result's rounding to 16 bits, and the sum's
+            assert float((result.double() - exact).abs().max()) <= 2.0 ** -8 * float(exact.abs().max())
+    for _ in range(2):
+        for args in ((a, w.cpu(), out), (a, w.float(), out), (a, w, out[:, :-1])):
+            with pytest.raises(ops.KernelError):
+                part._head_products(None, *args, "k_up")
+    torch.cuda.synchronize()
