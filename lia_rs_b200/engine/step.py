@@ -147,21 +147,22 @@ class StepRuntime:
         view = self._views.get((name, numel, dtype))
         return view if view is not None else self._keep_view((name, numel, dtype), self._scratch(name, numel, dtype))
 
-    def shaped(self, name, shape, dtype):
-        """`scratch` of as many elements as `shape` has, in that shape."""
+    def shaped(self, name, shape, dtype, most=0):
+        """`scratch` of as many elements as `shape` has, in that shape.  With `most` (elements) the buffer grows by doublings, up to
+        that many: for sizes that creep up from step to step, since every growth makes the captured graphs stale."""
         view = self._views.get((name, dtype, shape))
         if view is None:
             numel = 1
             for size in shape:
                 numel *= size
-            view = self._scratch(name, numel, dtype).view(shape)
+            view = self._scratch(name, numel, dtype, min(1 << max(0, numel - 1).bit_length(), most)).view(shape)
             self._keep_view((name, dtype, shape), view)
         return view
 
-    def _scratch(self, name, numel, dtype):
+    def _scratch(self, name, numel, dtype, room=0):
         buf = self._buffers.get((name, dtype))
         if buf is None or buf.numel() < numel:
-            buf = torch.empty(max(numel, 1), dtype=dtype, device=self.device)
+            buf = torch.empty(max(numel, room, 1), dtype=dtype, device=self.device)
             self._buffers[(name, dtype)] = buf
             self._moved()
         return buf[:numel]

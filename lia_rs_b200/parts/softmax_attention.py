@@ -351,12 +351,14 @@ class LatentAttention(Mixer):
         H, d, dr, dv, rank = self.heads, self.d, self.dr, self.dv, self.rank
         n, size, flag = q.shape[0], kv.page_size, ctx.error_flag
         scratch = ctx.runtime.scratch
-        records = ctx.runtime.shaped("latent.records", (pages * size, rank + dr), torch.bfloat16)
+        # (as large as the keys that the portions see: by doublings, so that a long prompt filled in portions moves them a few times)
+        most = self.EXPAND_BYTES // 2
+        records = ctx.runtime.shaped("latent.records", (pages * size, rank + dr), torch.bfloat16, most)
         table = ctx.runtime.shaped("latent.table", kv.block_table.shape, torch.int32)
         ops.latent_gather(ctx.prefill_segments, ctx.n_prefill_segments, ctx.slots, kv.block_table, kv.k_pages, kv.v_pages,
                           records.view(pages, size, rank + dr), table, self.window, error_flag=flag)
         width = H * (d + dr + dv)
-        expanded = ctx.runtime.shaped("latent.expanded", (pages * size, width), torch.bfloat16)
+        expanded = ctx.runtime.shaped("latent.expanded", (pages * size, width), torch.bfloat16, most)
         linear(rt, STORE, records, self.w_expand, expanded, error_flag=flag, name="expand")
         paged = expanded.view(pages, size, width)
         keys, values = paged[:, :, :H * (d + dr)].unflatten(2, (H, d + dr)), paged[:, :, H * (d + dr):].unflatten(2, (H, dv))
