@@ -129,6 +129,7 @@ class StepRuntime:
         self._views.clear()
 
     def workspace(self, name, shape, dtype):
+        shape = tuple(shape)
         view = self._views.get((name, shape, dtype))
         return view if view is not None else self._keep_view((name, shape, dtype), self._workspace(name, shape, dtype))
 

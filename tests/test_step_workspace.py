@@ -41,3 +41,9 @@ def test_kept_views_are_bounded_and_dropping_them_moves_nothing(monkeypatch):
             view = runtime.scratch("a", numel, torch.float32)
             assert view.numel() == numel and view.data_ptr() == at and len(runtime._views) <= 5
     assert runtime.generation == generation
+
+
+def test_a_shape_may_be_a_list():
+    runtime = cpu_workspace()
+    view = runtime.workspace("a", [3, 8], torch.float32)
+    assert view.shape == (3, 8) and runtime.workspace("a", torch.Size([3, 8]), torch.float32) is view
