@@ -180,7 +180,9 @@ class PagedAttention:
         work_bytes, work_flops = self._work(ctx, q.element_size())
         if self.variant == "generic":
             rows = None
-            if ctx.n_prefill_segments and self._prefill_kernel()[1]:
+            # (the prompt kernel reads and writes 16 bytes at a time; the kernel for every size takes any base)
+            together = q.data_ptr() | kv.k_pages.data_ptr() | kv.v_pages.data_ptr() | out.data_ptr()
+            if ctx.n_prefill_segments and self._prefill_kernel()[1] and together % 16 == 0:
                 kernel, per_tile = self._prefill_kernel()
                 tiles = sum((count + per_tile - 1) // per_tile for _, _, count, _ in ctx.segments if count > 1)
                 kernel(q, kv.k_pages, kv.v_pages, ctx.prefill_segments, ctx.n_prefill_segments, tiles, ctx.slots, kv.block_table, out,

@@ -86,3 +86,29 @@ def test_a_missing_page_is_flagged_and_reads_nothing():
     ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
     ops.attention_prefill_f32(q, pages, pages, ints([0, 0, 8]), 1, 1, ints([0] * 8), table, out, 1, 1, 64, 1.0, error_flag=flag)
     assert int(flag) == 2
+
+
+def test_operands_without_16_byte_bases_go_to_the_kernel_for_every_size():
+    from types import SimpleNamespace
+    from lia_rs_b200.parts.paged_attention import PagedAttention
+    g = torch.Generator(device="cuda").manual_seed(5)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    nq, nkv, d, n = 4, 2, 32, 70
+    pages = torch.randn(2, 30, 5, nkv, d, device="cuda", generator=g)
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    segments = [(0, 0, n - 1, 0), (1, 20, 1, n - 1)]
+    ctx = SimpleNamespace(n_tokens=n, n_prefill_segments=1, segments=segments, prefill_segments=ints([0, 0, n - 1]), error_flag=flag,
+                          slots=ints([0] * (n - 1) + [1]), positions=ints(list(range(n - 1)) + [20]), decode_rows=ints([n - 1]))
+    table = torch.arange(30, dtype=torch.int32, device="cuda").view(2, 15)
+    attention = PagedAttention(torch.float32, nq, nkv, d, None, 0.3)
+    q = torch.randn(n, nq * d, device="cuda", generator=g)
+    want = torch.zeros_like(q)
+    aligned_kv = SimpleNamespace(k_pages=pages[0], v_pages=pages[1], block_table=table)
+    attention.forward(ctx, q, aligned_kv, want)
+    for shifted in ("q", "k", "v", "out"):
+        place = lambda name, t: unaligned(t) if name == shifted else t
+        kv = SimpleNamespace(k_pages=place("k", pages[0]), v_pages=place("v", pages[1]), block_table=table)
+        out = place("out", torch.zeros_like(q))
+        attention.forward(ctx, place("q", q), kv, out)
+        assert torch.equal(out, want), shifted
+    assert int(flag) == 0
