@@ -358,10 +358,12 @@ def embedding_sinusoidal(tokens, positions, table, freq, out, scale: float, copy
 def rmsnorm(x, weight, out, eps: float, out_scale: float = 1.0, rows_index=None):
     _cuda(weight, out, rows_index)
     rows, hidden = out.shape
-    if not x.is_cuda or x.dtype != torch.float32 or x.shape[1] != hidden or x.stride(1) != 1 or x.stride(0) < hidden:
+    whole = x.is_contiguous()              # (a dimension of size one may then have any stride)
+    if not x.is_cuda or x.dtype != torch.float32 or x.shape[1] != hidden or \
+            not (whole or (x.stride(1) == 1 and x.stride(0) >= hidden)):
         raise KernelError("rmsnorm takes 32-bit rows (of any stride) of the same width as its output")
     with _timed("rmsnorm"):
-        _check(lib().lia_rmsnorm(_p(x), x.stride(0), _p(rows_index), _p(weight), dtype_code(weight.dtype), _p(out),
+        _check(lib().lia_rmsnorm(_p(x), hidden if whole else x.stride(0), _p(rows_index), _p(weight), dtype_code(weight.dtype), _p(out),
                                  dtype_code(out.dtype), rows, hidden, eps, out_scale, _stream()), "rmsnorm")
 
 
@@ -769,10 +771,13 @@ def attention_prefill_tc(q, k_pages, v_pages, segments, n_segments, n_tiles, slo
     The pages' rows may lie apart (views [pages, page_size, nkv, d] of wider rows); `gate` (32-bit rows, an element each, or
     with `gate_head` a head each): the output is multiplied by its sigmoid before it is rounded."""
     _cuda(q, segments, slots, block_table, out, error_flag, partial, sinks)
+    strides = []
     for pages in (k_pages, v_pages):
-        if not pages.is_cuda or pages.stride(3) != 1 or pages.stride(2) != pages.shape[3] or \
-                pages.stride(0) != pages.stride(1) * pages.shape[1]:
+        whole = pages.is_contiguous()      # (a dimension of size one may then have any stride)
+        if not pages.is_cuda or not (whole or (pages.dim() == 4 and pages.stride(3) == 1 and pages.stride(2) == pages.shape[3] and
+                                              pages.stride(0) == pages.stride(1) * pages.shape[1])):
             raise KernelError("attention_prefill_tc: the pages' rows have one stride and whole heads side by side")
+        strides.append(0 if whole else pages.stride(1))
     if gate is not None and (gate.dtype != torch.float32 or gate.stride(1) != 1 or gate.shape[0] != q.shape[0]
                              or gate.shape[1] < (nq if gate_head else out.shape[1])):
         raise KernelError("attention_prefill_tc: a gate is 32-bit rows of an element (or a head) each")
@@ -790,7 +795,7 @@ def attention_prefill_tc(q, k_pages, v_pages, segments, n_segments, n_tiles, slo
                                               _p(slots), _p(block_table), block_table.shape[1], _p(out), nq, nkv, d, dv,
                                               k_pages.shape[1], int(window or 0), scale, k_pages.shape[0], splits,
                                               _p(partial) if splits > 1 else None, q.shape[0], 1 if sink else 0, _p(sinks),
-                                              float(softcap or 0.0), k_pages.stride(1), v_pages.stride(1), _p(gate),
+                                              float(softcap or 0.0), *strides, _p(gate),
                                               0 if gate is None else gate.stride(0), 1 if gate_head else 0, _p(error_flag),
                                               _stream()), "attention_prefill_tc")
 
@@ -1170,8 +1175,9 @@ def latent_prepare(q_rows, shared_rows, latent_norm, eps, freq, rot_dims, positi
     [tokens, heads dr] (or a view [tokens, heads, dr] with contiguous rows); see csrc/qk_prepare.cu.  `pairs`: the rotation pairs element 2i with 2i + 1 (else i with i + rot_dims / 2).
     `shared_rows` None: only the queries are prepared (the pages are filled by another layer)."""
     _cuda(latent_norm, freq, positions, slots, block_table, latent_pages, key_pages, error_flag)
-    if not (q_plain.is_cuda and q_rotated.is_cuda) or q_plain.stride(-1) != 1 or q_rotated.stride(-1) != 1:
-        raise KernelError("latent_prepare: the queries go to CUDA tensors with contiguous rows")
+    for t in (q_plain, q_rotated):
+        if not t.is_cuda or not (t.is_contiguous() or t.stride(-1) == 1):
+            raise KernelError("latent_prepare: the queries go to CUDA tensors with contiguous rows")
     _f32(q_rows, shared_rows, latent_norm, freq)
     n = q_rows.shape[0]
     if q_rows.stride(1) != 1 or q_rows.shape[1] < heads * (d + dr):
@@ -1182,17 +1188,23 @@ def latent_prepare(q_rows, shared_rows, latent_norm, eps, freq, rot_dims, positi
     if not (q_plain.dtype == q_rotated.dtype == latent_pages.dtype == key_pages.dtype) or q_plain.numel() != heads * n * d \
             or q_rotated.numel() != n * heads * dr or latent_pages.shape[-1] != rank or key_pages.shape[-1] != dr:
         raise KernelError("latent_prepare: outputs and pages must have one element type and the parts' sizes")
-    if tuple(q_plain.shape) != (heads, n, d):
-        q_plain = q_plain.view(heads, n, d)
-    if q_rotated.dim() != 2 and tuple(q_rotated.shape) != (n, heads, dr):
-        q_rotated = q_rotated.view(n, heads * dr)
-    rotated_head = q_rotated.stride(1) if q_rotated.dim() == 3 else dr
+    # contiguous queries of any shape are planes, and whole tokens, one behind the other
+    plain, rotated = (n * d, d), (dr, heads * dr)
+    if not q_plain.is_contiguous():
+        if tuple(q_plain.shape) != (heads, n, d):
+            raise KernelError("latent_prepare: queries that lie apart are [heads, tokens, d]")
+        plain = q_plain.stride()[:2]
+    if not q_rotated.is_contiguous():
+        if tuple(q_rotated.shape) not in ((n, heads, dr), (n, heads * dr)):
+            raise KernelError("latent_prepare: rotated parts that lie apart are [tokens, heads, dr] or [tokens, heads dr]")
+        rotated = (q_rotated.stride(1) if q_rotated.dim() == 3 else dr, q_rotated.stride(0))
     with _timed("latent_prepare"):
         _check(lib().lia_latent_prepare(_p(q_rows), q_rows.stride(0), _p(shared_rows),
                                         0 if shared_rows is None else shared_rows.stride(0),
                                         _p(latent_norm), float(eps), _p(freq), int(rot_dims), _p(positions), _p(slots),
-                                        _p(block_table), block_table.shape[1], _p(q_plain), q_plain.stride(0),
-                                        q_plain.stride(1), _p(q_rotated), rotated_head, q_rotated.stride(0), _p(latent_pages), _p(key_pages), dtype_code(q_plain.dtype), n, heads, d, dr, rank,
+                                        _p(block_table), block_table.shape[1], _p(q_plain), *plain,
+                                        _p(q_rotated), *rotated, _p(latent_pages), _p(key_pages), dtype_code(q_plain.dtype),
+                                        n, heads, d, dr, rank,
                                         latent_pages.shape[1], latent_pages.shape[0],
                                         1 if write_kv and shared_rows is not None else 0, 1 if pairs else 0,
                                         _p(error_flag), _stream()), "latent_prepare")
@@ -1352,7 +1364,8 @@ def latent_attention(q1, q2, latent_pages, part_pages, positions, slots, block_t
     if splits > 1 and (partial is None or partial.dtype != torch.float32 or partial.numel() < splits * heads * n * (rank + 2)):
         raise KernelError("latent_attention: the ranges need 32-bit scratch of splits * heads * tokens * (rank + 2) words")
     with _timed("latent_attention", label, work_bytes, work_flops):
-        _check(lib().lia_latent_attention(_p(q1), _p(q2), q2.stride(0), q2.stride(1) if q2.dim() == 3 else dr, _p(latent_pages),
+        q2_strides = (heads * dr, dr) if q2.is_contiguous() else (q2.stride(0), q2.stride(1) if q2.dim() == 3 else dr)
+        _check(lib().lia_latent_attention(_p(q1), _p(q2), *q2_strides, _p(latent_pages),
                                           _p(part_pages), _p(positions), _p(slots), _p(rows), _p(block_table), block_table.shape[1], _p(out), _p(partial) if splits > 1 else None,
                                           n, heads, rank, dr, latent_pages.shape[1], int(window or 0), scale,
                                           latent_pages.shape[0], splits, _p(error_flag), _stream()), "latent_attention")

@@ -90,3 +90,45 @@ def test_which_portions_are_expanded():
         seen = (last + 15) // 16 + 9
         assert seen <= pages < seen * 9 / 8 + 1 and tiles == 3
     assert plan([(0, 1 << 24, 64, 0)]) is None
+
+
+def test_contiguous_tensors_of_any_shape_and_stride():
+    """Contiguous outputs of latent_prepare in other shapes, and dimensions of size one with strides that mean nothing."""
+    from lia_rs_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(2)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    H, d, dr, rank, page = 3, 32, 16, 32, 4
+    odd = lambda t, dim: t.as_strided(t.shape, [0 if i == dim else s for i, s in enumerate(t.stride())], t.storage_offset())
+
+    def prepare(n, plain, rotated):
+        rows = torch.randn(n, H * (d + dr), device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+        pages = [torch.zeros(4, page, 1, size, device="cuda", dtype=torch.bfloat16) for size in (rank, dr)]
+        freq = torch.full((dr // 2,), 0.3, device="cuda")
+        ops.latent_prepare(rows, None, None, 1e-5, freq, dr, ints(list(range(n))), ints([0] * n), ints([[0, 1, 2, 3]]), plain, rotated,
+                           *pages, H, d, dr, rank)
+        return plain.reshape(-1), rotated.reshape(-1)
+
+    zeros = lambda *shape: torch.zeros(*shape, device="cuda", dtype=torch.bfloat16)
+    want = prepare(5, zeros(H, 5, d), zeros(5, H * dr))
+    assert float(want[0].float().abs().sum()) > 0 < float(want[1].float().abs().sum())
+    for plain, rotated in ((zeros(H * 5, d), zeros(5 * H, dr)), (zeros(H * 5 * d), zeros(5, H, dr)), (zeros(5, H * d), zeros(5 * H * dr))):
+        got = prepare(5, plain, rotated)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    want = prepare(1, zeros(H, 1, d), zeros(1, H * dr))
+    got = prepare(1, odd(zeros(H, 1, d), 1), odd(zeros(1, H * dr), 0))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+    x, weight = torch.randn(1, 64, device="cuda", generator=g), torch.ones(64, device="cuda")
+    out, other = (torch.zeros(1, 64, device="cuda") for _ in range(2))
+    ops.rmsnorm(x, weight, out, 1e-5)
+    ops.rmsnorm(odd(x, 0), weight, other, 1e-5)
+    assert torch.equal(out, other) and float(out.abs().sum()) > 0
+
+    q = torch.randn(9, 2 * 64, device="cuda", generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(1, 16, 1, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    results = []
+    for keys, values in ((k, v), (odd(k, 0), odd(v, 2)), (k[:, :, 0], v[:, :, 0])):
+        out = torch.zeros_like(q)
+        ops.attention_prefill_tc(q, keys, values, ints([0, 0, 9]), 1, 1, ints([0] * 9), ints([[0]]), out, 2, 1, 64, None, 0.1)
+        results.append(out)
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2]) and float(out.float().abs().sum()) > 0
