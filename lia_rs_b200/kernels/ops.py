@@ -778,7 +778,7 @@ def attention_prefill_tc(q, k_pages, v_pages, segments, n_segments, n_tiles, slo
                                               pages.stride(0) == pages.stride(1) * pages.shape[1])):
             raise KernelError("attention_prefill_tc: the pages' rows have one stride and whole heads side by side")
         strides.append(0 if whole else pages.stride(1))
-    if gate is not None and (gate.dtype != torch.float32 or gate.stride(1) != 1 or gate.shape[0] != q.shape[0]
+    if gate is not None and (not gate.is_cuda or gate.dtype != torch.float32 or gate.stride(1) != 1 or gate.shape[0] != q.shape[0]
                              or gate.shape[1] < (nq if gate_head else out.shape[1])):
         raise KernelError("attention_prefill_tc: a gate is 32-bit rows of an element (or a head) each")
     _check_sinks(sinks, nq)

@@ -132,3 +132,48 @@ def test_contiguous_tensors_of_any_shape_and_stride():
         ops.attention_prefill_tc(q, keys, values, ints([0, 0, 9]), 1, 1, ints([0] * 9), ints([[0]]), out, 2, 1, 64, None, 0.1)
         results.append(out)
     assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2]) and float(out.float().abs().sum()) > 0
+
+
+@pytest.mark.parametrize("d,dv", [(192, 128), (96, 64)])
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("form", ["none", "elements", "unaligned elements", "heads"])
+def test_gated_epilogue_against_64_bits(d, dv, splits, form):
+    """Whole keys and values of an expanded latent, the keys whole or in ranges, the output times the gate's sigmoid."""
+    from lia_rs_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(d + splits)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    H, page, portions = 3, 8, [(1, 300, 150), (0, 0, 2), (2, 120, 129)]              # slot, first position, tokens
+    n, blocks = sum(p[2] for p in portions), 60
+    q = torch.randn(n, H * d, device="cuda", generator=g).to(torch.bfloat16)
+    rows = torch.randn(3 * blocks, page, H * (d + dv), device="cuda", generator=g).to(torch.bfloat16)       # keys of all heads, then values
+    keys, values = rows[:, :, :H * d].unflatten(2, (H, d)), rows[:, :, H * d:].unflatten(2, (H, dv))
+    table = torch.randperm(3 * blocks, generator=torch.Generator().manual_seed(1)).view(3, blocks).to(torch.int32).cuda()
+    first = 3 if form == "unaligned elements" else 4                                 # the gate's columns behind others
+    gate = None if form == "none" else 4 * torch.randn(n, first + H * dv, device="cuda", generator=g)[:, first:]
+    if form == "heads":
+        gate = gate[:, :H]
+    segments, slots, want, at = [], [], [], 0
+    for slot, start, count in portions:
+        segments += [at, start, count]
+        slots += [slot] * count
+        mine = rows[table[slot].long()].reshape(blocks * page, -1)[:start + count].double()
+        k, v = mine[:, :H * d].view(-1, H, d), mine[:, H * d:].view(-1, H, dv)
+        scores = torch.einsum("thd,jhd->htj", q[at:at + count].double().view(count, H, d), k) * d ** -0.5
+        later = torch.arange(start + count, device="cuda") > torch.arange(start, start + count, device="cuda")[:, None]
+        want.append(torch.einsum("htj,jhv->thv", scores.masked_fill(later, float("-inf")).softmax(-1), v))
+        at += count
+    want = torch.cat(want)
+    if gate is not None:
+        want = want * torch.sigmoid(gate.double().reshape(n, H, -1))
+    out, flag = torch.zeros(n, H * dv, device="cuda", dtype=torch.bfloat16), ints([0])
+    tiles = sum((count + 127) // 128 for _, _, count in portions)
+    partial = torch.empty(ops.attention_prefill_tc_partial_floats(n, H, dv, splits), device="cuda") if splits > 1 else None
+    call = lambda gate: ops.attention_prefill_tc(q, keys, values, ints(segments), 3, tiles, ints(slots), table, out, H, H, d, None, d ** -0.5,
+                                                 flag, splits=splits, partial=partial, gate=gate, gate_head=form == "heads")
+    call(gate)
+    # probabilities and outputs are rounded to 16 bits, 2^-9 of themselves each, and the output is linear in both
+    off = (out.double().view(n, H, dv) - want).norm() / want.norm()
+    assert float(off) < 2 * 2.0 ** -9 and int(flag) == 0
+    if gate is not None:
+        with pytest.raises(ops.KernelError):
+            call(gate.cpu())
