@@ -370,7 +370,7 @@ class LatentAttention(Mixer):
             more = dict(splits=splits, partial=scratch("attn.prefill_partial", words, torch.float32))
         ops.attention_prefill_tc(q.view(n, H * (d + dr)), keys, values, ctx.prefill_segments, ctx.n_prefill_segments, tiles,
                                  ctx.slots, table, out, H, H, d + dr, self.window, self.scale, flag,
-                                 work_flops=self._work(ctx)[1], gate=gate, gate_head=self.gate_span > 1, **more)
+                                 work_flops=self._work(ctx, expanded=True)[1], gate=gate, gate_head=self.gate_span > 1, **more)
 
     def _attend_in_latent(self, ctx, q_plain, q_rotated, kv, out, rows=None):
         """out [tokens, heads, dv] (any strides) = attention in the latent's space of the tokens whose queries these are, q_plain
@@ -401,14 +401,16 @@ class LatentAttention(Mixer):
         ctas = max(1, n * ((self.heads + 15) // 16))
         return max(1, min(2 * ctx.runtime.sm_count // ctas, 16, longest // 128))
 
-    def _work(self, ctx):
-        """(cache bytes the single tokens read, flops of the prompt portions), for the profile only."""
+    def _work(self, ctx, expanded=False):
+        """(cache bytes the single tokens read, flops of the prompt portions in the latent's space, or over expanded keys and
+        values), for the profile only."""
         if ops._profiler is None:
             return 0, 0
         seen = lambda p: min(p + 1, self.window or p + 1)
         keys = sum(seen(start) for _, start, count, _ in ctx.segments if count == 1)
         pairs = sum(seen(start + i) for _, start, count, _ in ctx.segments if count > 1 for i in range(count))
-        return keys * (self.rank + self.dr) * 2, 2 * self.heads * (2 * self.rank + self.dr) * pairs
+        length = self.d + self.dr + self.dv if expanded else 2 * self.rank + self.dr
+        return keys * (self.rank + self.dr) * 2, 2 * self.heads * length * pairs
 
     TENSOR_CORES_FROM = 1             # tokens from which the heads' products go to the tensor cores (bfloat16)
 

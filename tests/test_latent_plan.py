@@ -25,3 +25,13 @@ def test_steps_of_one_graph_key_have_the_same_plans():
         ctx = step(start)
         plan = [part._expansion(ctx) for part in layers]
         assert plans.setdefault(DecoderModel.graph_key(model, ctx), plan) == plan, start
+
+
+def test_the_profile_counts_what_the_path_computes(monkeypatch):
+    from lia_rs_b200.kernels import ops
+    monkeypatch.setattr(ops, "_profiler", object())
+    part, ctx = layer(None), step(0, 100)
+    part.rank = 512
+    pairs = 100 * 101 // 2
+    assert part._work(ctx)[1] == 2 * 16 * (2 * 512 + 64) * pairs
+    assert part._work(ctx, expanded=True)[1] == 2 * 16 * (128 + 64 + 128) * pairs
