@@ -655,16 +655,49 @@ int launch_runs(const ScanArgs& p, const ConvTail& tail, cudaStream_t stream) {
 }
 }  // namespace
 
-// 1 if the kernel that walks whole portions takes these: at most 64 states, every row's pieces of four elements aligned.
-LIA_EXPORT int lia_selective_scan_walks_runs(const void* x, const void* dt_raw, const void* bc, long long ld_bc, int b_offset,
-                                             int c_offset, const void* z, long long ld_z, const void* out, int channels, int states) {
+namespace {
+bool run_sizes(const void* x, const void* dt_raw, const void* bc, long long ld_bc, int b_offset, int c_offset, const void* z, long long ld_z,
+               const void* out, int channels, int states) {
     return channels > 0 && states > 0 && states <= 64 && ((channels | states | b_offset | c_offset) & 3) == 0 && ((ld_bc | ld_z) & 3) == 0 &&
-                   (((uintptr_t)x | (uintptr_t)dt_raw | (uintptr_t)bc | (uintptr_t)z | (uintptr_t)out) & 15u) == 0
+           (((uintptr_t)x | (uintptr_t)dt_raw | (uintptr_t)bc | (uintptr_t)z | (uintptr_t)out) & 15u) == 0;
+}
+
+// Which way the portions go where all are open (`tokens` of them in `portions` portions; us on a B200, the run kernel beside the other).
+// Short ones, under eight tokens on average: the kernel for every size, which takes the step's single tokens in the same launch, where
+// there are any or where the run kernel's CTAs are more than one round (3 tokens and 32 single ones, 16 states: 7.1 beside 4.4 at 256
+// channels, 17.7 beside 13.9 at 4,096; 4 x 3 tokens of 4,096 channels 11.6 beside 5.6; 8 tokens and 32 single ones 7.3 beside 7.4).
+// Long ones of few channels: the run kernel's time is a chain, that of one token times the tokens, while the device is nearly idle, and
+// chunks side by side are faster.  Both times are estimated: a run's as its chain or the device's rate, whichever is longer; the chunks' as
+// their launches and their chains of 64 tokens, and a rate.  2,048 tokens of 256 channels and 4 / 16 / 32 / 64 states: 89 beside 77, 89
+// beside 107, 119 beside 126, 193 beside 132; 4,096 tokens of them 175 beside 101, 145, 153, 235; of 1,024 channels 175 beside 132 with 4
+// states and 175 beside 241 with 16; 2,048 tokens of 4,096 channels and 16 states 164 beside 406.  Over 756 sizes (128 to 4,096
+// channels, 4 to 64 states, 256 to 8,192 tokens in one to four portions) the choice costs more than 4% in seven, 18% at most.
+enum ScanRoute { SCAN_WHOLE, SCAN_RUNS, SCAN_CHUNKS };
+ScanRoute scan_route(int channels, int states, int tokens, int portions, int n_single) {
+    if (portions <= 0) return SCAN_WHOLE;
+    if (tokens < 8 * portions && (n_single > 0 || (long long)channels * portions > 8192)) return SCAN_WHOLE;
+    const int wide = states <= 16 ? 0 : states <= 32 ? 1 : 2;                     // states a lane: 1, 2 or 4
+    constexpr float CHAIN[3] = {0.0432f, 0.0578f, 0.0943f}, RATE[3] = {1.96e-5f, 2.75e-5f, 4.7e-5f};
+    const float n = (float)tokens, width = (float)channels;
+    const float runs = fmaxf(n / (float)portions * CHAIN[wide], n * width * RATE[wide]);
+    const float chunks = (states <= 4 ? 50.f : 75.f) + n * (0.005f + width * (9e-6f + 2e-6f * (float)states));
+    return runs > chunks ? SCAN_CHUNKS : SCAN_RUNS;
+}
+}  // namespace
+
+// 1 if the kernel that walks whole portions serves these (at most 64 states, every row's pieces of four elements aligned, and faster
+// than the others for a step of `n_tokens` rows, `n_single` of them single tokens, in `n_segments` portions).
+LIA_EXPORT int lia_selective_scan_walks_runs(const void* x, const void* dt_raw, const void* bc, long long ld_bc, int b_offset,
+                                             int c_offset, const void* z, long long ld_z, const void* out, int channels, int states,
+                                             int n_tokens, int n_segments, int n_single) {
+    return run_sizes(x, dt_raw, bc, ld_bc, b_offset, c_offset, z, ld_z, out, channels, states) &&
+                   scan_route(channels, states, n_tokens - n_single, n_segments, n_single) == SCAN_RUNS
                ? 1 : 0;
 }
 
 // `conv_state` (or null; slot s at conv_state + s conv_stride: [taps - 1, channels]): the portions leave their last taps - 1 inputs
-// there, read from conv_x [n, conv_ld]; only where lia_selective_scan_walks_runs says yes and the step has no single tokens.
+// there, read from conv_x [n, conv_ld]; only where lia_selective_scan_walks_runs says yes and the step has no single tokens.  Without
+// chunk_scratch no portion is cut into chunks.
 LIA_EXPORT int lia_selective_scan(const float* x, const float* dt_raw, const float* dt_bias, const float* A,
                                   const float* bc, long long ld_bc, int b_offset, int c_offset, const float* D,
                                   const float* z, long long ld_z, float* state, long long state_stride,
@@ -688,7 +721,10 @@ LIA_EXPORT int lia_selective_scan(const float* x, const float* dt_raw, const flo
     p.out = out; p.channels = channels; p.states = states;
     p.chunk_state = chunk_scratch;
     p.chunk_dt = chunk_scratch ? chunk_scratch + ((long long)n_tokens / CHUNK + n_segments) * channels * states : nullptr;
-    if (n_segments > 0 && lia_selective_scan_walks_runs(x, dt_raw, bc, ld_bc, b_offset, c_offset, z, ld_z, out, channels, states)) {
+    const bool open = n_segments > 0 && run_sizes(x, dt_raw, bc, ld_bc, b_offset, c_offset, z, ld_z, out, channels, states);
+    const ScanRoute route = scan_route(channels, states, n_tokens - n_single, n_segments, n_single);
+    if (open && route == SCAN_WHOLE) chunked = false;
+    if (open && (conv_state || route == SCAN_RUNS || (route == SCAN_CHUNKS && !chunked))) {
         const int rc = out_dtype == LIA_F32 ? launch_runs<float>(p, {conv_state, conv_stride, conv_x, conv_ld, taps}, stream)
                      : out_dtype == LIA_BF16 ? launch_runs<__nv_bfloat16>(p, {conv_state, conv_stride, conv_x, conv_ld, taps}, stream)
                                              : LIA_ERR_DTYPE;

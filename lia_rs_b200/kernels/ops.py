@@ -141,7 +141,7 @@ class _Signatures:
                           c_void_p, c_int, c_int, c_int, c_int, c_void_p, ctypes.c_longlong, c_void_p, ctypes.c_longlong, c_void_p,
                           ctypes.c_longlong, c_int, c_void_p]
     lia_selective_scan_walks_runs = [c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_void_p, ctypes.c_longlong, c_void_p,
-                                     c_int, c_int]
+                                     c_int, c_int, c_int, c_int, c_int]
     lia_selective_scan_chunk_floats = [c_int, c_int, c_int, c_int]
     lia_gemm_simt_batched = [c_int, c_void_p, c_int, c_int, ctypes.c_longlong, c_void_p, c_int, c_int, ctypes.c_longlong,
                              c_void_p, c_int, c_int, ctypes.c_longlong, c_int, c_int, c_int, c_int, c_float, c_void_p]
@@ -1252,11 +1252,13 @@ def selective_scan_chunk_floats(n_tokens: int, n_segments: int, channels: int, s
     return int(fn(int(n_tokens), int(n_segments), int(channels), int(states)))
 
 
-def selective_scan_walks_runs(x, dt_raw, bc, b_offset, c_offset, z, out, states: int) -> bool:
-    """Whether a step's portions are walked whole by the kernel that keeps a channel in eight lanes (it needs no scratch and can
-    leave the convolution's state): at most 64 states, rows whose pieces of four elements are aligned."""
+def selective_scan_walks_runs(x, dt_raw, bc, b_offset, c_offset, z, out, states: int, n_segments: int = 1, n_single: int = 0) -> bool:
+    """Whether a step's portions are walked whole by the kernel that keeps a channel in sixteen lanes (it needs no scratch and can
+    leave the convolution's state): at most 64 states, rows whose pieces of four elements are aligned, and sizes for which it is
+    the fastest (csrc/selective_scan.cu)."""
     return bool(lib().lia_selective_scan_walks_runs(_p(x), _p(dt_raw), _p(bc), bc.stride(0), int(b_offset), int(c_offset), _p(z),
-                                                    z.stride(0), _p(out), x.shape[1], int(states)))
+                                                    z.stride(0), _p(out), x.shape[1], int(states), x.shape[0], int(n_segments),
+                                                    int(n_single)))
 
 
 def selective_scan(x, dt_raw, dt_bias, A, bc, b_offset, c_offset, D, z, state, segments, n_segments, single_rows, slots, out,

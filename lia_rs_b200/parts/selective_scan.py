@@ -105,7 +105,8 @@ class SelectiveScan(Mixer):
         y = ctx.buffer("scan.y", (n, inner), dtype)
         chunk_scratch, more = None, {}
         bc = (projected, rank, rank + states)
-        whole = ctx.n_prefill_segments and ops.selective_scan_walks_runs(u, dt_raw, *bc, uz[:, inner:], y, states)
+        whole = ctx.n_prefill_segments and ops.selective_scan_walks_runs(u, dt_raw, *bc, uz[:, inner:], y, states,
+                                                                            ctx.n_prefill_segments, ctx.n_single)
         if taps > 1 and not single:
             if whole and not ctx.n_single:           # the scan's kernel leaves the convolution's state too
                 more = dict(conv_state=conv_state, conv_x=uz)
