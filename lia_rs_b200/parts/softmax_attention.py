@@ -224,7 +224,7 @@ class LatentAttention(Mixer):
         # a model keeps each distinct answer once)
         if not ctx.n_prefill_segments or not self.per_tile:
             return ()
-        return ((self.window, self.per_tile, self.heads * (self.d + self.dr + self.dv), self._expansion(ctx)),)
+        return ((self.window, self.per_tile, self.heads, self.d, self.dr, self.dv, self.rank, self._expansion(ctx)),)
 
     @staticmethod
     def _names(params, prefix):
@@ -316,7 +316,8 @@ class LatentAttention(Mixer):
             w_keys[:, d:, rank:] = torch.eye(self.dr, dtype=w_keys.dtype, device=w_keys.device)
             self.w_expand[H * (d + self.dr):, :rank] = self.w_v_up.view(H * dv, rank)
 
-    EXPAND_FROM = 16                  # tokens a portion, on average, from which the records are expanded
+    EXPAND_FROM = 16                  # tokens a portion, on average, from which the records are expanded at all
+    EXPAND_FREELY = 2048              # keys that the portions see up to which that is enough (see _expansion)
     EXPAND_BYTES = 1 << 30            # most memory that the expanded keys and values of one step may take
 
     def _expansion(self, ctx):
@@ -327,7 +328,13 @@ class LatentAttention(Mixer):
         In the latent's space a pair of query and key costs 2 rank + dr multiply-adds a head on `mma.sync`, expanded d + dr + dv
         on tcgen05 (1,088 against 320 at 2B-widths) beside the expansion's d + dr + dv products of length rank a key and head,
         whatever the number of queries: 2,048 tokens over themselves took 796 us beside 2 x 127 us for the queries' and the
-        outputs' way into that space and back."""
+        outputs' way into that space and back.
+
+        Few tokens over many keys do not pay for the expansion: they must be as many as its multiply-adds a key are more than an
+        eighth of those of a pair in the latent's space (21 at 2B widths, 10 at 0.5B; 16 at least).  A layer in us, in the latent's
+        space / expanded, 2B widths, gated: 16 tokens behind 0 / 512 / 2,048 / 8,192 / 32,768 keys 46/44, 52/45, 61/60, 103/121,
+        268/347; 24 tokens 49/42, 57/48, 68/60, 122/121, 338/347; 32 tokens 45/42, 56/48, 73/61, 146/122, 432/346; four portions of 16,
+        24, 32 tokens behind 8,192 keys 271/353, 346/365, 495/370.  0.5B: 16 tokens behind 2,048 and 8,192 keys 44/38, 78/62."""
         if not ctx.n_prefill_segments or not self.per_tile:
             return None
         size = ctx.runtime.cache.page_size
@@ -340,7 +347,10 @@ class LatentAttention(Mixer):
                 tokens += count
         step = 1 << max(0, pages.bit_length() - 4)
         pages = (pages + step - 1) // step * step
-        if tokens < self.EXPAND_FROM * ctx.n_prefill_segments or \
+        need = self.EXPAND_FROM
+        if pages * size > self.EXPAND_FREELY:
+            need = max(need, (self.d + self.dr + self.dv) * (self.rank + self.dr) // (8 * (2 * self.rank + self.dr)))
+        if tokens < need * ctx.n_prefill_segments or \
                 pages * size * self.heads * (self.d + self.dr + self.dv) * 2 > self.EXPAND_BYTES:
             return None
         return pages, tiles

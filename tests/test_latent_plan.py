@@ -7,7 +7,7 @@ from lia_rs_b200.parts.softmax_attention import LatentAttention
 
 def layer(window):
     part = LatentAttention.__new__(LatentAttention)
-    part.window, part.per_tile, part.heads, part.d, part.dr, part.dv = window, 128, 16, 128, 64, 128
+    part.window, part.per_tile, part.heads, part.d, part.dr, part.dv, part.rank = window, 128, 16, 128, 64, 128, 512
     return part
 
 
@@ -27,11 +27,20 @@ def test_steps_of_one_graph_key_have_the_same_plans():
         assert plans.setdefault(DecoderModel.graph_key(model, ctx), plan) == plan, start
 
 
+def test_few_tokens_over_many_keys_stay_in_the_latents_space():
+    wide, narrow = layer(None), layer(None)
+    narrow.d, narrow.dr, narrow.dv, narrow.rank = 64, 32, 64, 256
+    plans = lambda part, start, count: part._expansion(step(start, count)) is not None
+    for part in (wide, narrow):
+        assert not plans(part, 0, 15) and plans(part, 0, 16) and plans(part, 2000, 16) and plans(part, 30000, 32)
+    assert not plans(wide, 8192, 20) and plans(wide, 8192, 21) and plans(narrow, 8192, 16)
+    assert plans(layer(1024), 8192, 16)                                 # a window: the portion sees 1,039 keys
+
+
 def test_the_profile_counts_what_the_path_computes(monkeypatch):
     from lia_rs_b200.kernels import ops
     monkeypatch.setattr(ops, "_profiler", object())
     part, ctx = layer(None), step(0, 100)
-    part.rank = 512
     pairs = 100 * 101 // 2
     assert part._work(ctx)[1] == 2 * 16 * (2 * 512 + 64) * pairs
     assert part._work(ctx, expanded=True)[1] == 2 * 16 * (128 + 64 + 128) * pairs
