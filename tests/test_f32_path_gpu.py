@@ -86,6 +86,12 @@ def test_a_missing_page_is_flagged_and_reads_nothing():
     ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
     ops.attention_prefill_f32(q, pages, pages, ints([0, 0, 8]), 1, 1, ints([0] * 8), table, out, 1, 1, 64, 1.0, error_flag=flag)
     assert int(flag) == 2
+    # token t attends over keys 0 .. min(t, 3) of page 2 alone: sums of 64 products and of four, their exponentials' scores off by as much
+    k = pages[2, :, 0].double()
+    for t in range(8):
+        seen = k[:min(t, 3) + 1]
+        want = torch.softmax(seen @ q[t].double(), dim=0) @ seen
+        assert float((out[t].double() - want).abs().max()) < 64 * 2.0 ** -23 * float((k.abs() @ q[t].double().abs()).max())
 
 
 def test_operands_without_16_byte_bases_go_to_the_kernel_for_every_size():

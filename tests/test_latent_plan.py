@@ -37,6 +37,13 @@ def test_few_tokens_over_many_keys_stay_in_the_latents_space():
     assert plans(layer(1024), 8192, 16)                                 # a window: the portion sees 1,039 keys
 
 
+def test_the_expansion_keeps_to_its_memory():
+    """Pages of 16 keys, 16 heads of 128 + 64 + 128 elements of two bytes: 6,553 pages fit into 1 GB, after rounding 6,144."""
+    part = layer(None)
+    assert part._expansion(step(6144 * 16 - 2048))[0] == 6144
+    assert part._expansion(step(6144 * 16 - 2047)) is None
+
+
 def test_the_profile_counts_what_the_path_computes(monkeypatch):
     from lia_rs_b200.kernels import ops
     monkeypatch.setattr(ops, "_profiler", object())

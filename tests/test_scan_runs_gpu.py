@@ -1,4 +1,4 @@
-"""The kernel that walks whole portions of a selective scan, eight lanes a channel, against the plain recurrence in 64-bit and the
+"""The kernel that walks whole portions of a selective scan, sixteen lanes a channel, against the plain recurrence in 64-bit and the
 kernel for every size; and the convolution that gives a thread eight rows, against the one that gives it one."""
 import pytest
 import torch
