@@ -761,6 +761,20 @@ def attention_prefill_tc_tokens_per_tile(group: int, d: int, dv: int = None) -> 
     return int(lib().lia_attention_prefill_tc_tokens_per_tile(group, d, d if dv is None else dv))
 
 
+def _row_stride(pages):
+    """Elements from one row of the pages [pages, page_size, nkv, d] to the next (0: they lie side by side), or None where they have
+    no one stride.  A dimension of size one may have any stride."""
+    if not pages.is_cuda:
+        return None
+    if pages.is_contiguous():
+        return 0
+    if pages.dim() != 4 or pages.stride(3) != 1 or (pages.shape[2] > 1 and pages.stride(2) != pages.shape[3]):
+        return None
+    count, size = pages.shape[:2]
+    row = pages.stride(1) if size > 1 else pages.stride(0)
+    return row if count == 1 or pages.stride(0) == row * size else None
+
+
 def attention_prefill_tc(q, k_pages, v_pages, segments, n_segments, n_tiles, slots, block_table, out, nq, nkv, d,
                          window, scale, error_flag=None, label=None, work_flops=0, splits=1, partial=None, sink=False,
                          softcap=None, sinks=None, gate=None, gate_head=False):
@@ -771,13 +785,9 @@ def attention_prefill_tc(q, k_pages, v_pages, segments, n_segments, n_tiles, slo
     The pages' rows may lie apart (views [pages, page_size, nkv, d] of wider rows); `gate` (32-bit rows, an element each, or
     with `gate_head` a head each): the output is multiplied by its sigmoid before it is rounded."""
     _cuda(q, segments, slots, block_table, out, error_flag, partial, sinks)
-    strides = []
-    for pages in (k_pages, v_pages):
-        whole = pages.is_contiguous()      # (a dimension of size one may then have any stride)
-        if not pages.is_cuda or not (whole or (pages.dim() == 4 and pages.stride(3) == 1 and pages.stride(2) == pages.shape[3] and
-                                              pages.stride(0) == pages.stride(1) * pages.shape[1])):
-            raise KernelError("attention_prefill_tc: the pages' rows have one stride and whole heads side by side")
-        strides.append(0 if whole else pages.stride(1))
+    strides = [_row_stride(pages) for pages in (k_pages, v_pages)]
+    if None in strides:
+        raise KernelError("attention_prefill_tc: the pages' rows have one stride and whole heads side by side")
     if gate is not None and (not gate.is_cuda or gate.dtype != torch.float32 or gate.stride(1) != 1 or gate.shape[0] != q.shape[0]
                              or gate.shape[1] < (nq if gate_head else out.shape[1])):
         raise KernelError("attention_prefill_tc: a gate is 32-bit rows of an element (or a head) each")

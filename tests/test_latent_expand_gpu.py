@@ -66,7 +66,8 @@ def test_expanded_portions_against_plain_functions(d, dr, dv, rank, page, form):
         assert float((out - want).norm(dim=-1).max() / want.norm(dim=-1).max()) < 2 * REL
 
 
-def test_a_prompt_that_outgrows_the_expansion(monkeypatch):
+@pytest.mark.parametrize("page,pages", [(16, [7, 12]), (1, [104, 192])])
+def test_a_prompt_that_outgrows_the_expansion(page, pages, monkeypatch):
     """Portions of one prompt on both sides of the expansion's memory limit: the same attention."""
     from lia_rs_b200.parts.softmax_attention import LatentAttention
     g = torch.Generator().manual_seed(9)
@@ -74,14 +75,14 @@ def test_a_prompt_that_outgrows_the_expansion(monkeypatch):
     w = tensors(96, m, "gated", g)
     params = dict(hidden=96, heads=3, head_dim=64, rot_dim=32, v_head_dim=64, kv_rank=256, scale=m["scale"], norm_eps=1e-5,
                   rot=m["rot"], q_rank=None, gate="sigmoid", rot_pairs=True)
-    runner = PartRunner("latent_attention", params, w, "bfloat16", page_size=16, slots=1, tokens=1024)
-    monkeypatch.setattr(LatentAttention, "EXPAND_BYTES", 12 * 16 * 3 * 160 * 2)                  # twelve pages
+    runner = PartRunner("latent_attention", params, w, "bfloat16", page_size=page, slots=page, tokens=1024)
+    monkeypatch.setattr(LatentAttention, "EXPAND_BYTES", 192 * 3 * 160 * 2)                      # 192 keys
     ways, rows, got = [], {"a": torch.randn(500, 96, generator=g).to(torch.bfloat16).float()}, []
     whole = LatentAttention._expansion
     monkeypatch.setattr(LatentAttention, "_expansion", lambda part, ctx: ways.append(whole(part, ctx)) or ways[-1])
     for count in (100, 92, 60, 248):
         got.append(runner.step([("a", count)], rows)["a"])
-    assert [way and way[0] for way in ways] == [7, 12, None, None]
+    assert [way and way[0] for way in ways] == pages + [None, None]
     h, positions = rows["a"].to(F64), torch.arange(500)
     want = pz.latent_attention(h, positions, w, m, pz.latent_cache(h, positions, w["dkv"], w["dkv.norm"], m, 1e-5))
     off = torch.cat(got) - want
