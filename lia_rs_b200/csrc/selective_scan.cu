@@ -20,7 +20,10 @@
 
 namespace {
 constexpr int MAX_TAPS = 8;
-constexpr int CONV_TILED_FROM = 64;    // rows of a step from which eight of them share a thread's window
+// rows x channels of a step from which eight rows share a thread's window: below, eight times fewer threads are too few (us, a row a
+// thread / eight, four taps: 100 x 2,048 4.4/5.6, 64 x 4,096 6.0/5.6, 100 x 4,096 6.2/5.7, 1,024 x 256 5.7/5.6, 300 x 2,048 8.9/6.1; two
+// taps: 64 x 4,096 4.3/4.9, 100 x 4,096 4.7/4.9, 1,024 x 256 4.2/4.9, 2,048 x 256 5.5/5.0, 300 x 2,048 7.1/5.0)
+constexpr long long CONV_TILED_FROM = 3 << 17;
 
 // how many of the rows just before row t continue the same run (at most `most`)
 __device__ __forceinline__ int run_before(const int* __restrict__ positions, const int* __restrict__ slots, int t,
@@ -558,7 +561,7 @@ LIA_EXPORT int lia_causal_conv(const float* x, long long ld, const float* taps_w
     if (channels <= 0 || taps < 1 || taps > MAX_TAPS || ld < channels || (taps > 1 && !state) || act < 0 || act > 1)
         return LIA_ERR_SIZE;
     const size_t copy_size = copy_dtype == LIA_BF16 ? 2 : 4;
-    if (!update_single && n_tokens >= CONV_TILED_FROM && taps >= 2 && taps <= 4 && channels % 4 == 0 && ld % 4 == 0 &&
+    if (!update_single && (long long)n_tokens * channels >= CONV_TILED_FROM && taps >= 2 && taps <= 4 && channels % 4 == 0 && ld % 4 == 0 &&
         (((uintptr_t)x | (uintptr_t)out) & 15u) == 0 && ((uintptr_t)out_copy & (4 * copy_size - 1)) == 0 &&
         (n_tokens + CONV_ROWS - 1) / CONV_ROWS <= 65535) {
         const dim3 tiles((channels / 4 + CONV_THREADS - 1) / CONV_THREADS, (n_tokens + CONV_ROWS - 1) / CONV_ROWS);

@@ -72,7 +72,7 @@ def test_runs_against_the_plain_recurrence(channels, states, lengths):
 
 
 @pytest.mark.parametrize("taps", [2, 3, 4, 6])
-@pytest.mark.parametrize("channels", [4, 36, 516])
+@pytest.mark.parametrize("channels", [4, 36, 516, 3324])
 def test_convolution_of_eight_rows_a_thread(taps, channels):
     from lia_rs_b200.kernels import ops
     g = torch.Generator(device="cuda").manual_seed(taps * 1000 + channels)
