@@ -264,7 +264,9 @@ int sm_count_of_device() {
 // less from shared memory per multiply-add: 450 x 1,280: 65.8 in 8 x 16, 41.1 in 16 x 32, 53 in 32 x 32; 600 x 1,024: 69.8, 59.5 and 53.4
 // (the kernel above: 107); 600 x 32,000: 1,129 in 16 x 32, 1,058 in 32 x 32, 983 in 32 x 64 (40 TFLOP/s, 54% of the pipes).  So by how many
 // tiles of a shape an SM would get; at most 16 rows keep 16 x 32 however many columns (8 x 32,000: 46.9 against 69.5 in 32 x 64).  The
-// gated form, 4,096 pairs: 264 at 600 rows in 64 x 32 pairs (32 x 32: 273; the kernel above: 511), 41.1 at 48 rows in 16 x 32 pairs (47.3).
+// gated form, 4,096 pairs: 264 at 600 rows in 64 x 32 pairs (32 x 32: 273; the kernel above: 511), 41.1 at 48 rows in 16 x 32 pairs (47.3);
+// 100 rows 84 in 32 x 32 pairs, 91 in 16 x 32, 98 in 64 x 32 (two CTAs on some SMs, none on others; the kernel above: 85), 8,192 pairs 121,
+// 162 and the kernel above 134.
 template <int MODE>
 int launch_tiled(const float* A, int lda, const float* W, int ldw, float* out, int ldo, int M, int N, int K, float alpha,
                  cudaStream_t stream, int batch, long long a_batch, long long w_batch, long long out_batch, int act) {
@@ -272,6 +274,7 @@ int launch_tiled(const float* A, int lda, const float* W, int ldw, float* out, i
     return launch_tile<BM, BN, TM, TN, MODE>(A, lda, W, ldw, out, ldo, M, N, K, alpha, stream, batch, a_batch, w_batch, out_batch, act)
     if constexpr (MODE == GEMM_SWIGLU) {
         if (M <= 64) LIA_TILE(16, 32, 2, 4);
+        if (M <= 128) LIA_TILE(32, 32, 4, 4);
         LIA_TILE(64, 32, 4, 4);
     } else {
         const long long sms = sm_count_of_device();
