@@ -46,7 +46,7 @@ class PartRunner:
         cache_request, state_request = cls.cache_request(params), cls.state_request(params)
         self.has_cache, self.has_state = cache_request is not None, state_request is not None
         self.cache = CacheManager({0: cache_request} if cache_request else {}, {0: state_request} if state_request else {}, tokens,
-                                  slots, page_size, tokens, self.dtype, DEV)
+                                  page_size, slots, tokens, self.dtype, DEV)
         self.runtime = StepRuntime(self.cache, 1000, tokens, DEV)
         self.part = cls(params, {"L." + k: v.to(DEV) for k, v in weights.items()}, "L.", Runtime(DEV, self.dtype))
         self.live = {}
