@@ -430,7 +430,14 @@ LIA_EXPORT int lia_moe_route(const void* x, int dtype, long long ld, const float
     const int resident = experts + extra <= 16 ? 2 * 148 : 148;
     int tokens = n <= resident ? 1 : n <= 2 * resident ? 2 : 4;
     while (tokens > 1 && tokens * one > 200 * 1024) tokens /= 2;
-    const int threads = experts + extra <= 8 ? 256 : experts + extra <= 16 ? 512 : 1024;
+    // Many more tokens than are resident, of rows that are not long: CTAs of 256 threads, of which an SM holds more.  us, with as many
+    // threads as for few tokens / 256: hidden 1,024, 2,048 tokens, 9, 17, 65 and 129 outputs 12.3/10.0, 26/14, 55/35, 84/60; hidden 2,048
+    // 16.8/15.3, 34/22, 84/57, 134/104; hidden 1,024, 600 tokens, 17 and 65 outputs 13.7/11.6, 27.7/25.3; 1,024 tokens 14.1/12.9; not so:
+    // 65 and 129 outputs, 1,024 tokens 28/30, 43/52; hidden 2,048, 17 outputs, 600 tokens 17.9/17.3.
+    const int outputs = experts + extra;
+    const bool many = tokens == 4 && hidden <= 2048 &&
+                      (n > 8 * 148 || (n >= 4 * 148 && hidden <= 1024 && outputs > 16 && (outputs <= 32 || (outputs <= 160 && n <= 5 * 148))));
+    const int threads = many || outputs <= 8 ? 256 : outputs <= 16 ? 512 : 1024;
 #define LIA_ROUTE(T, TOKENS)                                                                                             \
     return lia_launch(moe_route_kernel<T, TOKENS>, dim3((n + TOKENS - 1) / TOKENS), dim3(threads), TOKENS * one, stream,     \
                       (const T*)x, ld, router, n, hidden, experts, top, scale, extra, correction, groups, keep,          \
