@@ -378,7 +378,8 @@ Plan make_plan(int M, int N, int K, int sm_count) {
 // many full barriers the blocks take in turn.
 // The ring is used again: half of it lands while the other half is multiplied.  As many stages as there is room for, an odd number
 // too (200 KB and an even number: gate/up of a 2B-class layer at 17 / 64 / 128 tokens 16.5 / 18.1 / 20.6 us, down 10.5 / 11.7 /
-// 14.8; so 13.7 / 16.3 / 19.5 and 9.8 / 11.2 / 13.7).  Single stages as they fall free give up what consecutive boxes of the same
+// 14.8; so 13.5 / 15.1 / 18.2 and 9.3 / 10.6 / 12.7, with 13.7 / 16.3 / 19.5 and 9.8 / 11.2 / 13.7 before barriers and stages were
+// counted along).  Beside the latter, single stages as they fall free give up what consecutive boxes of the same
 // rows of W save: 17.1 / 19.2 / 22.1 and 11.7 / 13.7 / 16.4.
 // An odd ring hands a stage from one of two issuers to the other, and a wait by parity cannot tell the fill that is wanted from the
 // one two fills before: an issuer that skips a fill could pass early and multiply what has not landed.  Then twice as many barriers
