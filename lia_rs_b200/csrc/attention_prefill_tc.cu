@@ -98,7 +98,8 @@ attention_prefill_tc_kernel(Params p) {
     // tensor memory: two score buffers of 128 columns, the output's head_dim columns (128 kept), and two buffers of
     // probabilities of 64 columns (128 keys as bf16 pairs)
     constexpr int TMEM_COLS = 512;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const bool leader = elect_one();
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t q_s = smem_base, kv_s = q_s + Q_BYTES;   // kv_s: [stage][K, V]
     uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -269,7 +270,7 @@ attention_prefill_tc_kernel(Params p) {
             mbar_arrive(smem_u32(&v_full[st]));
         }
         if (!ok && p.error_flag) atomicExch(p.error_flag, 3);
-    } else if (warp == SOFTMAX_WARPS && lane == 0 && n_tiles > 0) {
+    } else if (warp == SOFTMAX_WARPS && leader && n_tiles > 0) {
         // ---- MMA issuer ----
         const uint32_t idesc_s = instr_desc(ROWS, KT), idesc_o = instr_desc_b_mn(ROWS, DV);
         bool ok = mbar_wait(smem_u32(&q_full), 0u);

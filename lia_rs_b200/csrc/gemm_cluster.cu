@@ -86,7 +86,8 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     constexpr int A_TILES = (MODE == GEMM_SWIGLU) ? 2 : 1;
     constexpr int ACC_W = TILE_F * A_TILES;                 // floats per token in the exchange buffer
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const bool leader = elect_one();
     const uint32_t a_bytes = TILE_F * BLOCK_K * 2, b_bytes = (uint32_t)s.n_tile * BLOCK_K * 2;
     const uint32_t stage_bytes = A_TILES * a_bytes + b_bytes;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -120,7 +121,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const uint32_t tmem_base = tmem_base_slot;
     pdl_launch_dependents();
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && leader) {
         // ---- TMA producer: W at once, X when the kernel ahead has finished ----
         // (a batch's boxes are issued tile by tile of W, so that consecutive requests read consecutive 128-byte pieces of the
         // same rows)
@@ -165,10 +166,9 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             for (int i = max(0, issued - s.stages); i < issued; ++i)      // copies in flight must land before the CTA may end
                 mbar_wait(smem_u32(&full_bar[i % s.bars]), (uint32_t)(i / s.bars) & 1u);
         }
-    } else if ((warp == 1 || warp == 2) && lane == 0) {
-        // ---- MMA issuers.  Issuing one tcgen05.mma costs a thread some 130 cycles, four times what a tile this
-        //      narrow computes for, so two threads issue: they take the K blocks in turn, each into accumulators of
-        //      its own (an MMA that adds to the accumulator of the one before it would wait for it, too).  The
+    } else if ((warp == 1 || warp == 2) && leader) {
+        // ---- MMA issuers.  Two threads issue: they take the K blocks in turn, each into accumulators of
+        //      its own (an MMA that adds to the accumulator of the one before it would wait for it).  The
         //      epilogue adds the accumulators up in a fixed order.  An issuer does not wait for the blocks it skips, so
         //      every full barrier has one issuer that waits for all its fills in turn (their number is even) ----
         const int issuers = s.chains >= 2 ? 2 : 1;

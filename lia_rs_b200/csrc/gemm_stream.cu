@@ -102,6 +102,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         }
     }
 }
+// One thread of a warp whose threads have all come here, and known to the compiler as one: behind `lane == 0` every bulk copy is gone about
+// thread by thread.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\t.reg .b32 R;\n\telect.sync R|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // `bytes` (a multiple of 16) from global `src` to shared `dst`, both 16-byte aligned.
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -261,7 +268,8 @@ gemm_stream_kernel(Args a) {
     __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], sums_full[2], sums_empty[2];
     __shared__ float sums[2][MMA_WARPS][ROWS][NT * 8 + 1];
     __shared__ float squares[MMA_WARPS][TOKENS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const bool leader = elect_one();
     const uint32_t smem_base = smem_u32(smem);
     uint8_t* x_s = smem + (size_t)a.stages * a.stage_bytes;
     constexpr int X_ROWS = NT * 8;
@@ -297,11 +305,11 @@ gemm_stream_kernel(Args a) {
             for (int c = 0; c < a.chunks; ++c, ++it, st = (st + 1 == a.stages ? 0 : st + 1), phase ^= (st == 0 ? 1u : 0u)) {
                 if (it == a.early && !asked) { __syncwarp(); asked_wait<ASKED>(); asked = true; }
                 if (it >= a.stages) {
-                    if (lane == 0) ok = mbar_wait(smem_u32(&empty_bar[st]), phase ^ 1u);
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
+                    ok = mbar_wait(smem_u32(&empty_bar[st]), phase ^ 1u);
+                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                 }
-                if (lane == 0) {
+                if (leader) {
                     const uint32_t full = smem_u32(&full_bar[st]);
                     const int k0 = c * a.ck;
                     const uint32_t bytes = (uint32_t)min(a.ck, a.K - k0) * 2u;

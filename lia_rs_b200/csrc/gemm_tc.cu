@@ -143,7 +143,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __shared__ int last_flag;
 
     constexpr int A_TILES = GATED(MODE) ? 2 : 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const bool leader = elect_one();
     const uint32_t a_bytes = TILE_F * BLOCK_K * 2, b_bytes = (uint32_t)s.n_tile * BLOCK_K * 2;
     const uint32_t stage_bytes = A_TILES * a_bytes + b_bytes;
     // dynamic shared memory is aligned to 1024 bytes by hand (the swizzle pattern repeats every 1024)
@@ -183,7 +184,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         units = min(*s.group_count, s.t_tiles) * s.f_tiles;
     }
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && leader) {
         // ---- TMA producer ----
         // The first ring of W boxes is asked for before the kernel ahead of this one has finished: the
         // weights do not depend on it.  X does, so its boxes wait.
@@ -231,7 +232,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             for (int i = max(0, issued - s.stages); i < issued; ++i)
                 mbar_wait(smem_u32(&full_bar[i % s.stages]), (uint32_t)(i / s.stages) & 1u);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && leader) {
         // ---- MMA issuer ----
         // a tile of more than 256 tokens takes two MMAs per K step: 256 tokens, then the rest
         const int n_first = s.n_tile > 256 ? 256 : s.n_tile, n_rest = s.n_tile - n_first;

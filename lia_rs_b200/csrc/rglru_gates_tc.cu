@@ -53,7 +53,8 @@ rglru_gates_tc_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_co
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[GATES_STAGES], empty_bar[GATES_STAGES], acc_full;
     __shared__ uint32_t tmem_base_slot;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const bool leader = elect_one();
     constexpr uint32_t W_BYTES = TILE_F * BLOCK_K * 2;
     const uint32_t stage_bytes = 2 * W_BYTES + (uint32_t)p.n_tile * BLOCK_K * 2;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -81,7 +82,7 @@ rglru_gates_tc_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_co
     const uint32_t tmem_base = tmem_base_slot;
     pdl_launch_dependents();
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && leader) {
         // ---- TMA producer: the first ring of weights is asked for before the kernel ahead has finished ----
         bool ok = true;
         const int ahead = p.kblocks < GATES_STAGES ? p.kblocks : GATES_STAGES;
@@ -111,7 +112,7 @@ rglru_gates_tc_kernel(const __grid_constant__ CUtensorMap map_r, const __grid_co
             for (int kb = max(0, issued - GATES_STAGES); kb < issued; ++kb)      // the copies that may still be in flight
                 mbar_wait(smem_u32(&full_bar[kb % GATES_STAGES]), (uint32_t)(kb / GATES_STAGES) & 1u);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && leader) {
         // ---- MMA issuer ----
         const uint32_t idesc = instr_desc(TILE_F, p.n_tile);
         const uint64_t desc_r0 = smem_desc(smem_base), desc_i0 = smem_desc(smem_base + W_BYTES), desc_u0 = smem_desc(smem_base + 2 * W_BYTES);

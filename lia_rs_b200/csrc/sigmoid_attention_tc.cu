@@ -124,7 +124,8 @@ sigmoid_attention_tc_kernel(Params p) {
     constexpr int PIECES = D / 8;                      // 16-byte pieces per row
     constexpr uint32_t Q_BYTES = ROWS * D * 2, KV_BYTES = KT * D * 2;
     constexpr int TMEM_COLS = 512;                     // two buffers of 128 columns (scores, then weights) and the output's D
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const bool leader = elect_one();
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t q_s = smem_base, kv_s = q_s + Q_BYTES;   // kv_s: [stage][K, V]
 
@@ -292,7 +293,7 @@ sigmoid_attention_tc_kernel(Params p) {
             mbar_arrive(smem_u32(&v_full[st]));
         }
         if (!ok && p.error_flag) atomicExch(p.error_flag, 3);
-    } else if (warp == WEIGHT_WARPS && lane == 0 && n_tiles > 0) {
+    } else if (warp == WEIGHT_WARPS && leader && n_tiles > 0) {
         // ---- MMA issuer ----
         const uint32_t idesc_s = instr_desc(ROWS, KT), idesc_o = instr_desc_b_mn(ROWS, D);
         bool ok = mbar_wait(smem_u32(&q_full), 0u);
