@@ -40,19 +40,12 @@
 // its loop; the CTA then waits (bounded) for its copies in flight, frees its TMEM and returns.
 #include <algorithm>
 
+#include "gemm_pair.cuh"
 #include "tcgen05.cuh"
 
 using namespace tc5;
 
-#define GEMM_STORE 0
-#define GEMM_ACCUM 1
-#define GEMM_SWIGLU 2
-// More forms of the kernel, instantiations of their own so that the three above are what they were: the gated form
-// with a ReLU gate, out = up * relu(gate), and the storing forms with out = relu(alpha * sum)^2 and out = xIELU(alpha * sum).
-#define GEMM_REGLU 3
-#define GEMM_STORE_RELU2 4
-#define GEMM_STORE_XIELU 5
-#define GATED(MODE) ((MODE) == GEMM_SWIGLU || (MODE) == GEMM_REGLU)
+#define GATED(MODE) GEMM_GATED(MODE)
 
 namespace {
 constexpr int THREADS = 192;
@@ -440,6 +433,14 @@ int pow2_at_least(int x) {
     return p;
 }
 
+// What a round of tiles of n tokens takes (us).  Measured on a B200 (247 products of 160 to 4,096 tokens, within 9%, with 0.8 us for the
+// whole and 0.14 a megabyte of output): 2.6 us, and per K block the longest of its MMAs' time (0.38 at 256 tokens, twice that for
+// the gated product's two accumulators), the time the SM needs to take the block in (a row of W or X is 128 bytes), and 0.21.
+double round_cost(bool gated, int n, int kblocks) {
+    const double weights = gated ? 2.0 : 1.0;
+    return 2.6 + kblocks * std::max(0.214, std::max(0.00148 * weights * n, 0.00093 * (128.0 * weights + n)));
+}
+
 // How the product is cut: tokens per tile, K ranges per tile.  A function of the sizes and of the SM
 // count alone, so the same product is always cut the same way.
 struct Plan {
@@ -458,28 +459,19 @@ Plan make_plan(int mode, int M, int N, int K, int sm_count, long long scratch_fl
         while (p.n_tile < M) p.n_tile *= 2;
     } else {
         // many tokens: the tile width (a multiple of 32, the epilogue's step) that leaves the SMs least idle: rounds of
-        // tiles times the time of one.  Measured on a B200: a tile takes 5.5 us plus, per K block, the longest of
-        // three: its MMAs' time (0.43 us at 256 tokens at the clocks a long product runs at, in proportion below;
-        // twice that for the gated product's two accumulators); the time its SM needs to take the block in (an SM
-        // takes in about 108 GB/s: 16 KB of W, or 32, and 128 bytes per token; this is what a narrow tile waits
-        // for, and why narrower tiles on more SMs beat wide ones on few); and what its producer thread needs to
-        // issue the block's two to four TMA boxes (0.1 us each).  Ties go to the wider tile (fewer bytes through
+        // tiles times the time of one (round_cost).  Ties go to the wider tile (fewer bytes through
         // shared memory per flop).  Up to 512 tokens wide (all of TMEM, so one buffer: the epilogue and the next tile
         // take turns), 256 for the gated product, where that saves a round: 2,048 tokens x 2,560 features are 140
         // tiles of 320 tokens, one round, against 260 of 160.  Down to 32 tokens where the tiles would otherwise be
         // too few for the SMs: K is NOT cut for more than 128 tokens (the CTA that arrives last would add up ranges
         // of hundreds of tokens alone, which costs more than narrow tiles do).
-        const double weights = swiglu ? 2.0 : 1.0;
         const int widest = std::min(swiglu ? 256 : 512, (M + 31) / 32 * 32);
         double best = -1;
         p.n_tile = widest;
         for (int n = widest; n >= 32; n -= 32) {
             const long long tiles = (long long)p.f_tiles * ((M + n - 1) / n);
             const long long rounds = (tiles + sm_count - 1) / sm_count;
-            const double mma = weights * 0.43 * n / 256.0;
-            const double intake = (weights * 16384.0 + n * 128.0) / 108e3;
-            const double issue = 0.1 * (weights + (n > 256 ? 2.0 : 1.0));
-            const double cost = (double)rounds * (5.5 + kblocks * std::max(mma, std::max(intake, issue)));
+            const double cost = (double)rounds * round_cost(swiglu, n, kblocks);
             if (best < 0 || cost < best) { best = cost; p.n_tile = n; }
         }
     }
@@ -533,6 +525,18 @@ LIA_EXPORT int lia_gemm_tc(int mode, const void* X, int ldx, const void* W, int 
     if (out_dtype != LIA_F32 && out_dtype != LIA_BF16) return LIA_ERR_DTYPE;
     const bool swiglu = mode == GEMM_SWIGLU;
     const Plan plan = make_plan(mode, M, N, K, sm_count, scratch ? scratch_floats : 0);
+    // Many tokens: pairs of SMs where they are expected to be faster by the twentieth that the estimates are sure of.  They are for
+    // products of several rounds or wide tiles (us, one CTA a tile / pairs: 2,048 x 8,192 x 2,048 72 / 51, 4,096 x 2,048 x 6,144 110 / 76, 256 x 2,048 pairs x
+    // 2,048 14.1 / 9.5), and not where tiles of one CTA make one full round (2,048 x 2,048 x 6,144 36.1 / 38.9, 1,111 x 3,088 x 1,024 9.8 / 11.0).
+    const int out_bytes = out_dtype == LIA_F32 ? 4 : 2;
+    if (M > 128 && sm_count >= 2 && ((uintptr_t)out & 15u) == 0 && ((long long)ldo * out_bytes) % 16 == 0) {
+        const long long rounds = ((long long)plan.f_tiles * plan.t_tiles + sm_count - 1) / sm_count;
+        const double alone = 0.8 + rounds * round_cost(swiglu, plan.n_tile, (K + BLOCK_K - 1) / BLOCK_K) + 0.14e-6 * out_bytes * M * N;
+        if (gemm_pair_estimate(mode, M, N, K, out_bytes, sm_count) < 0.95 * alone) {
+            const int form = act == 5 ? GEMM_STORE_XIELU : act == 3 ? GEMM_STORE_RELU2 : act == 4 ? GEMM_REGLU : mode;
+            return gemm_pair_launch(form, X, ldx, W, ldw, out, out_dtype, ldo, M, N, K, alpha, sm_count, 0, act_p, act_n, error_flag, stream);
+        }
+    }
 
     Shape s;
     s.M = M; s.N = N; s.K = K; s.n_total = swiglu ? 2 * N : N;
