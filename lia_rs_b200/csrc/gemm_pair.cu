@@ -23,6 +23,9 @@
 // Tiles are narrower than 256 rows of W (a multiple of 32; of 64 for the gated product) where that leaves the pairs less idle in
 // the last round: see plan_width.
 //
+// Grouped products (a mixture of experts): the first product's token tiles are those of a list on the device, each with a group whose
+// matrix it is multiplied with (see lia_gemm_pair_grouped); a second, plain product (a shared expert's) may share the launch.
+//
 // Programmatic dependent launch: the first ring of W boxes is asked for before the kernel ahead has finished; X waits.
 // Every wait on an mbarrier is bounded; a role that gives up raises the error flag and leaves its loop, and all threads of both
 // CTAs still meet at the cluster barrier before TMEM is freed.
@@ -43,12 +46,18 @@ constexpr int CHUNK_F = 32;                      // features of an epilogue piec
 constexpr int RASTER = 8;                        // token tiles that neighbouring pairs share the rows of W of
 constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;  // clears the bit of a shared::cluster address that tells the pair's CTAs apart
 
+// One product of a launch.
+struct Part {
+    int M, N, kblocks, f_tiles, t_tiles;
+};
 struct Shape {
-    int M, N;
+    Part part[2];             // the second only in launches of two products
     int n_tile;               // rows of W per tile (gated: gate and up rows together)
     int width;                // output features per tile: n_tile, or half of it for the gated product
-    int stages, kblocks, f_tiles, t_tiles;
-    int tmem_cols;
+    int stages, tmem_cols;
+    const int* group_tiles;   // grouped: per token tile of the first product (group, first row, rows)
+    const int* group_count;   // grouped: the number of token tiles
+    int group_rows;           // grouped: rows of W per group
     float alpha;
     float act_p, act_n;       // xIELU's two constants
     int* error_flag;
@@ -94,13 +103,30 @@ __device__ __forceinline__ void arrive_on_first(uint32_t bar) {
 // The index-th tile: RASTER token tiles walk the rows of W together, so that what runs at the same time shares both operands in L2.
 struct Unit {
     int t0, f0;               // first token, first output feature
+    int w0;                   // first row of W: f0, plus the group's first row
+    int t_end;                // tokens from here on are not the tile's
+    int second;               // the second product's
 };
-__device__ __forceinline__ Unit unit_at(const Shape& s, int index) {
-    const int band = index / (RASTER * s.f_tiles), t_first = band * RASTER;
-    const int across = min(RASTER, s.t_tiles - t_first), rest = index - band * RASTER * s.f_tiles;
+// GROUPED: the first product's tiles are the list's (`first_units` of them by width), the second product's follow.
+template <bool GROUPED>
+__device__ __forceinline__ Unit unit_at(const Shape& s, int index, int first_units, int listed) {
     Unit u;
-    u.t0 = (t_first + rest % across) * PAIR_M;
-    u.f0 = (rest / across) * s.width;
+    u.second = GROUPED && index >= first_units ? 1 : 0;
+    if (u.second) index -= first_units;
+    const Part& p = s.part[GROUPED ? u.second : 0];
+    const int t_tiles = GROUPED && !u.second ? listed : p.t_tiles;
+    const int band = index / (RASTER * p.f_tiles), t_first = band * RASTER;
+    const int across = min(RASTER, t_tiles - t_first), rest = index - band * RASTER * p.f_tiles;
+    const int tile = t_first + rest % across;
+    u.f0 = u.w0 = (rest / across) * s.width;
+    if (GROUPED && !u.second) {
+        u.w0 += s.group_tiles[3 * tile] * s.group_rows;
+        u.t0 = s.group_tiles[3 * tile + 1];
+        u.t_end = u.t0 + s.group_tiles[3 * tile + 2];
+    } else {
+        u.t0 = tile * PAIR_M;
+        u.t_end = p.M;
+    }
     return u;
 }
 
@@ -137,10 +163,15 @@ __device__ __forceinline__ void put_row(uint8_t* piece, int lane, const float (&
                        pack_pair(v[8 * j + 6], v[8 * j + 7]));
 }
 
-template <int MODE, typename TO>
+// The tensor maps of a launch's products: W, X and the output of the first, then of the second.
+template <bool GROUPED>
+struct Maps {
+    CUtensorMap w[GROUPED ? 2 : 1], x[GROUPED ? 2 : 1], o[GROUPED ? 2 : 1];
+};
+
+template <int MODE, typename TO, bool GROUPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                 const __grid_constant__ CUtensorMap map_o, Shape s) {
+gemm_pair_kernel(const __grid_constant__ Maps<GROUPED> maps, const __grid_constant__ Shape s) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[MAX_STAGES], empty_bar[MAX_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_slot;
@@ -153,7 +184,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const uint32_t stage_bytes = A_BYTES + (uint32_t)half_n * BLOCK_K * 2;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t staging_base = smem_base + (uint32_t)s.stages * stage_bytes;      // a piece of [32 tokens][32 features] a warp
-    const int units = s.f_tiles * s.t_tiles;
+    int first_units = s.part[0].f_tiles * s.part[0].t_tiles, listed = s.part[0].t_tiles;
+    int units = first_units + (GROUPED ? s.part[1].f_tiles * s.part[1].t_tiles : 0);
     const int first_unit = blockIdx.x >> 1, stride = gridDim.x >> 1;
 
     if (warp == 0 && lane == 0) {
@@ -167,9 +199,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_o) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.w[0]) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[0]) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.o[0]) : "memory");
     }
     if (warp == 1) {
         // both CTAs of the pair allocate, with the same destination offset
@@ -184,21 +216,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
     pdl_launch_dependents();
+    if (GROUPED) {
+        pdl_wait();           // the list of tiles is the work of a kernel ahead
+        listed = min(*s.group_count, s.part[0].t_tiles);
+        first_units = listed * s.part[0].f_tiles;
+        units = first_units + s.part[1].f_tiles * s.part[1].t_tiles;
+    }
 
     if (warp == 0 && leader) {
         // ---- TMA producer (both CTAs): this CTA's 128 tokens, its half of the tile's rows of W ----
         // gated: the first CTA brings gate rows, the second up rows of the same features
-        const int w_first = GEMM_GATED(MODE) ? (rank == 0 ? 0 : s.N) : (int)rank * half_n;
+        const auto w_first = [&](const Part& p) { return GEMM_GATED(MODE) ? (rank == 0 ? 0 : p.N) : (int)rank * half_n; };
         bool ok = true;
         int ahead = 0;
-        {   // the first ring of W boxes goes out before the kernel ahead has finished: weights depend on nothing
+        if (!GROUPED) {   // the first ring of W boxes goes out before the kernel ahead has finished: weights depend on nothing
             int it = 0;
             for (int index = first_unit; index < units && it < s.stages; index += stride) {
-                const Unit u = unit_at(s, index);
-                for (int kb = 0; kb < s.kblocks && it < s.stages; ++kb, ++it) {
+                const Unit u = unit_at<GROUPED>(s, index, first_units, listed);
+                for (int kb = 0; kb < s.part[0].kblocks && it < s.stages; ++kb, ++it) {
                     const uint32_t full = smem_u32(&full_bar[it]);
                     if (rank == 0) mbar_expect_tx(full, 2 * stage_bytes);
-                    tma_load_pair(smem_base + (uint32_t)it * stage_bytes + A_BYTES, &map_w, kb * BLOCK_K, w_first + u.f0, full);
+                    tma_load_pair(smem_base + (uint32_t)it * stage_bytes + A_BYTES, &maps.w[0], kb * BLOCK_K, w_first(s.part[0]) + u.w0, full);
                 }
             }
             ahead = it;
@@ -207,17 +245,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         int it = 0, st = 0;
         uint32_t phase = 0;
         for (int index = first_unit; index < units && ok; index += stride) {
-            const Unit u = unit_at(s, index);
-            const int t_mine = u.t0 + (int)rank * HALF_M, w_mine = w_first + u.f0;
-            for (int kb = 0; kb < s.kblocks; ++kb, ++it) {
+            const Unit u = unit_at<GROUPED>(s, index, first_units, listed);
+            const int which = GROUPED ? u.second : 0;
+            const Part& p = s.part[which];
+            const CUtensorMap *map_w = &maps.w[which], *map_x = &maps.x[which];
+            const int t_mine = u.t0 + (int)rank * HALF_M, w_mine = w_first(p) + u.w0;
+            for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
                 const uint32_t full = smem_u32(&full_bar[st]);
                 const uint32_t dst = smem_base + (uint32_t)st * stage_bytes;
                 if (it >= ahead) {
                     if (!mbar_wait(smem_u32(&empty_bar[st]), phase ^ 1u)) { ok = false; break; }
                     if (rank == 0) mbar_expect_tx(full, 2 * stage_bytes);
-                    tma_load_pair(dst + A_BYTES, &map_w, kb * BLOCK_K, w_mine, full);
+                    tma_load_pair(dst + A_BYTES, map_w, kb * BLOCK_K, w_mine, full);
                 }
-                tma_load_pair(dst, &map_x, kb * BLOCK_K, t_mine, full);
+                tma_load_pair(dst, map_x, kb * BLOCK_K, t_mine, full);
                 if (++st == s.stages) { st = 0; phase ^= 1u; }
             }
         }
@@ -240,7 +281,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             if (!mbar_wait(smem_u32(&acc_empty[buf]), (((uint32_t)n_unit >> 1) & 1u) ^ 1u)) { ok = false; break; }
             tc_fence_after();
             const uint32_t acc = tmem_base + (uint32_t)(buf * s.n_tile);
-            for (int kb = 0; kb < s.kblocks; ++kb) {
+            const int kblocks = s.part[GROUPED && index >= first_units ? 1 : 0].kblocks;
+            for (int kb = 0; kb < kblocks; ++kb) {
                 if (!mbar_wait(smem_u32(&full_bar[st]), phase)) { ok = false; break; }
                 tc_fence_after();
                 const uint64_t da = desc_a0 + stage_offset, db = desc_b0 + stage_offset;
@@ -264,15 +306,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         bool ok = true;
         int n_unit = 0;
         for (int index = first_unit; index < units && ok; index += stride, ++n_unit) {
-            const Unit u = unit_at(s, index);
+            const Unit u = unit_at<GROUPED>(s, index, first_units, listed);
+            const int N = s.part[GROUPED ? u.second : 0].N;
+            const CUtensorMap* map_o = &maps.o[GROUPED ? u.second : 0];
             const int t = u.t0 + (int)rank * HALF_M + group * 32;
             const int buf = n_unit & 1;
             if (!mbar_wait(smem_u32(&acc_full[buf]), ((uint32_t)n_unit >> 1) & 1u)) { ok = false; break; }
             tc_fence_after();
             const uint32_t lane_addr = tmem_base + ((uint32_t)(group * 32) << 16) + (uint32_t)(buf * s.n_tile);
-            if (t < s.M) {
+            if (t < u.t_end) {
                 for (int c0 = set * CHUNK_F; c0 < s.width; c0 += 2 * CHUNK_F) {
-                    if (u.f0 + c0 >= s.N) break;
+                    if (u.f0 + c0 >= N) break;
                     float acc[32], up[32];
                     tmem_load32_nowait(lane_addr + (uint32_t)c0, acc);
                     if (GEMM_GATED(MODE)) tmem_load32_nowait(lane_addr + (uint32_t)(s.width + c0), up);
@@ -285,8 +329,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                     fence_async_smem();
                     __syncwarp();
                     if (lane == 0) {
-                        if (MODE == GEMM_ACCUM) tma_reduce_add_2d(&map_o, piece_addr, u.f0 + c0, t);
-                        else tma_store_2d(&map_o, piece_addr, u.f0 + c0, t);
+                        if (MODE == GEMM_ACCUM) tma_reduce_add_2d(map_o, piece_addr, u.f0 + c0, t);
+                        else tma_store_2d(map_o, piece_addr, u.f0 + c0, t);
                         tma_commit_group();
                     }
                 }
@@ -329,18 +373,33 @@ int make_piece_map(CUtensorMap* map, void* base, int out_dtype, int M, int N, in
     return r == CUDA_SUCCESS ? LIA_OK : LIA_ERR_DRIVER;
 }
 
-template <int MODE, typename TO>
-int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mo, const Shape& s, int pairs, cudaStream_t stream) {
+template <int MODE, typename TO, bool GROUPED>
+int launch(const Maps<GROUPED>& maps, const Shape& s, int pairs, cudaStream_t stream) {
     static std::atomic<bool> configured{false};
     if (!configured.load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(gemm_pair_kernel<MODE, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
+        if (cudaFuncSetAttribute(gemm_pair_kernel<MODE, TO, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
             cudaGetLastError();
             return LIA_ERR_LAUNCH;
         }
         configured.store(true, std::memory_order_release);
     }
-    return lia_launch(gemm_pair_kernel<MODE, TO>, dim3(2 * pairs), dim3(THREADS), (size_t)SMEM_BYTES, stream, mw, mx, mo, s);
+    return lia_launch(gemm_pair_kernel<MODE, TO, GROUPED>, dim3(2 * pairs), dim3(THREADS), (size_t)SMEM_BYTES, stream, maps, s);
 }
+
+// The parts of a launch that follow from the tile's width.
+void set_width(Shape* s, bool gated, int n_tile, int out_bytes) {
+    s->n_tile = n_tile;
+    s->width = gated ? n_tile / 2 : n_tile;
+    s->tmem_cols = pow2_columns(2 * n_tile);
+    const int staging = EPILOGUE_WARPS * 32 * CHUNK_F * out_bytes, stage_bytes = HALF_M * BLOCK_K * 2 + (n_tile / 2) * BLOCK_K * 2;
+    s->stages = std::min(MAX_STAGES, (SMEM_BYTES - 1024 - staging) / stage_bytes);
+}
+Part part_of(int M, int N, int K, int width) {
+    return {M, N, (K + BLOCK_K - 1) / BLOCK_K, (N + width - 1) / width, (M + PAIR_M - 1) / PAIR_M};
+}
+
+// What a tile of n rows of W and so many K blocks takes in a round of tiles (us; see plan_width).
+double tile_cost(int kblocks, int n) { return kblocks * std::max(0.152, 0.026 + 0.00108 * n) + 0.54; }
 
 // Rows of W per tile, and the time this is expected to take (us).  Measured on a B200 (2,023 products of 160 to 4,096 tokens by 160 to 8,192
 // features, K 128 to 8,192, in tiles of 32 to 256 rows; within 7%): a product begins and ends in 3.8 us, a round of tiles costs 0.54 and per
@@ -356,7 +415,7 @@ double plan_width(bool gated, int M, int N, int K, int out_bytes, int sm_count, 
         const int width = gated ? n / 2 : n;
         const long long tiles = (long long)t_tiles * ((N + width - 1) / width);
         const long long rounds = (tiles + pairs - 1) / pairs;
-        const double cost = 3.8 + rounds * (kblocks * std::max(0.152, 0.026 + 0.00108 * n) + 0.54) + 0.16e-6 * out_bytes * M * N;
+        const double cost = 3.8 + rounds * tile_cost(kblocks, n) + 0.16e-6 * out_bytes * M * N;
         if (best < 0 || cost < best) { best = cost; *n_tile = n; }
     }
     return best;
@@ -373,38 +432,94 @@ int gemm_pair_launch(int mode, const void* X, int ldx, const void* W, int ldw, v
     const bool gated = GEMM_GATED(mode);
     if (n_tile == 0) plan_width(gated, M, N, K, out_dtype == LIA_F32 ? 4 : 2, sm_count, &n_tile);
     if (n_tile < 32 || n_tile > 256 || n_tile % (gated ? 64 : 32) || sm_count < 2) return LIA_ERR_SIZE;
-    Shape s;
-    s.M = M; s.N = N; s.n_tile = n_tile; s.width = gated ? n_tile / 2 : n_tile;
-    s.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
-    s.f_tiles = (N + s.width - 1) / s.width;
-    s.t_tiles = (M + PAIR_M - 1) / PAIR_M;
-    s.tmem_cols = pow2_columns(2 * n_tile);
+    Shape s = {};
+    set_width(&s, gated, n_tile, out_dtype == LIA_F32 ? 4 : 2);
+    s.part[0] = part_of(M, N, K, s.width);
     s.alpha = alpha; s.act_p = act_p; s.act_n = act_n; s.error_flag = error_flag;
-    const int esize = out_dtype == LIA_F32 ? 4 : 2;
-    const int staging = EPILOGUE_WARPS * 32 * CHUNK_F * esize;
-    const int stage_bytes = HALF_M * BLOCK_K * 2 + (n_tile / 2) * BLOCK_K * 2;
-    s.stages = std::min(MAX_STAGES, (SMEM_BYTES - 1024 - staging) / stage_bytes);
-
-    CUtensorMap mw, mx, mo;
+    Maps<false> maps;
     int rc;
-    if ((rc = make_map(&mw, W, gated ? 2 * N : N, K, ldw, n_tile / 2)) != LIA_OK) return rc;
-    if ((rc = make_map(&mx, X, M, K, ldx, HALF_M)) != LIA_OK) return rc;
-    if ((rc = make_piece_map(&mo, out, out_dtype, M, N, ldo)) != LIA_OK) return rc;
-    const int pairs = (int)std::min((long long)(sm_count / 2), (long long)s.f_tiles * s.t_tiles);
+    if ((rc = make_map(&maps.w[0], W, gated ? 2 * N : N, K, ldw, n_tile / 2)) != LIA_OK) return rc;
+    if ((rc = make_map(&maps.x[0], X, M, K, ldx, HALF_M)) != LIA_OK) return rc;
+    if ((rc = make_piece_map(&maps.o[0], out, out_dtype, M, N, ldo)) != LIA_OK) return rc;
+    const int pairs = (int)std::min((long long)(sm_count / 2), (long long)s.part[0].f_tiles * s.part[0].t_tiles);
 #define LIA_PAIR(MODE)                                                                             \
     case MODE:                                                                                     \
-        return out_dtype == LIA_F32 ? launch<MODE, float>(mw, mx, mo, s, pairs, stream)            \
-                                    : launch<MODE, __nv_bfloat16>(mw, mx, mo, s, pairs, stream)
+        return out_dtype == LIA_F32 ? launch<MODE, float, false>(maps, s, pairs, stream)           \
+                                    : launch<MODE, __nv_bfloat16, false>(maps, s, pairs, stream)
     switch (mode) {
         LIA_PAIR(GEMM_STORE);
         LIA_PAIR(GEMM_SWIGLU);
         LIA_PAIR(GEMM_REGLU);
         LIA_PAIR(GEMM_STORE_RELU2);
         LIA_PAIR(GEMM_STORE_XIELU);
-        case GEMM_ACCUM: return launch<GEMM_ACCUM, float>(mw, mx, mo, s, pairs, stream);
+        case GEMM_ACCUM: return launch<GEMM_ACCUM, float, false>(maps, s, pairs, stream);
     }
 #undef LIA_PAIR
     return LIA_ERR_SIZE;
+}
+
+// A grouped product and, in the same launch, a plain one.  The first: X [rows_cap, K] bf16 = the tokens' rows sorted by group, every group's
+// rows beginning at a multiple of 32 (a warp's stores, beyond which a tile writes nothing); W [groups, n_total, K] (n_total = N, or 2N for SWIGLU: gate rows then up rows); out [rows_cap, N].  `tiles`
+// [3 * max_tiles] on the device lists (group, first row, rows) per token tile, `n_tiles` [1] how many there are; `expected` (a number of
+// tiles) decides the tiles' width only.  Rows of out that belong to no tile's rows may be written.  The second (M2 0: none): out2 [M2, N2] = X2 [M2, K2] W2^T
+// in the same form.  mode: GEMM_SWIGLU (bf16 or f32 out), GEMM_STORE, or GEMM_STORE with 3 above its byte (relu(sum)^2).
+// What bounds it is W: eight experts of 2,048 pairs x 2,048 are 134 MB, 20 us of memory.  A launch for either product of a
+// mixture, routed and shared expert in tiles of one CTA each, took 2 x 32 and 2 x 22 us at 512 tokens (eight experts of 2,048, two chosen); so the whole
+// part went from 102 to 77.
+LIA_EXPORT int lia_gemm_pair_grouped(int mode, const void* X, int ldx, int rows_cap, const void* W, int ldw, int groups, void* out,
+                                     int out_dtype, int ldo, int N, int K, const int* tiles, const int* n_tiles, int max_tiles, int expected,
+                                     const void* X2, int ldx2, int M2, const void* W2, int ldw2, void* out2, int ldo2, int N2, int K2,
+                                     int sm_count, int* error_flag, cudaStream_t stream) {
+    const int act = mode >> 8;
+    mode &= 0xff;
+    if ((mode != GEMM_STORE && mode != GEMM_SWIGLU) || (act != 0 && !(mode == GEMM_STORE && act == 3))) return LIA_ERR_SIZE;
+    if (rows_cap <= 0 || N <= 0 || max_tiles <= 0) return LIA_ERR_SIZE;
+    if (K <= 0 || K % 8 || ldx < K || ldw < K || ldo < N || sm_count < 2 || groups <= 0 || !tiles || !n_tiles || M2 < 0)
+        return LIA_ERR_SIZE;
+    if (M2 > 0 && (N2 <= 0 || K2 <= 0 || K2 % 8 || ldx2 < K2 || ldw2 < K2 || ldo2 < N2)) return LIA_ERR_SIZE;
+    if (out_dtype != LIA_F32 && out_dtype != LIA_BF16) return LIA_ERR_DTYPE;
+    const bool gated = mode == GEMM_SWIGLU;
+    const int out_bytes = out_dtype == LIA_F32 ? 4 : 2, n_total = gated ? 2 * N : N;
+    if (((uintptr_t)out & 15u) || ((long long)ldo * out_bytes) % 16 || (M2 > 0 && (((uintptr_t)out2 & 15u) || ((long long)ldo2 * out_bytes) % 16)))
+        return LIA_ERR_ALIGN;
+    if ((long long)groups * n_total > 0x7fffffffLL) return LIA_ERR_SIZE;
+    // the width that leaves the pairs least idle, with as many tiles in the list as are expected
+    const int pairs = sm_count / 2, kblocks = (std::max(K, M2 > 0 ? K2 : 0) + BLOCK_K - 1) / BLOCK_K, step = gated ? 64 : 32;
+    double best = -1;
+    int n_tile = 256;
+    for (int n = 256; n >= step; n -= step) {
+        const int width = gated ? n / 2 : n;
+        const long long units = (long long)std::max(1, std::min(expected, max_tiles)) * ((N + width - 1) / width) +
+                                (M2 > 0 ? (long long)((M2 + PAIR_M - 1) / PAIR_M) * ((N2 + width - 1) / width) : 0);
+        const double cost = (units + pairs - 1) / pairs * tile_cost(kblocks, n);
+        if (best < 0 || cost < best) { best = cost; n_tile = n; }
+    }
+    Shape s = {};
+    set_width(&s, gated, n_tile, out_bytes);
+    s.part[0] = part_of(rows_cap, N, K, s.width);
+    s.part[0].t_tiles = max_tiles;
+    if (M2 > 0) s.part[1] = part_of(M2, N2, K2, s.width);
+    s.alpha = 1.0f; s.error_flag = error_flag;
+    s.group_tiles = tiles; s.group_count = n_tiles; s.group_rows = n_total;
+    Maps<true> maps;
+    int rc;
+    if ((rc = make_map(&maps.w[0], W, groups * n_total, K, ldw, n_tile / 2)) != LIA_OK) return rc;
+    if ((rc = make_map(&maps.x[0], X, rows_cap, K, ldx, HALF_M)) != LIA_OK) return rc;
+    if ((rc = make_piece_map(&maps.o[0], out, out_dtype, rows_cap, N, ldo)) != LIA_OK) return rc;
+    if (M2 > 0) {
+        if ((rc = make_map(&maps.w[1], W2, gated ? 2 * N2 : N2, K2, ldw2, n_tile / 2)) != LIA_OK) return rc;
+        if ((rc = make_map(&maps.x[1], X2, M2, K2, ldx2, HALF_M)) != LIA_OK) return rc;
+        if ((rc = make_piece_map(&maps.o[1], out2, out_dtype, M2, N2, ldo2)) != LIA_OK) return rc;
+    } else {
+        maps.w[1] = maps.w[0]; maps.x[1] = maps.x[0]; maps.o[1] = maps.o[0];
+    }
+    const long long units = (long long)s.part[0].f_tiles * max_tiles + (long long)s.part[1].f_tiles * s.part[1].t_tiles;
+    const int grid = (int)std::min((long long)pairs, units);
+    const bool f32 = out_dtype == LIA_F32;
+    if (gated) return f32 ? launch<GEMM_SWIGLU, float, true>(maps, s, grid, stream) : launch<GEMM_SWIGLU, __nv_bfloat16, true>(maps, s, grid, stream);
+    if (act == 3)
+        return f32 ? launch<GEMM_STORE_RELU2, float, true>(maps, s, grid, stream) : launch<GEMM_STORE_RELU2, __nv_bfloat16, true>(maps, s, grid, stream);
+    return f32 ? launch<GEMM_STORE, float, true>(maps, s, grid, stream) : launch<GEMM_STORE, __nv_bfloat16, true>(maps, s, grid, stream);
 }
 
 // The product on pairs of SMs with tiles of `n_tile` rows of W (0: as many as it would choose), for tests and measurements; lia_gemm_tc

@@ -10,8 +10,9 @@
 //    whose logistic function is the gate of a shared expert.
 //  * `moe_plan`: the (token, choice) pairs grouped by expert: where each expert's rows begin, which pair each sorted row
 //    is, where each pair went, and the list of (expert, first row, rows) tiles of `tile_rows` rows that the products run
-//    over.  With `pad` every expert's group begins at a multiple of `tile_rows` (rows in between belong to no pair), so
-//    that a tile of the tensor-core product (csrc/gemm_tc.cu, grouped) never holds rows of two experts.
+//    over.  With `pad` every expert's group begins at a multiple of `pad` rows (rows in between belong to no pair), so
+//    that what a tile of a tensor-core product stores never reaches another expert's rows (csrc/gemm_tc.cu, grouped: whole tiles, pad =
+//    tile_rows; csrc/gemm_pair.cu: 32 rows at a time).
 //    Which pair gets which row inside an expert's group is not fixed, and does not matter: every row of a product is
 //    computed for itself, its sum over K in ascending order.
 //  * `moe_gather`: the sorted rows' inputs side by side (rows of no pair are zero), for the tensor-core product.
@@ -190,7 +191,7 @@ __global__ void moe_plan_kernel(const int* __restrict__ ids, int pairs, int expe
     if (threadIdx.x == 0) {
         int at = 0, tile = 0;
         for (int e = 0; e < experts; ++e) {
-            if (pad) at = tile * tile_rows;
+            if (pad) at = (at + pad - 1) / pad * pad;
             starts[e] = at;
             tile_starts[e] = tile;
             at += counts[e];
@@ -457,13 +458,13 @@ LIA_EXPORT int lia_moe_route(const void* x, int dtype, long long ld, const float
 }
 
 // ids [pairs]; offsets [experts + 1]; order [pairs, or rows_cap with pad]; inverse [pairs]; tiles [3 * (pairs / tile_rows +
-// min(experts, pairs))]; n_tiles [1].  pad: every expert's rows begin at a multiple of tile_rows, and `order` is -1 on the
-// rows of no pair, up to rows_cap = tile_rows * the most tiles.
+// min(experts, pairs))]; n_tiles [1].  pad > 0: every expert's rows begin at a multiple of pad, and `order` is -1 on the
+// rows of no pair, up to rows_cap, at least pad * (pairs / pad + min(experts, pairs)).
 LIA_EXPORT int lia_moe_plan(const int* ids, int pairs, int experts, int tile_rows, int pad, int rows_cap, int* offsets,
                             int* order, int* inverse, int* tiles, int* n_tiles, cudaStream_t stream) {
     if (pairs <= 0) return LIA_OK;
-    if (experts <= 0 || experts > MOE_MAX_EXPERTS || tile_rows <= 0) return LIA_ERR_SIZE;
-    if (pad && rows_cap < (pairs / tile_rows + min(experts, pairs)) * tile_rows) return LIA_ERR_SIZE;
+    if (experts <= 0 || experts > MOE_MAX_EXPERTS || tile_rows <= 0 || pad < 0) return LIA_ERR_SIZE;
+    if (pad && rows_cap < ((long long)pairs / pad + min(experts, pairs)) * pad) return LIA_ERR_SIZE;
     return lia_launch(moe_plan_kernel, dim3(1), dim3(1024), 0, stream, ids, pairs, experts, tile_rows, pad, rows_cap, offsets,
                       order, inverse, tiles, n_tiles);
 }

@@ -63,6 +63,8 @@ class _Signatures:
                    c_void_p, ctypes.c_longlong, c_int, c_float, c_float, c_void_p, c_void_p]
     lia_gemm_pair = [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                      c_int, c_int, c_void_p, c_void_p]
+    lia_gemm_pair_grouped = [c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                             c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
     lia_gemm_cluster = [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                         c_int, c_void_p, c_void_p]
     lia_gemm_cluster_ring = [c_int, c_int, c_int, c_void_p]
@@ -1494,6 +1496,7 @@ def gate_rows(o, g, act: int, span: int = 1):
 
 # ---- a mixture of gated experts: csrc/moe.cu ----
 MOE_MAX_EXPERTS, MOE_MAX_TOP = 1024, 32
+PAIR_ROWS, PAIR_STORE_ROWS = 256, 32             # of the grouped product on pairs of SMs: rows of a token tile, rows that a warp stores at once
 
 
 def moe_tile_rows() -> int:
@@ -1544,20 +1547,26 @@ def moe_route(x, router, top: int, scale: float, ids, weights, shared_gate=None,
                                    1 if sigmoid else 0, 1 if two_best else 0, _p(ids), _p(weights), _p(shared_gate), _stream()), "moe_route")
 
 
-def moe_plan(ids, experts: int, offsets, order, inverse, tiles, n_tiles, tile_rows: int = 0, pad: bool = False):
+def moe_padded_rows(pairs: int, experts: int, pad: int) -> int:
+    """The most rows of `pairs` pairs grouped by expert, every expert's rows beginning at a multiple of `pad`."""
+    return (pairs // pad + min(experts, pairs)) * pad
+
+
+def moe_plan(ids, experts: int, offsets, order, inverse, tiles, n_tiles, tile_rows: int = 0, pad=False):
     """The pairs grouped by expert: offsets [experts + 1], order (which pair a sorted row is) and inverse [pairs], the list
     of (expert, first row, rows) tiles of `tile_rows` rows (0: the 32-bit product's) and its length.  `pad`: every
-    expert's rows begin at a multiple of tile_rows; `order` then has tile_rows * the most tiles entries, -1 on the rows
+    expert's rows begin at a multiple of it (True: of tile_rows); `order` then has `moe_padded_rows` entries, -1 on the rows
     of no pair."""
     _cuda(ids, offsets, order, inverse, tiles, n_tiles)
     pairs = ids.numel()
     tile_rows = tile_rows or moe_tile_rows()
+    pad = tile_rows if pad is True else int(pad)
     most = moe_max_tiles(pairs, experts, tile_rows)
-    if offsets.numel() < experts + 1 or order.numel() < (most * tile_rows if pad else pairs) or inverse.numel() < pairs or \
+    if offsets.numel() < experts + 1 or order.numel() < (moe_padded_rows(pairs, experts, pad) if pad else pairs) or inverse.numel() < pairs or \
             tiles.numel() < 3 * most:
         raise KernelError("moe_plan: a list is too short")
     with _timed("moe_plan"):
-        _check(lib().lia_moe_plan(_p(ids), pairs, int(experts), int(tile_rows), 1 if pad else 0, order.numel(), _p(offsets),
+        _check(lib().lia_moe_plan(_p(ids), pairs, int(experts), int(tile_rows), pad, order.numel(), _p(offsets),
                                   _p(order), _p(inverse), _p(tiles), _p(n_tiles), _stream()), "moe_plan")
 
 
@@ -1605,6 +1614,44 @@ def gemm_tc_grouped(mode, a, w, out, tile_rows: int, tiles, n_tiles, max_tiles: 
         _check(lib().lia_gemm_tc_grouped(mode | (int(act) << 8), _p(a), a.stride(0), rows, _p(w), K, w.shape[0], _p(out), dtype_code(out.dtype),
                                          out.stride(0), N, K, int(tile_rows), _p(tiles), _p(n_tiles), int(max_tiles), sms,
                                          _p(error_flag), _stream()), "gemm_tc_grouped")
+
+
+def moe_pair_tile_rows(pairs: int, experts: int) -> tuple:
+    """(rows of a token tile, rows that every expert's begin at a multiple of) of the product over the experts on pairs of SMs
+    (csrc/gemm_pair.cu), which takes the shared expert's product into the same launch; (0, 0) where there are few rows an expert, which the
+    one-CTA product (`gemm_tc_grouped`) is for: a tile is 256 rows of the MMA however few an expert has, which many small experts feel
+    first.  us of the whole part, one CTA / pairs: 8 experts of 2,048 and a shared one, hidden 2,048, two chosen, 8 tokens 59.7/60.4, 16 tokens
+    65.8/62.0, 64 80/63, 512 102/77, 2,048 188/174; 64 experts of 512, six chosen, 43 tokens 112/121, 128 126/125, 512 154/152, 2,048 289/264."""
+    return (PAIR_ROWS, PAIR_STORE_ROWS) if pairs >= min(12, max(4, experts / 5)) * experts else (0, 0)
+
+
+def gemm_pair_grouped(mode, a, w, out, tiles, n_tiles, max_tiles: int, pairs: int, shared=None, error_flag=None, label=None, act: int = 0):
+    """out[r] = a[r] @ w[e(r)]^T on pairs of SMs, rows sorted by expert as `moe_plan` lists them with `moe_pair_tile_rows`'s tiles
+    and padding; and in the same launch `shared` (a, w, out), a plain product of the same form (csrc/gemm_pair.cu)."""
+    a2, w2, out2 = shared or (None, None, None)
+    _cuda(a, w, out, tiles, n_tiles, a2, w2, out2)
+    rows, K = a.shape
+    N, gated = out.shape[1], mode == GEMM_SWIGLU
+    if w.dim() != 3 or w.shape[1] != (2 * N if gated else N) or w.shape[2] != K or out.shape[0] != rows or not w.is_contiguous() or \
+            a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or a.stride(1) != 1 or out.stride(1) != 1 or tiles.numel() < 3 * max_tiles:
+        raise KernelError("gemm_pair_grouped: shapes or element types do not agree")
+    M2 = N2 = K2 = lda2 = ldw2 = ldo2 = 0
+    if shared:
+        (M2, K2), N2 = a2.shape, out2.shape[1]
+        if w2.shape[0] != (2 * N2 if gated else N2) or w2.shape[1] != K2 or out2.shape[0] != M2 or out2.dtype != out.dtype or \
+                a2.dtype != torch.bfloat16 or w2.dtype != torch.bfloat16 or a2.stride(1) != 1 or w2.stride(1) != 1 or out2.stride(1) != 1:
+            raise KernelError("gemm_pair_grouped: the second product's shapes or element types do not agree")
+        lda2, ldw2, ldo2 = a2.stride(0), w2.stride(0), out2.stride(0)
+    experts = w.shape[0]
+    # token tiles to expect: an expert's rows spread around pairs / experts
+    rows_each = pairs / experts
+    expected = experts * max(1, round((rows_each + 2 * rows_each ** 0.5) / PAIR_ROWS))
+    _, sms = _device_scratch(a.device)
+    with _timed("gemm_pair_grouped", label, nbytes=(w.numel() + (w2.numel() if shared else 0)) * w.element_size(),
+                flops=2 * (pairs * w.shape[1] * K + M2 * (w2.shape[0] if shared else 0) * K2)):
+        _check(lib().lia_gemm_pair_grouped(mode | (int(act) << 8), _p(a), a.stride(0), rows, _p(w), K, experts, _p(out), dtype_code(out.dtype),
+                                           out.stride(0), N, K, _p(tiles), _p(n_tiles), int(max_tiles), expected, _p(a2), lda2, M2, _p(w2), ldw2,
+                                           _p(out2), ldo2, N2, K2, sms, _p(error_flag), _stream()), "gemm_pair_grouped")
 
 
 def moe_combine(residual, y, inverse, weights, shared_y, shared_gate, top: int, alpha: float, store: bool, x=None):

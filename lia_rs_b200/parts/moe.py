@@ -130,6 +130,8 @@ class ExpertMixture(FeedForward):
         self.router = torch.cat(router, dim=0).to(torch.float32).contiguous()
         self.correction = tensors[prefix + n["correction"]].to(torch.float32).contiguous() if params.get("correction") else None
         self.grouped = None          # whether the tensor-core product takes the experts' matrices: known at the first step
+        # whether the shared expert's can go with them (TMA reads whole rows of 16 bytes)
+        self.shared_fits = not self.shared or all(w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0 for w in (self.w_shared_gate_up, self.w_shared_down))
 
     def forward(self, ctx, x, residual, scale, store=False):
         rt, n = self.runtime, x.shape[0]
@@ -143,24 +145,39 @@ class ExpertMixture(FeedForward):
                       groups=self.groups, keep=self.keep, renormalise=self.renormalise, sigmoid=self.sigmoid, two_best=self.two_best)
         if self.grouped is None:
             self.grouped = ops.moe_grouped_accepts(x, self.w_gate_up, self.w_down)
+        # pairs of SMs take the shared expert's products into the same launches
+        tile_rows, pad = ops.moe_pair_tile_rows(pairs, experts) if self.grouped and self.shared_fits else (0, 0)
+        on_pairs = tile_rows > 0
         if self.grouped:
-            # the tensor cores: every expert's rows begin at a multiple of the tile, the rows' inputs are laid side by side
-            tile_rows = ops.moe_grouped_tile_rows(pairs, experts)
-            max_tiles = ops.moe_max_tiles(pairs, experts, tile_rows)
-            rows = max_tiles * tile_rows
+            # the tensor cores: every expert's rows begin at a multiple of what a tile stores at once, the rows' inputs are laid side by side
+            if not on_pairs:
+                tile_rows = pad = ops.moe_grouped_tile_rows(pairs, experts)
+            max_tiles, rows = ops.moe_max_tiles(pairs, experts, tile_rows), ops.moe_padded_rows(pairs, experts, pad)
         else:
-            tile_rows, max_tiles, rows = 0, ops.moe_max_tiles(pairs, experts), pairs
+            max_tiles, rows = ops.moe_max_tiles(pairs, experts), pairs
         lists = scratch("moe.lists", experts + 2 + rows + pairs + 3 * max_tiles, torch.int32)
         offsets, n_tiles = lists[:experts + 1], lists[experts + 1:experts + 2]
         order, inverse = lists[experts + 2:experts + 2 + rows], lists[experts + 2 + rows:experts + 2 + rows + pairs]
         tiles = lists[experts + 2 + rows + pairs:]
         # (pairs whose output names no expert, the identity outputs, get no row: `inverse` is negative there)
-        ops.moe_plan(ids.view(-1), experts, offsets, order, inverse, tiles, n_tiles, tile_rows, pad=self.grouped)
+        ops.moe_plan(ids.view(-1), experts, offsets, order, inverse, tiles, n_tiles, tile_rows, pad=pad)
         act = shaped("moe.act", (rows, self.ff), dtype)
         y = shaped("moe.y", (rows, self.hidden), torch.float32)
+        shared_y = None
+        if self.shared:
+            shared_act = ctx.buffer("moe.shared_act", (n, self.ffs), dtype)
+            shared_y = ctx.buffer("moe.shared_y", (n, self.hidden), torch.float32)
         if self.grouped:
             sorted_x = shaped("moe.x", (rows, self.hidden), dtype)
             ops.moe_gather(x, order, top, sorted_x)
+        if on_pairs:
+            ops.gemm_pair_grouped(SWIGLU if self.gated else STORE, sorted_x, self.w_gate_up, act, tiles, n_tiles, max_tiles, pairs,
+                                  (x, self.w_shared_gate_up, shared_act) if self.shared else None, error_flag=ctx.error_flag,
+                                  label="gate_up" if self.gated else "up", act=0 if self.gated else ops.ACT_RELU_SQUARED)
+            ops.gemm_pair_grouped(STORE, act, self.w_down, y, tiles, n_tiles, max_tiles, pairs,
+                                  (shared_act, self.w_shared_down, shared_y) if self.shared else None, error_flag=ctx.error_flag,
+                                  label="down")
+        elif self.grouped:
             if self.gated:
                 ops.gemm_tc_grouped(SWIGLU, sorted_x, self.w_gate_up, act, tile_rows, tiles, n_tiles, max_tiles, pairs,
                                     error_flag=ctx.error_flag, label="gate_up")
@@ -173,9 +190,7 @@ class ExpertMixture(FeedForward):
             ops.moe_gemm(1 if self.gated else 2, x, order, top, self.w_gate_up, act, tiles, n_tiles, max_tiles,
                          label="gate_up" if self.gated else "up")
             ops.moe_gemm(0, act, None, top, self.w_down, y, tiles, n_tiles, max_tiles, label="down")
-        shared_y = None
-        if self.shared:
-            shared_act = ctx.buffer("moe.shared_act", (n, self.ffs), dtype)
+        if self.shared and not on_pairs:
             if self.gated:
                 linear(rt, SWIGLU, x, self.w_shared_gate_up, shared_act, error_flag=ctx.error_flag, name="shared_gate_up")
             else:
@@ -183,7 +198,6 @@ class ExpertMixture(FeedForward):
                 if not linear(rt, STORE, x, self.w_shared_gate_up, shared_act, error_flag=ctx.error_flag, name="shared_up",
                               activation=ops.ACT_RELU_SQUARED, unactivated=shared_up):
                     ops.activation_rows(shared_up, shared_act, ops.ACT_RELU_SQUARED)
-            shared_y = ctx.buffer("moe.shared_y", (n, self.hidden), torch.float32)
             linear(rt, STORE, shared_act, self.w_shared_down, shared_y, error_flag=ctx.error_flag, name="shared_down")
         ops.moe_combine(residual, y, inverse, weights, shared_y, shared_gate, top, scale, store,
                         x=x if self.identity else None)
