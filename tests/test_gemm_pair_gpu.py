@@ -36,7 +36,7 @@ def test_tiles_of_every_width(M, N, K, dtype):
             product(M, N, K, mode, dtype, lambda mode, a, w, out, alpha, flag: ops.gemm_pair(mode, a, w, out, alpha, n, flag), pad=8)
 
 
-@pytest.mark.parametrize("M,N,K", [(160, 2048, 2048), (256, 6144, 256), (2048, 8192, 128), (4096, 1600, 64)])
+@pytest.mark.parametrize("M,N,K", [(64, 1000, 512), (128, 2048, 320), (160, 2048, 2048), (256, 6144, 256), (2048, 8192, 128), (4096, 1600, 64)])
 def test_products_that_go_there_by_themselves(M, N, K):
     from lia_rs_b200.kernels import ops
     for mode, dtype in ((ops.GEMM_STORE, torch.float32), (ops.GEMM_ACCUM, torch.float32), (ops.GEMM_SWIGLU, torch.bfloat16)):
