@@ -88,6 +88,137 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pages,
         if (c < chunks && i < d) orow[i] = from_float<T>(acc[c] * inv);
     }
 }
+// The same numbers for few (token, query head) items of 32-bit elements (the bits are the kernel's above): a CTA an item, ROW_KEYS keys at a
+// time, a warp a chunk of 32 of them.  What depends on nothing but a chunk's own keys, and on the maxima of the chunks before it, which
+// do not depend on any sum, is done side by side: scores, maxima, exponentials, the chunks' sums; the values come by asynchronous copies
+// meanwhile.  What is a chain, the sums over all keys in order, is left to a thread an element, from shared memory.
+// The kernel above has a warp walk the chunks one behind the other, several dependent trips to memory and 32 steps of the output each.  What
+// bounds this one is a tile's trips (its page numbers, then keys and values together) and the chain of the sums.  us, a warp / a CTA an
+// item, 16 query and 2 kv heads: of 64 elements, 3 tokens behind 150, 600 and 2,000 keys 60/10, 227/25, 749/74; 64 tokens behind 600 308/94; of
+// 128 elements, 3 tokens behind 600 312/34.
+constexpr int ROW_KEYS = 128;
+
+__global__ void __launch_bounds__(ROW_KEYS)
+attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
+                      const int* __restrict__ positions, const int* __restrict__ slots, const int* __restrict__ block_table,
+                      int table_stride, const int* __restrict__ rows, float* __restrict__ out, int nq, int nkv, int d, int page_size,
+                      int window, float scale, int num_pages, int* __restrict__ error_flag) {
+    extern __shared__ __align__(16) float values[];          // [ROW_KEYS][d]
+    __shared__ __align__(16) float q_shared[MAX_D], weights[ROW_KEYS];
+    __shared__ float chunk_max[ROW_KEYS / 32], chunk_sum[ROW_KEYS / 32], chunk_correction[ROW_KEYS / 32];
+    __shared__ int key_rows[ROW_KEYS];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = rows ? rows[blockIdx.x / nq] : (int)(blockIdx.x / nq), h = blockIdx.x % nq;
+    if (t < 0) return;
+    const int slot = slots[t];
+    if (slot < 0) return;
+    const int pos = positions[t], kvh = h / (nq / nkv), tid = threadIdx.x, warp = tid >> 5;
+    const float* qrow = q + ((size_t)t * nq + h) * d;
+    for (int i = tid; i < d; i += ROW_KEYS) q_shared[i] = qrow[i];
+    const int* table = block_table + (size_t)slot * table_stride;
+    const int first = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+    const int pieces = d / 4;
+    float acc[MAX_D / ROW_KEYS] = {};
+    float running_max = -INFINITY, running_sum = 0.f;
+    for (int base = first; base <= pos; base += ROW_KEYS) {
+        const int chunks = min(ROW_KEYS / 32, (pos - base) / 32 + 1);
+        const int j = base + tid;
+        bool valid = j <= pos;
+        int row = 0;
+        float score = -INFINITY;
+        if (valid) {
+            row = cache_row_of(table, j, page_size, -1, num_pages, error_flag);
+            valid = row >= 0;                                // a key without a page counts for nothing (and the flag is up)
+            row = valid ? row : 0;
+        }
+        key_rows[tid] = row;
+        __syncthreads();                                     // (and everyone is done with the tile before)
+        const int there = min(ROW_KEYS, pos - base + 1);
+        for (int e = tid; e < there * pieces; e += ROW_KEYS) {
+            const int r = e / pieces, c = (e - r * pieces) * 4;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(values + r * d + c)),
+                         "l"(v_pages + ((size_t)key_rows[r] * nkv + kvh) * d + c) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (valid) {
+            const float4* krow = reinterpret_cast<const float4*>(k_pages + ((size_t)row * nkv + kvh) * d);
+            float dot = 0.f;
+            for (int i = 0; i < pieces; i += 4) {            // (d is a multiple of 16)
+                float4 k[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) k[x] = krow[i + x];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const float4 w = *reinterpret_cast<const float4*>(q_shared + 4 * (i + x));
+                    dot = fmaf(w.x, k[x].x, dot);
+                    dot = fmaf(w.y, k[x].y, dot);
+                    dot = fmaf(w.z, k[x].z, dot);
+                    dot = fmaf(w.w, k[x].w, dot);
+                }
+            }
+            score = dot * scale;
+        }
+        const float own_max = warp_max(score);
+        if ((tid & 31) == 0) chunk_max[warp] = own_max;
+        __syncthreads();
+        for (int c = 0; c < warp; ++c) running_max = fmaxf(running_max, chunk_max[c]);
+        const float new_max = fmaxf(running_max, own_max);
+        const float correction = expf(running_max - new_max);
+        const float p = valid ? expf(score - new_max) : 0.f;
+        const float sum = warp_sum(p);
+        weights[tid] = p;
+        if ((tid & 31) == 0) {
+            chunk_sum[warp] = sum;
+            chunk_correction[warp] = correction;
+        }
+        running_max = new_max;
+        for (int c = warp + 1; c < chunks; ++c) running_max = fmaxf(running_max, chunk_max[c]);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        for (int c = 0; c < chunks; ++c) {
+            const float factor = chunk_correction[c];
+            running_sum = running_sum * factor + chunk_sum[c];
+#pragma unroll
+            for (int x = 0; x < MAX_D / ROW_KEYS; ++x) acc[x] *= factor;
+            const int count = min(32, there - 32 * c);
+#pragma unroll
+            for (int x = 0; x < MAX_D / ROW_KEYS; ++x) {
+                const int i = tid + x * ROW_KEYS;
+                if (i >= d) break;
+                const float* column = values + (size_t)32 * c * d + i;
+                const float* w = weights + 32 * c;
+#pragma unroll 8
+                for (int jj = 0; jj < count; ++jj) acc[x] = fmaf(w[jj], column[(size_t)jj * d], acc[x]);
+            }
+        }
+    }
+    const float inv = 1.0f / running_sum;
+    float* orow = out + ((size_t)t * nq + h) * d;
+#pragma unroll
+    for (int x = 0; x < MAX_D / ROW_KEYS; ++x)
+        if (tid + x * ROW_KEYS < d) orow[tid + x * ROW_KEYS] = acc[x] * inv;
+}
+
+// (token, query head) items up to which a CTA each is faster than a warp each, however few keys they see: a CTA keeps a tile's values in shared
+// memory, of which an SM holds one of 256 elements.  us behind 20 keys, a warp / a CTA: 256 elements 256 items 21.0/15.3, 512 20.9/27.0; 128
+// elements 1,024 items 19.2/15.5, 2,048 28.7/24.9, 4,096 44.7/46.8; 64 elements 4,096 27.0/21.0.
+long long rows_up_to(int d) { return d <= 128 ? 2048 : 256; }
+
+int launch_rows(const float* q, const float* k_pages, const float* v_pages, const int* positions, const int* slots, const int* block_table,
+                int table_stride, const int* rows, float* out, unsigned items, int nq, int nkv, int d, int page_size, int window, float scale,
+                int num_pages, int* error_flag, cudaStream_t stream) {
+    static std::atomic<bool> configured{false};
+    if (!configured.load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(attention_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROW_KEYS * MAX_D * (int)sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            return LIA_ERR_LAUNCH;
+        }
+        configured.store(true, std::memory_order_release);
+    }
+    return lia_launch(attention_rows_kernel, dim3(items), dim3(ROW_KEYS), (size_t)ROW_KEYS * d * sizeof(float), stream, q, k_pages, v_pages,
+                      positions, slots, block_table, table_stride, rows, out, nq, nkv, d, page_size, window, scale, num_pages, error_flag);
+}
 }  // namespace
 
 // q, out [tokens, nq, d]; k_pages, v_pages [num_pages, page_size, nkv, d]; all of `dtype`.
@@ -104,6 +235,9 @@ LIA_EXPORT int lia_attention_generic(const void* q, const void* k_pages, const v
     const long long items = (long long)n_tokens * nq;
     const long long blocks = (items + WARPS - 1) / WARPS;
     if (blocks > 2147483647LL) return LIA_ERR_SIZE;
+    if (dtype == LIA_F32 && items <= rows_up_to(d) && (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15u) == 0)
+        return launch_rows((const float*)q, (const float*)k_pages, (const float*)v_pages, positions, slots, block_table, table_stride, rows,
+                           (float*)out, (unsigned)items, nq, nkv, d, page_size, window, scale, num_pages, error_flag, stream);
     if (dtype == LIA_F32)
         attention_generic_kernel<float><<<(unsigned)blocks, WARPS * 32, 0, stream>>>(
             (const float*)q, (const float*)k_pages, (const float*)v_pages, positions, slots, block_table,
