@@ -503,13 +503,13 @@ def gemm_pair(mode, a, w, out, alpha: float = 1.0, n_tile: int = 0, error_flag=N
                                alpha, sms, int(n_tile), _p(error_flag), _stream()), "gemm_pair")
 
 
-def gemm_cluster_accepts(mode, a, w, out) -> bool:
+def gemm_cluster_accepts(mode, a, w, out, least: int = 2) -> bool:
     """Whether the cluster kernel takes this product: what the tcgen05 kernel takes, and so few output
-    tiles that at least two CTAs of a cluster can share each one's K."""
+    tiles that at least two CTAs (or `least`) of a cluster can share each one's K."""
     if not gemm_tc_accepts(mode, a, w, out):
         return False
     _, sms = _device_scratch(a.device)
-    return lib().lia_gemm_cluster_splits(mode, a.shape[0], out.shape[1], a.shape[1], sms) >= 2
+    return lib().lia_gemm_cluster_splits(mode, a.shape[0], out.shape[1], a.shape[1], sms) >= max(2, least)
 
 
 def gemm_cluster(mode, a, w, out, alpha: float = 1.0, error_flag=None, label=None):

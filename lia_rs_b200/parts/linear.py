@@ -14,7 +14,7 @@
   streams the weights once with one CTA per 16 rows (csrc/gemm_skinny.cu); beyond 16 tokens, the tcgen05 kernel that cuts K over a cluster (csrc/gemm_cluster.cu)
   while it applies (16 tokens of a 2B-class layer: 58 us with the few-token kernel, 63 us with the cluster
   kernel; 24 tokens: 82 against 66; 32 tokens: 91 against 70: every CTA of the few-token kernel reads all the
-  tokens' rows from L2) and up to 256 tokens (see `_cluster_tokens`); then the persistent tcgen05 kernels, which cut K through scratch
+  tokens' rows from L2) and up to 256 tokens, or where few tiles of a long K leave the SMs idle (see `_few_tiles`); then the persistent tcgen05 kernels, which cut K through scratch
   memory up to 128 tokens and beyond that cuts the tokens into tiles as narrow as fills the SMs (a 2B-class
   layer's four products at 512 tokens: 90 us, at 256 tokens 70 us with the cluster kernel for three of them);
 * what TMA cannot address goes to the few-token kernel if it can take it, else, and always for the 32-bit
@@ -36,12 +36,18 @@ def prepare_weight(weight: torch.Tensor, runtime) -> torch.Tensor:
 SKINNY_BEST_TOKENS = 16
 
 
-def _cluster_tokens(mode, K: int) -> int:
-    """Most tokens that the cluster kernel takes; beyond, the tiles of the persistent kernels (gemm_tc, which goes to pairs of SMs by itself)
-    are as fast or faster.  us, cluster kernel / those: gated products 6,144 x 2,048 at 48, 64, 128 tokens 14.5/13.3, 15.1/13.4, 18.4/13.7;
-    4,096 x 1,024 8.5/9.1, 9.3/8.0, 12.1/8.4; plain ones 2,048 x 2,048 at 256 tokens 9.4/9.9, 2,048 x 6,144 15.5/20.3; with short K 1,280 x 1,024
-    at 160, 192, 256 tokens 6.5/6.6, 6.9/6.7, 7.8/6.7, 3,072 x 1,024 6.7/6.9, 7.0/7.0, 7.9/7.2."""
-    return 63 if mode == SWIGLU else 256 if K > 1024 else 192
+def _few_tiles(mode, a, w, out) -> bool:
+    """Whether the cluster kernel is for this product: few tokens, or few output tiles and a long K, which four CTAs and more then share.
+    Beyond, the tiles of the persistent kernels (gemm_tc, which goes to pairs of SMs by itself) are as fast or faster.
+    us, cluster kernel / those: gated products 6,144 x 2,048 at 48, 64, 128 tokens 14.5/13.3, 15.1/13.4, 18.4/13.7; 4,096 x 1,024 8.5/9.1,
+    9.3/8.0, 12.1/8.4; plain ones 2,048 x 2,048 at 256 tokens 9.4/9.9, 2,048 x 6,144 15.5/20.3; with short K 1,280 x 1,024 at 160, 192, 256 tokens
+    6.5/6.6, 6.9/6.7, 7.8/6.7, 3,072 x 1,024 6.7/6.9, 7.0/7.0, 7.9/7.2.  Few tiles, with the CTAs that share one: 160 x 4,096 at 512 tokens (8) 7.8/14.2,
+    2,048 (4) 11.5/14.5; 512 x 2,048 at 1,024 (4) 9.1/9.5, 1,500 (2) 10.9/9.6; 1,024 x 4,096 at 512 (4) 12.2/14.8, 768 (2) 17.0/15.1; 256 x 1,024 at 512
+    (8) 7.0/6.9."""
+    tokens, K = a.shape
+    if tokens <= (63 if mode == SWIGLU else 256 if K > 1024 else 192):
+        return ops.gemm_cluster_accepts(mode, a, w, out)
+    return mode != SWIGLU and K > 1024 and ops.gemm_cluster_accepts(mode, a, w, out, least=4)
 
 
 _TC, _SKINNY, _CLUSTER, _SIMT, _STREAM = range(5)
@@ -62,7 +68,7 @@ def _choose(mode, a, w, out) -> int:
         return _TC
     if few and a.shape[0] <= SKINNY_BEST_TOKENS:
         return _SKINNY
-    if tensor_cores and a.shape[0] <= _cluster_tokens(mode, w.shape[1]) and ops.gemm_cluster_accepts(mode, a, w, out):
+    if tensor_cores and _few_tiles(mode, a, w, out):
         return _CLUSTER
     if tensor_cores:
         return _TC
