@@ -9,7 +9,7 @@
 `shared` (optional) is one more expert of a size of its own that every token uses, times a gate of one number per token.
 The router's product, the softmax, the choice and the weights are 32-bit; the (token, choice) pairs are grouped by expert
 on the device, each expert's rows go through its two products in tiles (bfloat16: the grouped product on the tensor
-cores, csrc/gemm_tc.cu, over rows padded to whole tiles per expert; 32-bit, and sizes that TMA cannot address: the
+cores, csrc/gemm_tc.cu over rows padded to whole tiles per expert or csrc/gemm_pair.cu over rows padded to 32; 32-bit, and sizes that TMA cannot address: the
 product on the 32-bit pipes), and one kernel adds a token's weighted rows, in the order of its choices, into the
 residual stream (csrc/moe.cu).  Nothing is decided on the host, so a step's launches
 depend on its number of tokens alone, and a token's result does not depend on what else is in the batch.
