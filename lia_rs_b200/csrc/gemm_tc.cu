@@ -529,12 +529,11 @@ LIA_EXPORT int lia_gemm_tc(int mode, const void* X, int ldx, const void* W, int 
     // products of several rounds or wide tiles (us, one CTA a tile / pairs: 2,048 x 8,192 x 2,048 72 / 51, 4,096 x 2,048 x 6,144 110 / 76, 256 x 2,048 pairs x
     // 2,048 14.1 / 9.5), and not where tiles of one CTA make one full round (2,048 x 2,048 x 6,144 36.1 / 38.9, 1,111 x 3,088 x 1,024 9.8 / 11.0).
     const int out_bytes = out_dtype == LIA_F32 ? 4 : 2;
-    // Gated products go there from 64 tokens where K would be cut (64 tokens, 4,096 pairs x 1,024 26.7 / 8.0; the cluster kernel 9.3).
-    const bool cut = plan.splits > 1;
-    if ((M > 128 || (swiglu && M >= 64 && cut)) && sm_count >= 2 && ((uintptr_t)out & 15u) == 0 && ((long long)ldo * out_bytes) % 16 == 0) {
+    // (up to 128 tokens K is cut and the ranges are added up with rounding: pairs have one accumulator for all of K, which is cut off at every step)
+    if (M > 128 && sm_count >= 2 && ((uintptr_t)out & 15u) == 0 && ((long long)ldo * out_bytes) % 16 == 0) {
         const long long rounds = ((long long)plan.f_tiles * plan.t_tiles + sm_count - 1) / sm_count;
         const double alone = 0.8 + rounds * round_cost(swiglu, plan.n_tile, (K + BLOCK_K - 1) / BLOCK_K) + 0.14e-6 * out_bytes * M * N;
-        if (cut || gemm_pair_estimate(mode, M, N, K, out_bytes, sm_count) < 0.95 * alone) {
+        if (gemm_pair_estimate(mode, M, N, K, out_bytes, sm_count) < 0.95 * alone) {
             const int form = act == 5 ? GEMM_STORE_XIELU : act == 3 ? GEMM_STORE_RELU2 : act == 4 ? GEMM_REGLU : mode;
             return gemm_pair_launch(form, X, ldx, W, ldw, out, out_dtype, ldo, M, N, K, alpha, sm_count, 0, act_p, act_n, error_flag, stream);
         }

@@ -34,18 +34,21 @@ def prepare_weight(weight: torch.Tensor, runtime) -> torch.Tensor:
 
 
 SKINNY_BEST_TOKENS = 16
+CLUSTER_MAX_TOKENS = 256
 
 
 def _few_tiles(mode, a, w, out) -> bool:
     """Whether the cluster kernel is for this product: few tokens, or few output tiles and a long K, which four CTAs and more then share.
-    Beyond, the tiles of the persistent kernels (gemm_tc, which goes to pairs of SMs by itself) are as fast or faster.
-    us, cluster kernel / those: gated products 6,144 x 2,048 at 48, 64, 128 tokens 14.5/13.3, 15.1/13.4, 18.4/13.7; 4,096 x 1,024 8.5/9.1,
-    9.3/8.0, 12.1/8.4; plain ones 2,048 x 2,048 at 256 tokens 9.4/9.9, 2,048 x 6,144 15.5/20.3; with short K 1,280 x 1,024 at 160, 192, 256 tokens
-    6.5/6.6, 6.9/6.7, 7.8/6.7, 3,072 x 1,024 6.7/6.9, 7.0/7.0, 7.9/7.2.  Few tiles, with the CTAs that share one: 160 x 4,096 at 512 tokens (8) 7.8/14.2,
+    Up to 256 tokens because of the sums: it adds up eight ranges of K with rounding, each in accumulators of its own, where the tiles of the
+    persistent kernels have one accumulator for all of K, which the tensor cores cut off (not round) at every step.  Relative error of 32-bit
+    outputs against 64 bits, cluster kernel / those, 64 tokens x 2,048 features: K 512 7.0e-8/4.7e-7, 2,048 1.1e-7/2.1e-6, 6,144 2.4e-7/6.8e-6; the
+    time does not decide it (us, 6,144 gated pairs x 2,048 at 48, 64, 128 tokens 14.5/13.3, 15.1/13.4, 18.4/13.7; plain 2,048 x 2,048 at 256
+    9.4/9.9, 2,048 x 6,144 15.5/20.3; 1,280 x 1,024 at 160, 192, 256 tokens 6.5/6.6, 6.9/6.7, 7.8/6.7).
+    Beyond 256 tokens it is the time: few tiles, with the CTAs that share one, us: 160 x 4,096 at 512 tokens (8) 7.8/14.2,
     2,048 (4) 11.5/14.5; 512 x 2,048 at 1,024 (4) 9.1/9.5, 1,500 (2) 10.9/9.6; 1,024 x 4,096 at 512 (4) 12.2/14.8, 768 (2) 17.0/15.1; 256 x 1,024 at 512
     (8) 7.0/6.9."""
     tokens, K = a.shape
-    if tokens <= (63 if mode == SWIGLU else 256 if K > 1024 else 192):
+    if tokens <= CLUSTER_MAX_TOKENS:
         return ops.gemm_cluster_accepts(mode, a, w, out)
     return mode != SWIGLU and K > 1024 and ops.gemm_cluster_accepts(mode, a, w, out, least=4)
 
