@@ -45,3 +45,32 @@ def test_grouped_and_plain_product_in_one_launch(rows, shared, N, K, N2, K2):
             want = form(x2.double() @ w2.double().T, N2)
             assert float((out2.double() - want).abs().max()) <= limit(want)
     assert int(flag) == 0
+
+
+@pytest.mark.parametrize("n", [16, 64, 256, 257])
+def test_a_shared_experts_sums_are_those_of_its_products_alone(n):
+    """Up to 256 tokens the cluster kernel's (or the few-token kernel's), more exact than a pair's one accumulator; beyond, one accumulator either way."""
+    from lia_rs_b200.cache import CacheManager
+    from lia_rs_b200.engine import StepEntry, StepRuntime
+    from lia_rs_b200.kernels import ops
+    from lia_rs_b200.parts import FEED_FORWARDS, Runtime, linear as lin
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *shape: (torch.randn(*shape, device="cuda", generator=g) * shape[-1] ** -0.5).to(torch.bfloat16)
+    h, ff, ffs, experts = 1024, 64, 2048, 4
+    tensors = {"L.router": rnd(experts, h), "L.shared.gate": rnd(ffs, h), "L.shared.up": rnd(ffs, h), "L.shared.down": rnd(h, ffs)}
+    for e in range(experts):                                                 # the routed experts add nothing
+        tensors.update({f"L.e{e}.gate": rnd(ff, h), f"L.e{e}.up": rnd(ff, h), f"L.e{e}.down": torch.zeros(h, ff, device="cuda", dtype=torch.bfloat16)})
+    runtime = Runtime("cuda:0", torch.bfloat16)
+    part = FEED_FORWARDS["expert_mixture"](dict(hidden=h, experts=experts, top=2, intermediate=ff, shared={"intermediate": ffs}, shared_gated=False),
+                                           tensors, "L.", runtime)
+    cache = CacheManager({}, {}, 32, 16, 1, 512, torch.bfloat16, "cuda:0")
+    steps, slot = StepRuntime(cache, 1000, 512, "cuda:0"), cache.admit()
+    assert cache.ensure(slot, 0, n) and ops.moe_pair_tile_rows(2 * n, experts) != (0, 0)
+    x = (rnd(n, h).float() * h ** 0.5).to(torch.bfloat16)
+    out, act, want = torch.zeros(n, h, device="cuda"), torch.empty(n, ffs, device="cuda", dtype=torch.bfloat16), torch.zeros(n, h, device="cuda")
+    part.forward(steps.begin([StepEntry(slot, [1] * n, 0, [])]), x, out, 1.0, store=True)
+    steps.finish()
+    alone = (lambda *product: lin.linear(runtime, *product)) if n <= 256 else ops.gemm_pair
+    alone(lin.SWIGLU, x, part.w_shared_gate_up, act)
+    alone(lin.STORE, act, part.w_shared_down, want)
+    assert torch.equal(out, want)
