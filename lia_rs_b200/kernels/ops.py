@@ -1616,13 +1616,20 @@ def gemm_tc_grouped(mode, a, w, out, tile_rows: int, tiles, n_tiles, max_tiles: 
                                          _p(error_flag), _stream()), "gemm_tc_grouped")
 
 
-def moe_pair_tile_rows(pairs: int, experts: int) -> tuple:
+def moe_pair_tile_rows(pairs: int, experts: int, shared: bool = False) -> tuple:
     """(rows of a token tile, rows that every expert's begin at a multiple of) of the product over the experts on pairs of SMs
-    (csrc/gemm_pair.cu), which takes the shared expert's product into the same launch; (0, 0) where there are few rows an expert, which the
-    one-CTA product (`gemm_tc_grouped`) is for: a tile is 256 rows of the MMA however few an expert has, which many small experts feel
-    first.  us of the whole part, one CTA / pairs: 8 experts of 2,048 and a shared one, hidden 2,048, two chosen, 8 tokens 59.7/60.4, 16 tokens
-    65.8/62.0, 64 80/63, 512 102/77, 2,048 188/174; 64 experts of 512, six chosen, 43 tokens 112/121, 128 126/125, 512 154/152, 2,048 289/264."""
-    return (PAIR_ROWS, PAIR_STORE_ROWS) if pairs >= min(12, max(4, experts / 5)) * experts else (0, 0)
+    (csrc/gemm_pair.cu); (0, 0) where the one-CTA product (`gemm_tc_grouped`) is for them.  `shared`: a shared expert's products would go into
+    the same launches.  Then pairs: two launches less are worth more than what follows costs (1,218 times of whole parts on a B200; pairs / one CTA, by
+    rows an expert: 8 experts of 2,048, hidden 2,048, 65 rows 0.85, 128 0.74, 512 0.87; 16 of 1,024, hidden 1,024, 32 to 300 0.73 to 0.89; 32 of 1,024 0.84 to 0.94;
+    64 of 512 0.89 to 0.99, of 1,408 24 to 60 1.00 to 1.03, 144 0.89; 128 of 768 16 to 140 0.93 to 1.02).
+    Without: pairs from 128 rows an expert (8 experts of 4,096 0.98, 160 rows 0.85; 64 of 1,024 0.93; 128 of 768 0.97), of which a one-CTA tile holds no
+    more and reads W again for the rest.  Below, a pair's tile is 256 rows of the MMA however few an expert has: 8 experts of 4,096, hidden 4,096, 11 to 13,
+    22 to 27, 45 to 54, 90 to 115 rows 1.04 to 1.14; 32 of 1,024 1.01 to 1.15; 128 of 256 1.10 to 1.15.  But where the rows an expert all but fill the one-CTA
+    tile, chance gives about every other expert a second one; among up to eight experts that is what the product waits for: 15 to 16, 30 to 32, 61 to 64
+    rows, 4 experts of 8,192 0.88 to 0.92, 8 of 2,048 0.87 to 0.98, of 4,096 0.95 to 0.99, of 14,336 0.90 to 0.95 (of 1,024, which L2 holds, 0.99 to 1.03);
+    16 of 4,096 1.01 to 1.04, 32 of 1,024 0.95 to 1.03, 128 of 256 1.10."""
+    filled = experts <= 8 and 16 * pairs >= 15 * moe_grouped_tile_rows(pairs, experts) * experts
+    return (PAIR_ROWS, PAIR_STORE_ROWS) if shared or filled or pairs >= 128 * experts else (0, 0)
 
 
 def gemm_pair_grouped(mode, a, w, out, tiles, n_tiles, max_tiles: int, pairs: int, shared=None, error_flag=None, label=None, act: int = 0):

@@ -145,11 +145,11 @@ class ExpertMixture(FeedForward):
                       groups=self.groups, keep=self.keep, renormalise=self.renormalise, sigmoid=self.sigmoid, two_best=self.two_best)
         if self.grouped is None:
             self.grouped = ops.moe_grouped_accepts(x, self.w_gate_up, self.w_down)
-        tile_rows, pad = ops.moe_pair_tile_rows(pairs, experts) if self.grouped and self.shared_fits else (0, 0)
-        on_pairs = tile_rows > 0
         # pairs of SMs take the shared expert's products into the same launches, but for the few tokens whose sums the cluster kernel forms more
         # exactly: relative error of its 32-bit outputs at 64 tokens, K 2,048, 1.1e-7, of a pair's one accumulator 2.1e-6
-        together = on_pairs and self.shared and n > CLUSTER_MAX_TOKENS
+        together = self.grouped and self.shared and self.shared_fits and n > CLUSTER_MAX_TOKENS
+        tile_rows, pad = ops.moe_pair_tile_rows(pairs, experts, together) if self.grouped else (0, 0)
+        on_pairs = tile_rows > 0
         if self.grouped:
             # the tensor cores: every expert's rows begin at a multiple of what a tile stores at once, the rows' inputs are laid side by side
             if not on_pairs:
