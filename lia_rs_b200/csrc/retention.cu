@@ -7,8 +7,8 @@
 //  * `retention_encode` rotates q and k in place (element i of a head with i + rot_dims/2 over the first rot_dims
 //    elements, angle float(position) * freq[i]) and multiplies k by d^(-1/2) after the rotation.
 //  * Single tokens (`retention_single`): one CTA per (token, head) updates the state in place and forms o from it.
-//  * Prompt portions are cut into chunks of CHUNK tokens (LONG for heads of 64 or 128 elements; on the tensor cores, retention_tc.cu, 128) that run
-//    side by side, in three launches:
+//  * Prompt portions are cut into chunks of CHUNK tokens (LONG for heads of 64 or 128 elements) that run side by side, in three
+//    launches:
 //      sums    U_c = sum_j decay^(len-1-j) k_j v_j^T of each chunk, from zero;
 //      carry   along each portion: the state that each chunk starts from takes U_c's place in scratch,
 //              S <- decay^len S + U_c, and the last S goes back to the request's state;
@@ -19,7 +19,6 @@
 // slot is negative belongs to nobody and is skipped.
 #include "common.cuh"
 #include "linear_recurrence.cuh"
-#include "retention_tc.cuh"
 
 namespace {
 constexpr int RET_THREADS = 256;
@@ -178,7 +177,7 @@ retention_sums_kernel(const float* __restrict__ rows, long long ld, const float*
     }
 }
 
-// along each portion: scratch[c] <- the state chunk c starts from; S <- decay^len S + U_c; state <- the last S.
+// along each portion: scratch[c] <- the state chunk c starts from; S <- decay^len S + U_c; state <- the last S
 template <int LENGTH>
 __global__ void __launch_bounds__(RET_THREADS)
 retention_carry_kernel(const float* __restrict__ decay, const int* __restrict__ segments, int n_segments,
@@ -629,7 +628,7 @@ LIA_EXPORT int lia_retention_encode(float* rows, long long ld, const float* freq
 LIA_EXPORT int lia_retention(const float* rows, long long ld, const float* decay, float* state, long long state_stride,
                              const int* segments, int n_segments, int max_chunks, const int* single_rows, int n_single,
                              const int* slots, void* out, int out_dtype, int heads, int d, int dv, float eps,
-                             float* scratch, long long scratch_floats, int* error_flag, cudaStream_t stream) {
+                             float* scratch, long long scratch_floats, cudaStream_t stream) {
     if (heads <= 0 || d <= 0 || dv <= 0 || d > RET_MAX || dv > RET_MAX || ld < (long long)2 * heads * (d + dv) ||
         state_stride < (long long)heads * d * dv)
         return LIA_ERR_SIZE;
@@ -643,21 +642,7 @@ LIA_EXPORT int lia_retention(const float* rows, long long ld, const float* decay
         // heads of 64 or 128 elements: longer chunks, of which there are no more than the caller made room for
         const bool tiled = vec && (d == 64 || d == 128) && (dv == 64 || dv == 128) &&
                            ((uintptr_t)out & (out_dtype == LIA_F32 ? 15u : 7u)) == 0;
-        // bfloat16 outputs, 32 tokens a portion on average (2 tokens of 16 heads of 64 x 64 are 13.2 us there, 11.5 here), and 1,024 heads x tokens:
-        // the tensor cores.  They are faster with fewer too (3 heads of 128 x 64, 129 tokens 20 us, 29 here); but a step of a few rows
-        // keeps outputs that are the 32-bit path's rounded, bit for bit, which is what the tests of these kernels hold on to.
-        const long long covered = (long long)(max_chunks - n_segments) * CHUNK;
-        if (tiled && out_dtype == LIA_BF16 && max_chunks >= 2 * n_segments && covered * heads >= 1024) {
-            // (at most as many chunks of 128 tokens as follow from the most chunks of 32)
-            const int chunks = (int)((covered + CHUNK - 1) / RETENTION_TC_CHUNK) + n_segments;
-            code = retention_tc_sums(rows, ld, decay, segments, n_segments, chunks, scratch, heads, d, dv, error_flag, stream);
-            if (code != LIA_OK) return code;
-            code = lia_launch(retention_carry_kernel<RETENTION_TC_CHUNK>, dim3(n_segments, heads, d * dv / RET_THREADS), dim3(RET_THREADS), 0,
-                              stream, decay, segments, n_segments, slots, scratch, state, state_stride, heads, d, dv);
-            if (code != LIA_OK) return code;
-            code = retention_tc_output(rows, ld, decay, segments, n_segments, chunks, scratch, out, heads, d, dv, eps, error_flag, stream);
-            if (code != LIA_OK) return code;
-        } else if (tiled) {
+        if (tiled) {
 #define LIA_TILES(TO, D, DV)                                                                                                  \
     launch_tiles<TO, D, DV>(rows, ld, decay, state, state_stride, segments, n_segments, max_chunks, slots, (TO*)out, heads, eps, scratch, stream)
 #define LIA_TILES_OF(TO)                                                                                                      \

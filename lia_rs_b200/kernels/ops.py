@@ -210,7 +210,7 @@ class _Signatures:
     lia_retention_encode = [c_void_p, ctypes.c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float,
                             c_void_p]
     lia_retention = [c_void_p, ctypes.c_longlong, c_void_p, c_void_p, ctypes.c_longlong, c_void_p, c_int, c_int, c_void_p,
-                     c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, ctypes.c_longlong, c_void_p, c_void_p]
+                     c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, ctypes.c_longlong, c_void_p]
     lia_gemm_mma_batched = [c_void_p, ctypes.c_longlong, ctypes.c_longlong, c_void_p, ctypes.c_longlong, ctypes.c_longlong, c_void_p, ctypes.c_longlong, ctypes.c_longlong, c_int, c_int, c_int, c_int, c_void_p]
 
 def dtype_code(dtype: torch.dtype) -> int:
@@ -1698,11 +1698,10 @@ def retention_encode(rows, freq, rot_dims: int, positions, slots, heads: int, d:
 
 
 def retention(rows, decay, state, segments, n_segments: int, max_chunks: int, single_rows, slots, out, heads: int, d: int,
-              dv: int, eps: float, scratch=None, error_flag=None):
+              dv: int, eps: float, scratch=None):
     """S <- decay_h S + k v^T, o = S^T q, out = o / rms(o) * silu(g) along the step's runs; rows [n, 2 heads (d + dv)]
-    32-bit = [q | k | v | g] as `retention_encode` left them, state [slots, heads, d, dv] 32-bit.  Portions with bfloat16 outputs and heads
-    of 64 or 128 elements run on the tensor cores (csrc/retention_tc.cu), which raise `error_flag` to 3 if a wait gives up."""
-    _cuda(decay, segments, single_rows, slots, out, scratch, error_flag)
+    32-bit = [q | k | v | g] as `retention_encode` left them, state [slots, heads, d, dv] 32-bit."""
+    _cuda(decay, segments, single_rows, slots, out, scratch)
     _f32(rows, decay, state, scratch)
     n_single = 0 if single_rows is None else single_rows.numel()
     if rows.stride(1) != 1 or rows.shape[1] < 2 * heads * (d + dv) or tuple(out.shape) != (rows.shape[0], heads * dv) or \
@@ -1712,7 +1711,7 @@ def retention(rows, decay, state, segments, n_segments: int, max_chunks: int, si
         _check(lib().lia_retention(_p(rows), rows.stride(0), _p(decay), _p(state), state.stride(0), _p(segments),
                                    int(n_segments), int(max_chunks), _p(single_rows), n_single, _p(slots), _p(out),
                                    dtype_code(out.dtype), heads, d, dv, float(eps), _p(scratch),
-                                   0 if scratch is None else scratch.numel(), _p(error_flag), _stream()), "retention")
+                                   0 if scratch is None else scratch.numel(), _stream()), "retention")
 
 
 # ---- gated linear attention (a linear recurrence with a decay per token and key channel): csrc/gated_linear_attention.cu ----

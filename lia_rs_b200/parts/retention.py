@@ -95,5 +95,5 @@ class Retention(Mixer):
                                       torch.float32) if chunks else None
         o = ctx.buffer("retention.o", (n, heads * dv), rt.compute_dtype)
         ops.retention(rows, self.decay, state, ctx.prefill_segments, portions, chunks, ctx.decode_rows, ctx.slots, o,
-                      heads, d, dv, self.eps, scratch=scratch, error_flag=flag)
+                      heads, d, dv, self.eps, scratch=scratch)
         linear(rt, STORE if store else ACCUM, o, self.w_o, residual, scale, error_flag=flag, name="o")
