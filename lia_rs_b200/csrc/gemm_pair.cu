@@ -44,7 +44,8 @@ constexpr int SMEM_BYTES = 226 * 1024;           // dynamic shared memory asked 
 constexpr int PAIR_M = 256, HALF_M = 128;        // tokens per tile, and per CTA
 constexpr int CHUNK_F = 32;                      // features of an epilogue piece
 constexpr int RASTER = 8;                        // token tiles that neighbouring pairs share the rows of W of
-constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;  // clears the bit of a shared::cluster address that tells the pair's CTAs apart
+// Clears the bit of a shared::cluster address that tells the pair's CTAs apart, as public sources for two-CTA loads have it (CUTLASS's copy_sm100_tma.hpp).
+constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;
 
 // One product of a launch.
 struct Part {
@@ -402,9 +403,10 @@ Part part_of(int M, int N, int K, int width) {
 double tile_cost(int kblocks, int n) { return kblocks * std::max(0.152, 0.026 + 0.00108 * n) + 0.54; }
 
 // Rows of W per tile, and the time this is expected to take (us).  Measured on a B200 (2,023 products of 160 to 4,096 tokens by 160 to 8,192
-// features, K 128 to 8,192, in tiles of 32 to 256 rows; within 7%): a product begins and ends in 3.8 us, a round of tiles costs 0.54 and per
+// features, K 128 to 8,192, in tiles of 32 to 256 rows; within 7%, and within a tenth for 1,206 of 1,520 others, one behind the other): a product begins and ends in 3.8 us, a round of tiles costs 0.54 and per
 // K block its MMAs' time, or 0.15 (what an MMA on two SMs takes at least, and the threads that issue it), and the stores 0.16 a megabyte.
-// A tile of 256 rows takes 0.30 a K block, 1,680 TFLOP/s over the device, so wide tiles are the rule, and narrower ones what fills the
+// A tile of 256 rows takes 0.30 a K block (8.4 MFLOP on two SMs: 2,070 TFLOP/s over the device while it lasts, at a short product's clocks; with its ends, and
+// at the clocks that the power cap leaves a long one, 4,096 x 10,240 x 4,096 takes 215, 1,600 TFLOP/s), so wide tiles are the rule, and narrower ones what fills the
 // last round: 2,048 x 6,144 pairs x 2,048 in 512 tiles of 96 pairs (6.9 rounds) 66.1, in 384 of 128 (5.2) 68.9; 1,111 x 2,048 x 6,144 24.2 in
 // tiles of 160 rows (one round), 36.5 in tiles of 256.
 double plan_width(bool gated, int M, int N, int K, int out_bytes, int sm_count, int* n_tile) {
@@ -523,13 +525,17 @@ LIA_EXPORT int lia_gemm_pair_grouped(int mode, const void* X, int ldx, int rows_
 }
 
 // The product on pairs of SMs with tiles of `n_tile` rows of W (0: as many as it would choose), for tests and measurements; lia_gemm_tc
-// chooses it by itself.
+// chooses it by itself.  The epilogue's variant rides above the mode's byte, as there.
 LIA_EXPORT int lia_gemm_pair(int mode, const void* X, int ldx, const void* W, int ldw, void* out, int out_dtype, int ldo, int M,
-                             int N, int K, float alpha, int sm_count, int n_tile, int* error_flag, cudaStream_t stream) {
+                             int N, int K, float alpha, int sm_count, int n_tile, float act_p, float act_n, int* error_flag, cudaStream_t stream) {
+    const int act = mode >> 8;
+    mode &= 0xff;
+    if (act != 0 && !(mode == GEMM_SWIGLU && act == 4) && !(mode == GEMM_STORE && (act == 3 || act == 5))) return LIA_ERR_SIZE;
     if (M <= 0 || N <= 0) return LIA_OK;
     if (K <= 0 || K % 8 || ldx < K || ldw < K || ldo < N || (mode != GEMM_STORE && mode != GEMM_ACCUM && mode != GEMM_SWIGLU))
         return LIA_ERR_SIZE;
     if ((out_dtype != LIA_F32 && out_dtype != LIA_BF16) || (mode == GEMM_ACCUM && out_dtype != LIA_F32)) return LIA_ERR_DTYPE;
     if (((uintptr_t)out & 15u) || ((long long)ldo * (out_dtype == LIA_F32 ? 4 : 2)) % 16) return LIA_ERR_ALIGN;
-    return gemm_pair_launch(mode, X, ldx, W, ldw, out, out_dtype, ldo, M, N, K, alpha, sm_count, n_tile, 0.f, 0.f, error_flag, stream);
+    const int form = act == 5 ? GEMM_STORE_XIELU : act == 3 ? GEMM_STORE_RELU2 : act == 4 ? GEMM_REGLU : mode;
+    return gemm_pair_launch(form, X, ldx, W, ldw, out, out_dtype, ldo, M, N, K, alpha, sm_count, n_tile, act_p, act_n, error_flag, stream);
 }

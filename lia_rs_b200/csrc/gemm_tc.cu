@@ -433,8 +433,8 @@ int pow2_at_least(int x) {
     return p;
 }
 
-// What a round of tiles of n tokens takes (us).  Measured on a B200 (247 products of 160 to 4,096 tokens, within 9%, with 0.8 us for the
-// whole and 0.14 a megabyte of output): 2.6 us, and per K block the longest of its MMAs' time (0.38 at 256 tokens, twice that for
+// What a round of tiles of n tokens takes (us).  Measured on a B200 (fitted to 247 products of 160 to 4,096 tokens, within 9%, with 0.8 us for the
+// whole and 0.14 a megabyte of output; one behind the other, 1,162 of 1,520 others are within a tenth): 2.6 us, and per K block the longest of its MMAs' time (0.38 at 256 tokens, twice that for
 // the gated product's two accumulators), the time the SM needs to take the block in (a row of W or X is 128 bytes), and 0.21.
 double round_cost(bool gated, int n, int kblocks) {
     const double weights = gated ? 2.0 : 1.0;
@@ -492,6 +492,21 @@ Plan make_plan(int mode, int M, int N, int K, int sm_count, long long scratch_fl
     return p;
 }
 
+// Many tokens: whether pairs of SMs take the product: where their estimate is a twentieth below this kernel's.  us, one CTA a tile / pairs: 2,048 x
+// 8,192 x 2,048 75.9 / 51.2, 4,096 x 2,048 x 6,144 92.4 / 73.0, 256 x 2,048 gated pairs x 2,048 13.7 / 9.9, 2,048 x 2,048 x 6,144 38.8 / 36.6; where tiles of one
+// CTA just make a full round they stay here (1,111 x 3,088 x 1,024 9.8 / 11.0).
+// Why a twentieth: the estimates are within a tenth of what three products of four take (1,520 products of 130 to 4,096 tokens, 160 to 10,240
+// features, K 72 to 4,096, in four forms, timed both ways), and the line leans to the kernel that they all went to once.  It sends 20 of them to pairs that are
+// 3 to 19% slower there (the worst, 3,500 x 8,192 x 128 added to the output, 37.1 / 44.2) and keeps 206 here that pairs would do 3 to 24% faster (1,024 x 8,192 x 512 in
+// bfloat16 13.2 / 10.7): 1.2% over the better kernel of each in the mean.  At equal estimates it would be 53, 49 and 0.6%.
+// (up to 128 tokens K is cut and the ranges are added up with rounding: pairs have one accumulator for all of K, which is cut off at every step)
+bool pairs_are_faster(const Plan& plan, int mode, int M, int N, int K, int out_bytes, int sm_count) {
+    if (M <= 128 || sm_count < 2) return false;
+    const long long rounds = ((long long)plan.f_tiles * plan.t_tiles + sm_count - 1) / sm_count;
+    const double alone = 0.8 + rounds * round_cost(mode == GEMM_SWIGLU, plan.n_tile, (K + BLOCK_K - 1) / BLOCK_K) + 0.14e-6 * out_bytes * M * N;
+    return gemm_pair_estimate(mode, M, N, K, out_bytes, sm_count) < 0.95 * alone;
+}
+
 template <int MODE, typename TO>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mo, TO* out, const Shape& s, int grid,
            cudaStream_t stream) {
@@ -525,18 +540,10 @@ LIA_EXPORT int lia_gemm_tc(int mode, const void* X, int ldx, const void* W, int 
     if (out_dtype != LIA_F32 && out_dtype != LIA_BF16) return LIA_ERR_DTYPE;
     const bool swiglu = mode == GEMM_SWIGLU;
     const Plan plan = make_plan(mode, M, N, K, sm_count, scratch ? scratch_floats : 0);
-    // Many tokens: pairs of SMs where they are expected to be faster by the twentieth that the estimates are sure of.  They are for
-    // products of several rounds or wide tiles (us, one CTA a tile / pairs: 2,048 x 8,192 x 2,048 72 / 51, 4,096 x 2,048 x 6,144 110 / 76, 256 x 2,048 pairs x
-    // 2,048 14.1 / 9.5), and not where tiles of one CTA make one full round (2,048 x 2,048 x 6,144 36.1 / 38.9, 1,111 x 3,088 x 1,024 9.8 / 11.0).
     const int out_bytes = out_dtype == LIA_F32 ? 4 : 2;
-    // (up to 128 tokens K is cut and the ranges are added up with rounding: pairs have one accumulator for all of K, which is cut off at every step)
-    if (M > 128 && sm_count >= 2 && ((uintptr_t)out & 15u) == 0 && ((long long)ldo * out_bytes) % 16 == 0) {
-        const long long rounds = ((long long)plan.f_tiles * plan.t_tiles + sm_count - 1) / sm_count;
-        const double alone = 0.8 + rounds * round_cost(swiglu, plan.n_tile, (K + BLOCK_K - 1) / BLOCK_K) + 0.14e-6 * out_bytes * M * N;
-        if (gemm_pair_estimate(mode, M, N, K, out_bytes, sm_count) < 0.95 * alone) {
-            const int form = act == 5 ? GEMM_STORE_XIELU : act == 3 ? GEMM_STORE_RELU2 : act == 4 ? GEMM_REGLU : mode;
-            return gemm_pair_launch(form, X, ldx, W, ldw, out, out_dtype, ldo, M, N, K, alpha, sm_count, 0, act_p, act_n, error_flag, stream);
-        }
+    if (((uintptr_t)out & 15u) == 0 && ((long long)ldo * out_bytes) % 16 == 0 && pairs_are_faster(plan, mode, M, N, K, out_bytes, sm_count)) {
+        const int form = act == 5 ? GEMM_STORE_XIELU : act == 3 ? GEMM_STORE_RELU2 : act == 4 ? GEMM_REGLU : mode;
+        return gemm_pair_launch(form, X, ldx, W, ldw, out, out_dtype, ldo, M, N, K, alpha, sm_count, 0, act_p, act_n, error_flag, stream);
     }
 
     Shape s;
@@ -587,6 +594,13 @@ LIA_EXPORT int lia_gemm_tc(int mode, const void* X, int ldx, const void* W, int 
     if (mode == GEMM_ACCUM) return launch<GEMM_ACCUM, float>(mw, mx, mo, (float*)out, s, grid, stream);
     if (out_dtype == LIA_F32) return launch<GEMM_SWIGLU, float>(mw, mx, mo, (float*)out, s, grid, stream);
     return launch<GEMM_SWIGLU, __nv_bfloat16>(mw, mx, mo, (__nv_bfloat16*)out, s, grid, stream);
+}
+
+// Whether lia_gemm_tc gives a product with an output that TMA can address to pairs of SMs (csrc/gemm_pair.cu).
+LIA_EXPORT int lia_gemm_tc_on_pairs(int mode, int out_dtype, int M, int N, int K, int sm_count) {
+    mode &= 0xff;
+    if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0) return 0;
+    return pairs_are_faster(make_plan(mode, M, N, K, sm_count, 0), mode, M, N, K, out_dtype == LIA_F32 ? 4 : 2, sm_count) ? 1 : 0;
 }
 
 // The grouped product: X [rows_cap, K] bf16 = the tokens' rows sorted by group, every group's rows beginning at a multiple

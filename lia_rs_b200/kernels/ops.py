@@ -61,8 +61,9 @@ class _Signatures:
     lia_attention_decode_ctas_per_sm = [c_int, c_int, c_int]
     lia_gemm_tc = [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                    c_void_p, ctypes.c_longlong, c_int, c_float, c_float, c_void_p, c_void_p]
+    lia_gemm_tc_on_pairs = [c_int, c_int, c_int, c_int, c_int, c_int]
     lia_gemm_pair = [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
-                     c_int, c_int, c_void_p, c_void_p]
+                     c_int, c_int, c_float, c_float, c_void_p, c_void_p]
     lia_gemm_pair_grouped = [c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                              c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
     lia_gemm_cluster = [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
@@ -491,16 +492,21 @@ def gemm_tc(mode, a, w, out, alpha: float = 1.0, error_flag=None, label=None, ac
                                  float(act_constants[1]), _p(error_flag), _stream()), "gemm_tc")
 
 
-def gemm_pair(mode, a, w, out, alpha: float = 1.0, n_tile: int = 0, error_flag=None):
+def gemm_tc_on_pairs(mode, out_dtype, M: int, N: int, K: int, sms: int) -> bool:
+    """Whether `gemm_tc` gives this product (its output addressable by TMA) to pairs of SMs, on a device of so many."""
+    return lib().lia_gemm_tc_on_pairs(mode, dtype_code(out_dtype), M, N, K, sms) != 0
+
+
+def gemm_pair(mode, a, w, out, alpha: float = 1.0, n_tile: int = 0, error_flag=None, act: int = 0, act_constants=(0.0, 0.0)):
     """out[M, N] (op)= alpha * a[M, K] @ w[N, K]^T on pairs of SMs with tiles of `n_tile` rows of w (0: chosen by the sizes); see
-    csrc/gemm_pair.cu.  `gemm_tc` goes there by itself for the products that it is faster for."""
+    csrc/gemm_pair.cu.  `gemm_tc` goes there by itself for the products that it is faster for; `act` as there."""
     M, K = a.shape
     N = out.shape[1]
     if w.shape[1] != K or out.shape[0] != M or w.shape[0] != (2 * N if mode == GEMM_SWIGLU else N):
         raise KernelError(f"gemm: shapes do not agree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     _, sms = _device_scratch(a.device)
-    _check(lib().lia_gemm_pair(mode, _p(a), a.stride(0), _p(w), w.stride(0), _p(out), dtype_code(out.dtype), out.stride(0), M, N, K,
-                               alpha, sms, int(n_tile), _p(error_flag), _stream()), "gemm_pair")
+    _check(lib().lia_gemm_pair(mode | (int(act) << 8), _p(a), a.stride(0), _p(w), w.stride(0), _p(out), dtype_code(out.dtype), out.stride(0), M, N, K,
+                               alpha, sms, int(n_tile), float(act_constants[0]), float(act_constants[1]), _p(error_flag), _stream()), "gemm_pair")
 
 
 def gemm_cluster_accepts(mode, a, w, out, least: int = 2) -> bool:
