@@ -2,7 +2,8 @@
 // 16 (up to 256), any number of heads and groups, any page size, prompt portions and single decoded
 // tokens alike.  One warp owns one (token, query head): it walks the visible keys 32 at a time,
 // each lane scoring one key, keeps the running maximum and sum of the softmax in 32-bit, and
-// accumulates the output with each lane owning head elements lane, lane+32, ...
+// accumulates the output with each lane owning head elements lane, lane+32, ...  Few (token, query head) items of 32-bit elements get
+// a CTA each instead (attention_rows_kernel), with the same bits.
 //
 // A token at position p of request slot s sees keys j with max(0, p - window + 1) <= j <= p
 // (window <= 0: all keys), read from that slot's pages.  The order of the work depends on p and the
@@ -200,9 +201,11 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k_p
         if (tid + x * ROW_KEYS < d) orow[tid + x * ROW_KEYS] = acc[x] * inv;
 }
 
-// (token, query head) items up to which a CTA each is faster than a warp each, however few keys they see: a CTA keeps a tile's values in shared
+// (token, query head) items up to which a CTA each is faster than a warp each: a CTA keeps a tile's values in shared
 // memory, of which an SM holds one of 256 elements.  us behind 20 keys, a warp / a CTA: 256 elements 256 items 21.0/15.3, 512 20.9/27.0; 128
-// elements 1,024 items 19.2/15.5, 2,048 28.7/24.9, 4,096 44.7/46.8; 64 elements 4,096 27.0/21.0.
+// elements 1,024 items 19.2/15.5, 2,048 28.7/24.9, 4,096 44.7/46.8; 64 elements 4,096 27.0/21.0.  The number of keys is known on the device alone: behind a
+// single key, a conversation's first token, many items are slower so (128 elements 512 items 7.6/8.6, 1,024 7.5/12.0, 2,048 7.6/19.0; 64 elements 2,048 6.1/10.3),
+// which every later token of theirs makes up for.
 long long rows_up_to(int d) { return d <= 128 ? 2048 : 256; }
 
 int launch_rows(const float* q, const float* k_pages, const float* v_pages, const int* positions, const int* slots, const int* block_table,
