@@ -18,7 +18,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 // knows such a branch to have one thread.  Behind `lane == 0` it does not, and goes about each of these instructions, whose
 // operands are a warp's, thread by thread, which is what a K block of a narrow tile then takes.  us, behind `lane == 0` and so: products of
 // 2,048 tokens x 160 x 4,096 24.7 / 17.0, 1,111 x 2,048 x 2,048 16.1 / 12.1, 2,048 x 2,048 x 6,144 39.5 / 36.4; 512 tokens through eight
-// experts and a shared one 126 / 107; steps of 1, 8 and 64 tokens (8 layers) 370, 394, 673 / 362, 384, 663.
+// experts and a shared one 126 / 107; steps of 8 and 64 tokens (8 layers) 395, 674 / 387, 662, of one 371 / 370.
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred P;\n\t.reg .b32 R;\n\telect.sync R|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
